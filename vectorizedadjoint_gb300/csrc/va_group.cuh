@@ -47,12 +47,12 @@ __device__ __forceinline__ dword shfl(dword v, int src, unsigned mask)
 template <int G>
 __device__ __forceinline__ double group_max(double v, unsigned mask)
 {
-    const bool nan = v != v;
+    const bool nan = is_nan64(v);
     const int base = (threadIdx.x & 31) / G * G;
     double m = 0.0;
 #pragma unroll
     for (int j = 0; j < G; j++)
-        m = fmax(m, __shfl_sync(mask, v, base + j));
+        m = max_nonneg64(m, fabs(__shfl_sync(mask, v, base + j)));
     return __any_sync(mask, nan) ? __longlong_as_double(0x7ff8000000000000ll) : m;
 }
 
@@ -276,7 +276,7 @@ __global__ void __launch_bounds__(256) forward_group_kernel(FwdParams a)
             continue;
         }
         if (at_top) {
-            if (Tab::FIXED ? !((t + dt) - t1 <= kDblEps) : !(t1 - t > kDblEps)) {
+            if (Tab::FIXED ? !less_equal_pos64((t + dt) - t1, kDblEps) : !greater_pos64(t1 - t, kDblEps)) {
                 finish();
                 alive = fetch();
                 continue;
@@ -293,7 +293,7 @@ __global__ void __launch_bounds__(256) forward_group_kernel(FwdParams a)
                 }
                 write();
             }
-            if (!Tab::FIXED && (t + dt) - t1 > kDblEps)
+            if (!Tab::FIXED && greater_pos64((t + dt) - t1, kDblEps))
                 dt = t1 - t;
             fails = 0;
             at_top = false;
@@ -303,11 +303,11 @@ __global__ void __launch_bounds__(256) forward_group_kernel(FwdParams a)
         const double err = group_max<G>(
             attempt<M, Tab, S>(y, ys, k0, p, t, dt, a.atol, a.rtol, ynew, ynew_s, knew), mask);
         bool ok;
-        if (err != err) {
+        if (is_nan64(err)) {
             status = ST_NONFINITE;
             continue;
         }
-        if (err > 1.0) {
+        if (greater_nonneg64(err, 1.0)) {
             dt = decrease_step<Tab, S>(dt, err, a.step_pow, li == 0 ? &a.ctl->pow_undecided : nullptr);
             rej++;
             ok = false;
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(256) forward_group_kernel(FwdParams a)
         if (ok) {
             count++;
             at_top = true;
-        } else if (!(dt > 0.0) || !isfinite(dt)) {
+        } else if (!positive_finite64(dt)) {
             status = ST_NONFINITE;
         }
     }

@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(256) backward_group_kernel_2level(AdjParams a)
         if (phase == 0) {
             // one attempt of the forward controller, as forward_group_kernel does
             if (at_top) {
-                if (!Tab::FIXED && (t + dt) - t1 > kDblEps)
+                if (!Tab::FIXED && greater_pos64((t + dt) - t1, kDblEps))
                     dt = t1 - t;
                 fails = 0;
                 at_top = false;
@@ -169,13 +169,13 @@ __global__ void __launch_bounds__(256) backward_group_kernel_2level(AdjParams a)
             S ynew_s[1], knew[1];
             const double err = group_max<G>(
                 attempt<M, Tab, S>(y, ys, k0, p, t, dt, a.atol, a.rtol, ynew, ynew_s, knew), mask);
-            if (err != err || fails >= a.max_fail) {
+            if (is_nan64(err) || fails >= a.max_fail) {
                 fail_instance(ST_RECOMPUTE_MISMATCH);
                 alive = fetch();
                 continue;
             }
             fails++;
-            if (err > 1.0) {
+            if (greater_nonneg64(err, 1.0)) {
                 dt = decrease_step<Tab, S>(dt, err, a.step_pow, li == 0 ? &a.ctl->pow_undecided : nullptr);
                 continue;
             }

@@ -180,6 +180,11 @@ __host__ __device__ __forceinline__ float fromf<float>(float v)
 }
 
 // ---------------------------------------------------------------- controller
+//
+// The controller's decisions compare non-negative numbers (or a number of any
+// sign with a positive constant), whose order is that of their bit patterns:
+// integer comparisons, where an FP64 compare would take the FP64 unit for 64
+// cycles (va_int64.cuh).
 
 // FP64 Newton steps of the step-factor root: two on the FP64 path (the
 // scheme the oracle shares), one on the reduced paths (~3e-14 relative,
@@ -211,7 +216,7 @@ __host__ __device__ __forceinline__ double decrease_step(double dt, double err, 
         else
             r = inv_root<Tab::ERROR_ORDER - 1, RootSteps<S>::value>(err);
         double f = 9.0 / 10.0 * r;
-        return dt * fmax(f, 1.0 / 5.0);
+        return dt * max_nonneg64(f, 1.0 / 5.0);
     }
 }
 
@@ -227,10 +232,10 @@ __host__ __device__ __forceinline__ double increase_step(double dt, double err, 
         (void)undecided;
         return dt;
     } else {
-        if (err < 0.5) {
+        if (greater_nonneg64(0.5, err)) {
             // 5^-p as the correctly rounded quotient (1/3125, 1/390625), what
             // pow(5.0, -p) returns
-            err = fmax(Tab::ERR_FLOOR, err);
+            err = max_nonneg64(Tab::ERR_FLOOR, err);
             double r;
             if (std::is_same<S, double>::value && step_pow)
                 r = cr_step_pow<Tab::STEPPER_ORDER>(err, undecided);
@@ -400,11 +405,10 @@ __host__ __device__ __forceinline__ double attempt_pair(const double (&y)[M::N],
         double m = 0.0;
 #pragma unroll
         for (int i = 0; i < N; i++) {
-            const double r = fabs(e[i]) / (atol + rtol * (1.0 * fabs(y[i]) + adt * fabs(k0[i])));
-            if (r != r)
+            const double r = quotient64(fabs(e[i]), atol + rtol * (1.0 * fabs(y[i]) + adt * fabs(k0[i])));
+            if (is_nan64(r))
                 return r;
-            if (r > m)
-                m = r;
+            m = max_nonneg64(m, r);
         }
         return m;
     }
@@ -697,7 +701,7 @@ __global__ void __launch_bounds__(256) forward_kernel(FwdParams a)
         if (at_top) {
             // while (less_with_sign(t, t1, dt))  (runge_kutta.hpp:155); fixed
             // steps: while (less_eq_with_sign(t + dt, t1, dt))  (:54)
-            if (Tab::FIXED ? !((t + dt) - t1 <= kDblEps) : !(t1 - t > kDblEps)) {
+            if (Tab::FIXED ? !less_equal_pos64((t + dt) - t1, kDblEps) : !greater_pos64(t1 - t, kDblEps)) {
                 finish();
                 alive = fetch();
                 continue;
@@ -716,7 +720,7 @@ __global__ void __launch_bounds__(256) forward_kernel(FwdParams a)
                 slot++;
             }
             // end clamp (runge_kutta.hpp:160-163)
-            if (!Tab::FIXED && (t + dt) - t1 > kDblEps)
+            if (!Tab::FIXED && greater_pos64((t + dt) - t1, kDblEps))
                 dt = t1 - t;
             fails = 0;
             at_top = false;
@@ -725,11 +729,11 @@ __global__ void __launch_bounds__(256) forward_kernel(FwdParams a)
         S ynew_s[N], knew[N];
         const double err = attempt<M, Tab, S>(y, ys, k0, p, t, dt, a.atol, a.rtol, ynew, ynew_s, knew);
         bool ok;
-        if (err != err) {
+        if (is_nan64(err)) {
             status = ST_NONFINITE;
             continue;
         }
-        if (err > 1.0) {
+        if (greater_nonneg64(err, 1.0)) {
             dt = decrease_step<Tab, S>(dt, err, a.step_pow, &a.ctl->pow_undecided);
             rej++;
             ok = false;
@@ -752,7 +756,7 @@ __global__ void __launch_bounds__(256) forward_kernel(FwdParams a)
         if (ok) {
             count++;
             at_top = true;
-        } else if (!(dt > 0.0) || !isfinite(dt)) {
+        } else if (!positive_finite64(dt)) {
             status = ST_NONFINITE;
         }
     }
@@ -1121,7 +1125,7 @@ __global__ void __launch_bounds__(256) backward_kernel_2level(AdjParams a)
         if (phase == 0) {
             // one attempt of the forward controller, as forward_kernel does
             if (at_top) {
-                if (!Tab::FIXED && (t + dt) - t1 > kDblEps)
+                if (!Tab::FIXED && greater_pos64((t + dt) - t1, kDblEps))
                     dt = t1 - t;
                 fails = 0;
                 at_top = false;
@@ -1129,13 +1133,13 @@ __global__ void __launch_bounds__(256) backward_kernel_2level(AdjParams a)
             double ynew[N];
             S ynew_s[N], knew[N];
             const double err = attempt<M, Tab, S>(y, ys, k0, p, t, dt, a.atol, a.rtol, ynew, ynew_s, knew);
-            if (err != err || fails >= a.max_fail) {
+            if (is_nan64(err) || fails >= a.max_fail) {
                 fail_instance(ST_RECOMPUTE_MISMATCH);
                 alive = fetch();
                 continue;
             }
             fails++;
-            if (err > 1.0) {
+            if (greater_nonneg64(err, 1.0)) {
                 dt = decrease_step<Tab, S>(dt, err, a.step_pow, &a.ctl->pow_undecided);
                 continue;
             }
