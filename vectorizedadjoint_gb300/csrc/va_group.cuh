@@ -65,6 +65,9 @@ struct ModelGLVLane {
     static constexpr int TPI = NN, NTOT = NN, PTOT = NN + NN * NN;
     static constexpr int N = 1, P = 1 + 2 * NN, PG = 1 + NN;
 
+    // whether `ok` holds on every lane of the group
+    __device__ __forceinline__ static bool all(bool ok) { return __all_sync(LaneGroup<NN>().mask, ok); }
+
     template <class S>
     __device__ __forceinline__ static void load_params(const double *par, int i, S (&p)[P])
     {

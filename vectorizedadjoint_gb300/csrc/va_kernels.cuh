@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "va_dword.cuh"
+#include "va_step64.cuh"
 #include "va_stepfactor.cuh"
 #include "va_tableau.cuh"
 
@@ -474,14 +475,65 @@ __host__ __device__ __forceinline__ void step_fixed(const double (&y)[M::N], con
 }
 
 // attempt_pair for the embedded pairs; a fixed-step tableau's step, with
-// error 0 (always accepted)
-template <class M, class Tab, class S>
+// error 0 (always accepted).  Double stages: the step with its products in
+// integers (attempt64); out of its range, the general one, called by value so
+// that the sweep's state stays in registers.
+template <int N>
+struct Attempt64 {
+    double ynew[N], knew[N], err;
+};
+template <int N, int P>
+struct State64 {
+    double y[N], k0[N], p[P], t, dt;
+};
+template <class M, class Tab>
+VA_HD_NOINLINE Attempt64<M::N> attempt_general64(State64<M::N, M::P> s, double atol, double rtol)
+{
+    Attempt64<M::N> o;
+    double same[M::N];
+    if constexpr (Tab::FIXED) {
+        step_fixed<M, Tab, double>(s.y, s.y, s.k0, s.p, s.t, s.dt, o.ynew, same);
+        o.err = 0.0;
+    } else {
+        o.err = attempt_pair<M, Tab, double>(s.y, s.y, s.k0, s.p, s.t, s.dt, atol, rtol, o.ynew, same, o.knew);
+    }
+    return o;
+}
+
+template <class M, class Tab, class S, bool INT64 = false>
 __host__ __device__ __forceinline__ double attempt(const double (&y)[M::N], const S (&ys)[M::N],
                                                    const S (&k0)[M::N], const S (&p)[M::P], double t,
                                                    double dt, double atol, double rtol, double (&ynew)[M::N],
                                                    S (&ynew_s)[M::N], S (&knew)[M::N])
 {
-    if constexpr (Tab::FIXED) {
+    if constexpr (INT64) {
+        constexpr int N = M::N;
+        double err;
+        if (!uniform64<M>(attempt64<M, Tab>(y, k0, p, t, dt, atol, rtol, ynew, knew, err))) {
+            State64<N, M::P> s;
+#pragma unroll
+            for (int i = 0; i < N; i++) {
+                s.y[i] = y[i];
+                s.k0[i] = k0[i];
+            }
+#pragma unroll
+            for (int k = 0; k < M::P; k++)
+                s.p[k] = p[k];
+            s.t = t;
+            s.dt = dt;
+            const Attempt64<N> o = attempt_general64<M, Tab>(s, atol, rtol);
+#pragma unroll
+            for (int i = 0; i < N; i++) {
+                ynew[i] = o.ynew[i];
+                knew[i] = o.knew[i];
+            }
+            err = o.err;
+        }
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            ynew_s[i] = ynew[i];
+        return err;
+    } else if constexpr (Tab::FIXED) {
         (void)atol;
         (void)rtol;
         (void)knew;
@@ -590,7 +642,7 @@ __device__ __forceinline__ void read_record(const double *r, double &t, double (
 
 // ------------------------------------------------------------ forward sweep
 
-template <class M, class Tab, class S>
+template <class M, class Tab, class S, bool INT64 = false>
 __global__ void __launch_bounds__(256) forward_kernel(FwdParams a)
 {
     constexpr int N = M::N, P = M::P;
@@ -727,7 +779,7 @@ __global__ void __launch_bounds__(256) forward_kernel(FwdParams a)
         }
         double ynew[N];
         S ynew_s[N], knew[N];
-        const double err = attempt<M, Tab, S>(y, ys, k0, p, t, dt, a.atol, a.rtol, ynew, ynew_s, knew);
+        const double err = attempt<M, Tab, S, INT64>(y, ys, k0, p, t, dt, a.atol, a.rtol, ynew, ynew_s, knew);
         bool ok;
         if (is_nan64(err)) {
             status = ST_NONFINITE;
@@ -767,7 +819,7 @@ __global__ void __launch_bounds__(256) forward_kernel(FwdParams a)
 // One back_prop_step (backpropagation.hpp:160-229) for step n with state y_n,
 // start time tn and h = t_{n+1} - t_n.  lam: in lambda_{n+1}, out lambda_n.
 template <class M, class Tab, class S>
-__host__ __device__ __forceinline__ void back_step(const double (&y)[M::N], double tn, double h,
+__host__ __device__ __forceinline__ void back_step_general(const double (&y)[M::N], double tn, double h,
                                           const S (&p)[M::P], double (&lam)[M::N],
                                           double (&mu)[M::PG])
 {
@@ -857,7 +909,60 @@ __host__ __device__ __forceinline__ void back_step(const double (&y)[M::N], doub
     }
 }
 
-template <class M, class Tab, class S>
+// back_step for double stages out of back_step64's range, by value
+template <int N, int P, int PG>
+struct Back64 {
+    double y[N], p[P], lam[N], mu[PG], tn, h;
+};
+template <class M, class Tab>
+VA_HD_NOINLINE Back64<M::N, M::P, M::PG> back_general64(Back64<M::N, M::P, M::PG> s)
+{
+    back_step_general<M, Tab, double>(s.y, s.tn, s.h, s.p, s.lam, s.mu);
+    return s;
+}
+
+template <class M, class Tab, class S, bool INT64 = false>
+__host__ __device__ __forceinline__ void back_step(const double (&y)[M::N], double tn, double h,
+                                                   const S (&p)[M::P], double (&lam)[M::N], double (&mu)[M::PG])
+{
+    if constexpr (INT64) {
+        double l[M::N], m[M::PG];
+        if (uniform64<M>(back_step64<M, Tab>(y, tn, h, p, lam, mu, l, m))) {
+#pragma unroll
+            for (int i = 0; i < M::N; i++)
+                lam[i] = l[i];
+#pragma unroll
+            for (int k = 0; k < M::PG; k++)
+                mu[k] = m[k];
+            return;
+        }
+        Back64<M::N, M::P, M::PG> s;
+#pragma unroll
+        for (int i = 0; i < M::N; i++) {
+            s.y[i] = y[i];
+            s.lam[i] = lam[i];
+        }
+#pragma unroll
+        for (int k = 0; k < M::P; k++)
+            s.p[k] = p[k];
+#pragma unroll
+        for (int k = 0; k < M::PG; k++)
+            s.mu[k] = mu[k];
+        s.tn = tn;
+        s.h = h;
+        s = back_general64<M, Tab>(s);
+#pragma unroll
+        for (int i = 0; i < M::N; i++)
+            lam[i] = s.lam[i];
+#pragma unroll
+        for (int k = 0; k < M::PG; k++)
+            mu[k] = s.mu[k];
+    } else {
+        back_step_general<M, Tab, S>(y, tn, h, p, lam, mu);
+    }
+}
+
+template <class M, class Tab, class S, bool INT64 = false>
 __global__ void __launch_bounds__(256) backward_kernel(AdjParams a)
 {
     constexpr int N = M::N, P = M::P;
@@ -965,7 +1070,7 @@ __global__ void __launch_bounds__(256) backward_kernel(AdjParams a)
         double y[N], tn;
         read_record<N>(record_ptr<RS>(a.pool, chunk, slot), tn, y);
         const double h = t_next - tn;
-        back_step<M, Tab, S>(y, tn, h, p, lam, mu);
+        back_step<M, Tab, S, INT64>(y, tn, h, p, lam, mu);
         note_lambda<N>(a, b, q, j, lam);
         t_next = tn;
         j--;
@@ -982,7 +1087,7 @@ __global__ void __launch_bounds__(256) backward_kernel(AdjParams a)
 // back_step through the segment in reverse.  Memory: one record per stride
 // steps plus (stride + 1) scratch records per thread, for one extra forward
 // evaluation of every step.
-template <class M, class Tab, class S>
+template <class M, class Tab, class S, bool INT64 = false>
 __global__ void __launch_bounds__(256) backward_kernel_2level(AdjParams a)
 {
     constexpr int N = M::N, P = M::P;
@@ -1132,7 +1237,7 @@ __global__ void __launch_bounds__(256) backward_kernel_2level(AdjParams a)
             }
             double ynew[N];
             S ynew_s[N], knew[N];
-            const double err = attempt<M, Tab, S>(y, ys, k0, p, t, dt, a.atol, a.rtol, ynew, ynew_s, knew);
+            const double err = attempt<M, Tab, S, INT64>(y, ys, k0, p, t, dt, a.atol, a.rtol, ynew, ynew_s, knew);
             if (is_nan64(err) || fails >= a.max_fail) {
                 fail_instance(ST_RECOMPUTE_MISMATCH);
                 alive = fetch();
@@ -1182,7 +1287,7 @@ __global__ void __launch_bounds__(256) backward_kernel_2level(AdjParams a)
                 yj[i] = r[2 + i];
             const double tn = r[0];
             const double h = scr[(size_t)(jb + 1) * RS] - tn;
-            back_step<M, Tab, S>(yj, tn, h, p, lam, mu);
+            back_step<M, Tab, S, INT64>(yj, tn, h, p, lam, mu);
             note_lambda<N>(a, b, q, first + jb, lam);
             jb--;
             if (jb < 0) {

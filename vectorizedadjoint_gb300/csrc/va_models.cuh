@@ -12,12 +12,16 @@
 // double-word multiply followed by a double-word add: the same O(u^2)
 // accuracy in about half the FP32 operations.  The FP64 forms keep the
 // reference's operation order (the FP64 path is compared bit for bit).
+// rhs64 and vjp64 are the double forms with their products on the integer pipe
+// (va_step64.cuh): the same operations in the same order, at most four noted
+// values multiplied together.
 // Parameter layouts follow the reference examples.
 #pragma once
 
 #include <type_traits>
 
 #include "va_dword.cuh"
+#include "va_int64.cuh"
 
 namespace va {
 
@@ -72,6 +76,25 @@ struct ModelVdP {
             gp[0] = w[1] * ((S(1) - x[0] * x[0]) * x[1]);
         }
     }
+    static constexpr bool kProducts64 = true;
+    __host__ __device__ __forceinline__ static void rhs64(const double *x, const double *p, double *f, MulRange &r)
+    {
+        const double a = 1.0 - mul_rn(mul_left(x[0], r), mul_right_in(x[0]));
+        f[0] = x[1];
+        f[1] = mul_rn(mul_left_in(mul_rn(mul_left_in(a), mul_right(p[0], r))), mul_right(x[1], r)) - x[0];
+    }
+    __host__ __device__ __forceinline__ static void vjp64(const double *w, const double *x, const double *p,
+                                                          double *gx, double *gp, MulRange &r)
+    {
+        const MulR x1 = mul_right(x[1], r), mu = mul_right(p[0], r);
+        const MulL w1 = mul_left(w[1], r), x0 = mul_left(x[0], r);
+        const double a = 1.0 - mul_rn(x0, mul_right_in(x[0]));
+        const MulL al = mul_left_in(a);
+        const double mx = mul_rn(mul_m2(x0), mu); // -2 mu x0
+        gx[0] = mul_rn(w1, mul_right_in(mul_rn(mul_left_in(mx), x1) - 1.0));
+        gx[1] = w[0] + mul_rn(w1, mul_right_in(mul_rn(al, mu)));
+        gp[0] = mul_rn(w1, mul_right_in(mul_rn(al, x1)));
+    }
 };
 
 // Van der Pol as in the reference example (examples/VanDerPol/main.cpp:41-42):
@@ -103,6 +126,26 @@ struct ModelVdPPetsc {
             gx[1] = w[0] + w[1] * (mu * (S(1) - x[0] * x[0]));
             gp[0] = w[1] * ((S(1) - x[0] * x[0]) * x[1] - x[0]);
         }
+    }
+    static constexpr bool kProducts64 = true;
+    __host__ __device__ __forceinline__ static void rhs64(const double *x, const double *p, double *f, MulRange &r)
+    {
+        const double a = 1.0 - mul_rn(mul_left(x[0], r), mul_right_in(x[0]));
+        f[0] = x[1];
+        f[1] = mul_rn(mul_left_in(mul_rn(mul_left_in(a), mul_right(x[1], r)) - x[0]), mul_right(p[0], r));
+    }
+    __host__ __device__ __forceinline__ static void vjp64(const double *w, const double *x, const double *p,
+                                                          double *gx, double *gp, MulRange &r)
+    {
+        const MulR x1 = mul_right(x[1], r), mu = mul_right(p[0], r);
+        const MulL w1 = mul_left(w[1], r), x0 = mul_left(x[0], r);
+        const double a = 1.0 - mul_rn(x0, mul_right_in(x[0]));
+        const MulL al = mul_left_in(a);
+        const double ax = mul_rn(al, x1); // (1 - x0^2) x1
+        const double c = mul_rn(mul_left_in(mul_rn(mul_m2(x0), x1) - 1.0), mu);
+        gx[0] = mul_rn(w1, mul_right_in(c));
+        gx[1] = w[0] + mul_rn(w1, mul_right_in(mul_rn(al, mu)));
+        gp[0] = mul_rn(w1, mul_right_in(ax - x[0]));
     }
 };
 
@@ -144,6 +187,25 @@ struct ModelDHO {
             gp[1] = w[1] * (S(-2) * om * x[1]);
         }
     }
+    static constexpr bool kProducts64 = true;
+    __host__ __device__ __forceinline__ static void rhs64(const double *x, const double *p, double *f, MulRange &r)
+    {
+        const MulL om = mul_left(p[0], r), ze = mul_left(p[1], r);
+        const MulR omr = mul_right_in(p[0]);
+        const double k = mul_rn(mul_neg(om), omr), c = mul_rn(mul_m2(ze), omr); // -om om, -2 ze om
+        f[0] = x[1];
+        f[1] = mul_rn(mul_left(x[0], r), mul_right_in(k)) + mul_rn(mul_left(x[1], r), mul_right_in(c));
+    }
+    __host__ __device__ __forceinline__ static void vjp64(const double *w, const double *x, const double *p,
+                                                          double *gx, double *gp, MulRange &r)
+    {
+        const MulL om = mul_left(p[0], r), ze = mul_left(p[1], r), w1 = mul_left(w[1], r);
+        const MulR omr = mul_right_in(p[0]), x0 = mul_right(x[0], r), x1 = mul_right(x[1], r);
+        gx[0] = mul_rn(w1, mul_right_in(mul_rn(mul_neg(om), omr)));
+        gx[1] = w[0] + mul_rn(w1, mul_right_in(mul_rn(mul_m2(ze), omr)));
+        gp[0] = mul_rn(w1, mul_right_in(mul_rn(mul_m2(om), x0) + mul_rn(mul_m2(ze), x1)));
+        gp[1] = mul_rn(w1, mul_right_in(mul_rn(mul_m2(om), x1)));
+    }
 };
 
 // Exponential decay y' = -k y; p = (k).  Its discrete adjoint has a closed
@@ -162,6 +224,18 @@ struct ModelDecay {
         (void)t;
         gx[0] = -p[0] * w[0];
         gp[0] = -x[0] * w[0];
+    }
+    static constexpr bool kProducts64 = true;
+    __host__ __device__ __forceinline__ static void rhs64(const double *x, const double *p, double *f, MulRange &r)
+    {
+        f[0] = mul_rn(mul_neg(mul_left(p[0], r)), mul_right(x[0], r));
+    }
+    __host__ __device__ __forceinline__ static void vjp64(const double *w, const double *x, const double *p,
+                                                          double *gx, double *gp, MulRange &r)
+    {
+        const MulR wr = mul_right(w[0], r);
+        gx[0] = mul_rn(mul_neg(mul_left(p[0], r)), wr);
+        gp[0] = mul_rn(mul_neg(mul_left(x[0], r)), wr);
     }
 };
 

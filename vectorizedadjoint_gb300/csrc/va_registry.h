@@ -88,6 +88,13 @@ void fill_fixed_decay(KernelSet &k);
 void fill_fixed_glv5(KernelSet &k);
 void fill_fixed_glv10(KernelSet &k);
 
+// Further FP64 sweeps of a built-in one-thread model (fp64_path in va_api.cu
+// chooses): products on the integer pipe (va_step64.cuh).  Null: not compiled.
+struct Fp64Kernels {
+    const void *int_fwd[kTableaux], *int_bwd[kTableaux];
+};
+const Fp64Kernels *fp64_kernels(int model); // null: none for the model
+
 // Shared-matrix GLV: bundles of kBundleNB instances per CTA of N threads
 // (FP64, FP32); the double-word sweeps take bundles of kBundleNBdw, whose
 // 128 registers per thread let two CTAs share an SM (GLV-256: 8% faster

@@ -1,0 +1,279 @@
+// One FP64 step, forward and backward, with its products on the integer pipe
+// (va_int64.cuh).  The FP64 unit is left to the additions.
+//
+// What bounds it: an FP64 instruction holds its quadrant's FP64 unit for 64
+// cycles, and an attempt of Dormand-Prince on Van der Pol is ~100 products
+// and ~75 sums (a back step ~130 and ~100), so the one-thread FP64 sweeps
+// are bound by the FP64 instruction count at every batch size.  A product in
+// integers issues in ~45 cycles beside the sums.
+//
+// The operations and their order are those of attempt_pair, step_fixed and
+// back_step; every sum is the FP64 instruction and every product the
+// correctly rounded one, so the results have the same bits.  A coefficient
+// that is zero adds nothing here (its product with a finite value is a zero,
+// which changes no sum but one that is -0 itself: such a sum is handled as
+// the addition would).
+//
+// Range.  The products need operands whose significand and exponent can be
+// taken apart (no infinities, NaNs or subnormals) and results that are
+// normal.  Every value that enters a product from outside the product chain
+// is noted in a MulRange; the chains below multiply at most four noted values
+// before the next one is noted, so with all of them within 2^-240 .. 2^240 (or
+// zero) no product leaves the normal range.  Otherwise the functions return
+// false and the caller takes the step over with FP64 instructions throughout
+// (attempt_pair, step_fixed, back_step): the same result, or the same
+// infinities and NaNs.
+#pragma once
+
+#include <type_traits>
+
+#include "va_int64.cuh"
+
+namespace va {
+
+constexpr int kChainRange = 240;
+
+// Models that write their right-hand side and VJP with integer products
+// (rhs64, vjp64); for the others (a model compiled by the caller) the model
+// functions run as they are.
+template <class M, class = void>
+struct HasProducts64 : std::false_type {
+};
+template <class M>
+struct HasProducts64<M, std::void_t<decltype(M::kProducts64)>> : std::bool_constant<M::kProducts64> {
+};
+
+template <class M>
+__host__ __device__ __forceinline__ void model_rhs64(const double *x, const double *p, double t, double *f,
+                                                     MulRange &r)
+{
+    if constexpr (HasProducts64<M>::value) {
+        (void)t;
+        M::rhs64(x, p, f, r);
+    } else {
+        (void)r;
+        M::template rhs<double>(x, p, t, f);
+    }
+}
+template <class M>
+__host__ __device__ __forceinline__ void model_vjp64(const double *w, const double *x, const double *p, double t,
+                                                     double *gx, double *gp, MulRange &r)
+{
+    if constexpr (HasProducts64<M>::value) {
+        (void)t;
+        M::vjp64(w, x, p, gx, gp, r);
+    } else {
+        (void)r;
+        M::template vjp<double>(w, x, p, t, gx, gp);
+    }
+}
+
+// Whether every lane that carries the instance stayed in range (a lane-group
+// model, whose functions exchange components, answers for its group).
+template <class M, class = void>
+struct Uniform64 {
+    __host__ __device__ static bool all(bool ok) { return ok; }
+};
+template <class M>
+struct Uniform64<M, std::void_t<decltype(M::TPI)>> {
+    __device__ static bool all(bool ok) { return M::all(ok); }
+};
+template <class M>
+__host__ __device__ __forceinline__ bool uniform64(bool ok)
+{
+    return Uniform64<M>::all(ok);
+}
+
+// c h for a tableau coefficient c, as a second factor
+__host__ __device__ __forceinline__ MulR coef_right(double c, const MulR &h)
+{
+    return mul_right_in(mul_rn(mul_left_in(c), h));
+}
+
+template <class Tab>
+constexpr bool zero_in_a()
+{
+    for (int m = 1; m < Tab::S; m++)
+        for (int j = 0; j < m; j++)
+            if (Tab::a(m, j) == 0.0)
+                return true;
+    return false;
+}
+
+// X_m = y + sum_{j<m} (a_mj dt) K_j (form_stage), the non-zero coefficients
+template <class Tab, int N>
+__host__ __device__ __forceinline__ void form_stage64(int m, const double (&y)[N], const MulL (&K)[Tab::S][N],
+                                                      const MulR &h, double (&X)[N])
+{
+#pragma unroll
+    for (int i = 0; i < N; i++)
+        X[i] = y[i];
+#pragma unroll
+    for (int j = 0; j < Tab::S - 1; j++)
+        if (j < m && Tab::a(m, j) != 0.0) {
+            const MulR c = coef_right(Tab::a(m, j), h);
+#pragma unroll
+            for (int i = 0; i < N; i++)
+                X[i] = X[i] + mul_rn(K[j][i], c);
+        }
+}
+
+// attempt_pair's (step_fixed's) step for double stages: y_new, k_new and the
+// error norm (0 for a fixed-step tableau).  False: out of range.
+template <class M, class Tab>
+__host__ __device__ __forceinline__ bool attempt64(const double (&y)[M::N], const double (&k0)[M::N],
+                                                   const double (&p)[M::P], double t, double dt, double atol,
+                                                   double rtol, double (&ynew)[M::N], double (&knew)[M::N],
+                                                   double &err)
+{
+    constexpr int N = M::N, NS = Tab::S;
+    MulRange r;
+    const MulR h = mul_right(dt, r);
+    MulL K[NS][N];
+    bool neg_zero = false;
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        K[0][i] = mul_left(k0[i], r);
+        if (zero_in_a<Tab>()) // no sum starts from -0: skipped zero terms change none
+            neg_zero = neg_zero || f64_bits(y[i]) == 1ull << 63;
+    }
+#pragma unroll
+    for (int m = 1; m < NS; m++) {
+        double X[N], f[N];
+        form_stage64<Tab, N>(m, y, K, h, X);
+        model_rhs64<M>(X, p, t + Tab::c(m) * dt, f, r);
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            K[m][i] = mul_left(f[i], r);
+    }
+#pragma unroll
+    for (int i = 0; i < N; i++)
+        ynew[i] = y[i];
+#pragma unroll
+    for (int j = 0; j < NS; j++)
+        if (Tab::b(j) != 0.0) {
+            const MulR c = coef_right(Tab::b(j), h);
+#pragma unroll
+            for (int i = 0; i < N; i++)
+                ynew[i] = ynew[i] + mul_rn(K[j][i], c);
+        }
+    if constexpr (Tab::FIXED) {
+        err = 0.0;
+    } else {
+        double e[N];
+        bool first = true;
+#pragma unroll
+        for (int j = 0; j < NS; j++)
+            if (Tab::e(j) != 0.0) {
+                const MulR c = coef_right(Tab::e(j), h);
+#pragma unroll
+                for (int i = 0; i < N; i++) {
+                    const double term = mul_rn(K[j][i], c);
+                    e[i] = first ? term : e[i] + term;
+                }
+                first = false;
+            }
+        if constexpr (Tab::FSAL) {
+            model_rhs64<M>(ynew, p, t + dt, knew, r);
+            const MulR c = coef_right(Tab::E_NEW, h);
+#pragma unroll
+            for (int i = 0; i < N; i++)
+                e[i] = e[i] + mul_rn(mul_left(knew[i], r), c);
+        }
+        // odeint's rel_error + norm_inf: one quotient per component, then max
+        const MulR ah = {h.h, h.l, h.e & 0x7fffffffu};
+        const MulL rt = mul_left(rtol, r);
+        err = 0.0;
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const MulL ak = {K[0][i].h, K[0][i].l, K[0][i].e & 0x7fffffffu};
+            const double s = fabs(y[i]) + mul_rn(ak, ah);
+            err = max_nonneg64(err, quotient64(fabs(e[i]), atol + mul_rn(rt, mul_right(s, r))));
+        }
+    }
+    return !r.beyond(kChainRange) && !neg_zero && !is_nan64(err);
+}
+
+// acc + (a zero with the given sign bit)
+__host__ __device__ __forceinline__ double add_zero64(double acc, uint32_t sign)
+{
+    return f64_bits(acc) == 1ull << 63 && !(sign & 0x80000000u) ? 0.0 : acc;
+}
+
+// back_step for double stages: lambda_n in ybar, mu's new sums in ms.  False:
+// out of range.
+template <class M, class Tab>
+__host__ __device__ __forceinline__ bool back_step64(const double (&y)[M::N], double tn, double hh,
+                                                     const double (&p)[M::P], const double (&lam)[M::N],
+                                                     const double (&mu)[M::PG], double (&ybar)[M::N],
+                                                     double (&ms)[M::PG])
+{
+    constexpr int N = M::N, P = M::PG, NS = Tab::S;
+    MulRange r;
+    const MulR h = mul_right(hh, r);
+    double X[NS][N];
+    bool neg_zero = false;
+    {
+        MulL K[NS][N];
+#pragma unroll
+        for (int m = 0; m < NS; m++) {
+            form_stage64<Tab, N>(m, y, K, h, X[m]);
+            if (m < NS - 1) {
+                double f[N];
+                model_rhs64<M>(X[m], p, tn + Tab::c(m) * hh, f, r);
+#pragma unroll
+                for (int i = 0; i < N; i++)
+                    K[m][i] = mul_left(f[i], r);
+            }
+        }
+        if (zero_in_a<Tab>()) {
+#pragma unroll
+            for (int i = 0; i < N; i++)
+                neg_zero = neg_zero || f64_bits(y[i]) == 1ull << 63;
+        }
+    }
+    double Kbar[NS][N];
+    MulL l[N];
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        ybar[i] = lam[i];
+        l[i] = mul_left(lam[i], r);
+    }
+#pragma unroll
+    for (int k = 0; k < P; k++)
+        ms[k] = mu[k];
+#pragma unroll
+    for (int m = 0; m < NS; m++) {
+        const MulR bh = coef_right(Tab::b(m), h);
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            Kbar[m][i] = Tab::b(m) != 0.0 ? mul_rn(l[i], bh)
+                                          : f64_from_bits((uint64_t)((l[i].e ^ h.e) & 0x80000000u) << 32);
+    }
+#pragma unroll
+    for (int m = NS - 1; m >= 0; m--) {
+        double gx[N], gp[P];
+        model_vjp64<M>(Kbar[m], X[m], p, tn + Tab::c(m) * hh, gx, gp, r);
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            ybar[i] += gx[i];
+            if (m == 0)
+                continue;
+            const MulL g = mul_left(gx[i], r);
+#pragma unroll
+            for (int k = 0; k < NS - 1; k++)
+                if (k < m) {
+                    if (Tab::a(m, k) != 0.0)
+                        Kbar[k][i] += mul_rn(mul_left_in(mul_rn(g, mul_right_in(Tab::a(m, k)))), h);
+                    else
+                        Kbar[k][i] = add_zero64(Kbar[k][i], g.e ^ h.e);
+                }
+        }
+#pragma unroll
+        for (int k = 0; k < P; k++)
+            ms[k] += gp[k];
+    }
+    return !r.beyond(kChainRange) && !neg_zero;
+}
+
+} // namespace va
