@@ -46,14 +46,14 @@ def check(oracle, model, tab, y0, p, t1, picks, stride=0, tol=1e-6):
 
 @pytest.mark.parametrize("model", sorted(NP))
 @pytest.mark.parametrize("tab", ["dopri5", "ck54", "rkf78"])
-@pytest.mark.parametrize("B", [1, 33, 1217, 5000])
+@pytest.mark.parametrize("B", [1, 33, 1217, 2433, 5000, 9800])
 def test_paths_bit_exact(oracle, cuda, model, tab, B):
     y0, p, t1 = draw(model, B, B)
     check(oracle, model, tab, y0, p, t1, sorted({0, B // 2, B - 1, min(31, B - 1), min(1216, B - 1)}))
 
 
 @pytest.mark.parametrize("tab,stride", [("dopri5", 0), ("ck54", 0), ("rkf78", 0), ("dopri5", 3)])
-@pytest.mark.parametrize("B", [7, 6000])
+@pytest.mark.parametrize("B", [7, 1300, 3000, 6000, 10000])
 def test_special_values_bit_exact(oracle, cuda, tab, stride, B):
     """Linear oscillators: zeros, both signs, no damping, no frequency, and magnitudes across and beyond the range of the
     integer products (the other instances of the same warp stay on it)."""
@@ -67,4 +67,29 @@ def test_special_values_bit_exact(oracle, cuda, tab, stride, B):
         p[21] = (0.0, 0.3)
         p[22] = (1e-80, 0.1)
         p[23], t1[23] = (1e3, 0.0), 0.05
-    check(oracle, "dho", tab, y0, p, t1, range(min(B, 40)), stride)
+    check(oracle, "dho", tab, y0, p, t1, range(min(B, 26)), stride)
+
+
+@pytest.mark.parametrize("tab", ["dopri5", "rkf78"])
+@pytest.mark.parametrize("stride", [0, 5])
+@pytest.mark.parametrize("B", [3, 1300])
+def test_team_seeds_history_and_refill(oracle, cuda, tab, stride, B):
+    """Teams with several seeds, direct parameter gradients, the adjoint history, and fewer resident teams than instances
+    (64-thread blocks, one per SM for a batch of more): the bits of single-seed calls on a batch that every lane path
+    takes, and of the one-lane sweeps (a block size that teams do not take)."""
+    y0, p, t1 = draw("vdp", B, 9)
+    rng = np.random.default_rng(3)
+    lam, mud = rng.standard_normal((B, 2, 2)), rng.standard_normal((B, 2, 1))
+    res = []
+    for block, bps in ((0, 0), (64, 1), (48, 0)):
+        s = Solver("vdp", 2, 1, B, nout=2, tableau=tab, atol=1e-6, rtol=1e-6, ckpt_stride=stride, block_size=block,
+                   blocks_per_sm=bps)
+        s.set_adjoint_history(4)
+        f = s.forward(dev(y0), dev(p), dev(np.zeros(B)), dev(t1))
+        g = s.backward(dev(p), dev(lam), dev(mud))
+        hist = s.adjoint_history(B - 1, times=False)[1]
+        res.append([v.cpu().numpy() for v in (f["yT"], f["n_acc"], f["n_rej"], g["status"], g["dy0"], g["dp"])] + [hist])
+        s.close()
+    for r in res[:2]:
+        for a, b in zip(r, res[2]):
+            np.testing.assert_array_equal(a, b)

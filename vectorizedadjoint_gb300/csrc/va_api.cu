@@ -56,7 +56,10 @@ struct va_handle {
     int sm_count = 0;
     const va::KernelSet *ks = nullptr;
     const va::ModelKernels *user = nullptr; // a device model compiled outside the library
-    const void *sw_fwd = nullptr, *sw_bwd = nullptr; // FP64 sweeps in the place of the table's (fp64_path)
+    // FP64 sweeps in the place of the table's (fp64_path): every-step sweeps
+    // and the two-level backward; the lanes that carry one instance in them
+    const void *sw_fwd = nullptr, *sw_bwd = nullptr, *sw_bwd2 = nullptr;
+    int lanes = 1;
     int bps = 0; // resident blocks per SM of the default launch shape (0: the occupancy limit)
     int N = 0, P = 0;
     int RS = 0; // doubles per checkpoint record at the current stride (record_layout)
@@ -195,26 +198,56 @@ const void *bwd_kernel(const va_handle *h)
     return h->sw_bwd ? h->sw_bwd : h->ks->bwd[h->opt.tableau][h->opt.precision];
 }
 
-// FP64 sweeps of the built-in one-thread models: products on the integer
-// pipe for the 5(4) pairs.  The FP64 unit bounds these sweeps; with the
-// products off it, Van der Pol with 65,536 instances takes 9.2 ms against
-// 19.6 ms, and a single instance 3.7 ms against 4.4 ms.  Fehlberg 7(8) and
-// the two-level backward keep the FP64 products: their code is too long for
-// the instruction caches that way (measured 16.1 against 9.8 ms with 5,003
-// instances, and 24.7 against 14.0 ms with 9,001).
+// FP64 sweeps of the built-in one-thread models, by the batch size.
 //
-// Launch shape: one block per SM, of 256 threads (two warps on each quadrant
-// to overlap integer and FP64 work) when the batch fills them, else of 128.
-// More resident warps only spread the instruction fetch: 65,536 instances
-// 9.2 ms with 256 x 1, 10.7 with 128 x 2, 12.3 with 128 x 4 and with 128 x 1;
-// 30,000 instances 7.0 ms with 256 x 1, 6.8 with 128 x 1.
+// Teams (va_team64.cuh): the widest whose warps do not outnumber the quadrants
+// (4 per SM), since a second warp on a quadrant would share its FP64 unit.
+// Forward + backward, Van der Pol T = 20, ms with teams of 16 / 8 / 4 / 2 lanes
+// and with one lane (integer products):
+//     B = 1,216   2.50 / 3.16 / 3.99 / 5.03   5.11
+//     B = 2,400   3.67 / 3.18 / 3.99 / 5.04   5.11
+//     B = 4,800   6.57 / 4.74 / 4.00 / 5.02   5.05
+//     B = 9,600   9.42 / 8.39 / 6.25 / 5.06   5.20
+//     B = 19,000  16.9 / 12.3 / 10.2 / 8.15   5.77
+// Fehlberg 7(8) (32 / 16 / 8 lanes, one lane with FP64 products): 600: 2.52 /
+// 3.18 / 3.94, 9.52; 1,200: 3.93 / 3.22 / 3.96, 9.61; 5,003: 8.53 / 7.74 / 6.45,
+// 9.79; 9,600: 14.5 / 9.58 / 7.31, 9.84; 19,000: 28.4 / 18.0 / 12.1, 9.87 -- its
+// narrowest team serves up to four warps per quadrant.
+//
+// Larger batches: products on the integer pipe for the 5(4) pairs
+// (va_step64.cuh); Van der Pol with 65,536 instances 9.2 ms against 19.6 ms
+// with FP64 products.  Fehlberg 7(8) and the two-level backward keep the FP64
+// products there: their code is too long for the instruction caches that way
+// (16.1 against 9.8 ms with 5,003 instances, 24.7 against 14.0 ms with 9,001).
+// One block per SM, of 256 threads (two warps on each quadrant to overlap
+// integer and FP64 work) when the batch fills them, else of 128; more resident
+// warps only spread the instruction fetch: 65,536 instances 9.2 ms with 256 x
+// 1, 10.7 with 128 x 2, 12.3 with 128 x 4 and with 128 x 1; 30,000 instances
+// 7.0 ms with 256 x 1, 6.8 with 128 x 1.
 void fp64_path(va_handle *h)
 {
+    h->lanes = h->ks ? h->ks->tpi : 1;
     const va::Fp64Kernels *k = h->user || !h->ks ? nullptr : va::fp64_kernels(h->prob.model);
-    if (!k || h->opt.precision != VA_PREC_FP64 || !k->int_fwd[h->opt.tableau])
+    if (!k || h->opt.precision != VA_PREC_FP64)
         return;
-    h->sw_fwd = k->int_fwd[h->opt.tableau];
-    h->sw_bwd = k->int_bwd[h->opt.tableau];
+    const int t = h->opt.tableau;
+    const int64_t lanes = 128LL * h->sm_count; // one warp on every quadrant
+    if (h->opt.block_size <= 0 || h->opt.block_size % 32 == 0) { // a team's lanes share a warp
+        for (const va::TeamKernels &w : k->team[t]) {
+            const int per_quadrant = t == VA_TAB_RKF78 && w.g == 8 ? 4 : 1;
+            if (w.g && (int64_t)h->prob.batch * w.g <= per_quadrant * lanes) {
+                h->lanes = w.g;
+                h->sw_fwd = w.fwd;
+                h->sw_bwd = w.bwd;
+                h->sw_bwd2 = w.bwd2;
+                return;
+            }
+        }
+    }
+    if (!k->int_fwd[t])
+        return;
+    h->sw_fwd = k->int_fwd[t];
+    h->sw_bwd = k->int_bwd[t];
     if (h->opt.block_size <= 0 && h->opt.blocks_per_sm <= 0) {
         h->fwd_block = h->bwd_block = h->prob.batch > 256 * h->sm_count ? 256 : 128;
         h->bps = 1;
@@ -229,7 +262,7 @@ int grid_for(va_handle *h, const void *fn, int block, int instances)
     int bps = h->opt.blocks_per_sm > 0 ? std::min(h->opt.blocks_per_sm, occ) : occ;
     if (h->bps > 0)
         bps = std::min(bps, h->bps);
-    long need = ((long)instances * h->ks->tpi + block - 1) / block;
+    long need = ((long)instances * h->lanes + block - 1) / block;
     long g = (long)h->sm_count * bps;
     return (int)std::max(1L, std::min(g, need));
 }
@@ -478,12 +511,15 @@ int bundle_grid(va_handle *h)
 constexpr int kTwoLevelBlock = 64, kTwoLevelBlocksPerSm = 4;
 constexpr int kTwoLevelGroupBlock = 256, kTwoLevelGroupBlocksPerSm = 2;
 
+// Teams (sw_bwd2): the same blocks, kTwoLevelBlock / lanes instances each.
 int two_level_block(const va_handle *h) { return h->ks->tpi > 1 ? kTwoLevelGroupBlock : kTwoLevelBlock; }
 
 // instances one block of the two-level backward carries at once
 int two_level_per_block(const va_handle *h)
 {
     const int g = h->ks->tpi;
+    if (h->sw_bwd2)
+        return kTwoLevelBlock / h->lanes;
     return g > 1 ? kTwoLevelGroupBlock / 32 * (32 / g) : kTwoLevelBlock;
 }
 
@@ -771,7 +807,8 @@ va_status enqueue_backward(va_handle *h, const double *params, const double *lam
         a.max_fail = h->opt.max_rejects;
         a.step_pow = h->opt.step_pow;
         VA_CUDA(h, cudaMemsetAsync(&h->ctl->adj_next, 0, sizeof(unsigned int), s));
-        VA_CUDA(h, launch(h, h->ks->bwd2[h->opt.tableau][h->opt.precision], two_level_grid(h), two_level_block(h),
+        VA_CUDA(h, launch(h, h->sw_bwd2 ? h->sw_bwd2 : h->ks->bwd2[h->opt.tableau][h->opt.precision],
+                          two_level_grid(h), two_level_block(h),
                           &a, s));
         return VA_OK;
     }
@@ -807,7 +844,7 @@ struct TunedShape {
 int grid_of(va_handle *h, const void *fn, int block, int bps)
 {
     const int occ = std::max(1, occupancy_of(h, fn, block));
-    const long need = ((long)h->prob.batch * h->ks->tpi + block - 1) / block;
+    const long need = ((long)h->prob.batch * h->lanes + block - 1) / block;
     return (int)std::max(1L, std::min((long)h->sm_count * std::min(bps, occ), need));
 }
 

@@ -95,6 +95,15 @@ struct ModelVdP {
         gx[1] = w[0] + mul_rn(w1, mul_right_in(mul_rn(al, mu)));
         gp[0] = mul_rn(w1, mul_right_in(mul_rn(al, x1)));
     }
+    // vjp's outputs as w[kVjpW] W_o (+ w[0] for o = kVjpAdd)
+    static constexpr int kVjpW = 1, kVjpAdd = 1;
+    __host__ __device__ __forceinline__ static void vjp_weights(const double *x, const double *p, double *W)
+    {
+        const double a = 1.0 - x[0] * x[0];
+        W[0] = -2.0 * p[0] * x[0] * x[1] - 1.0;
+        W[1] = p[0] * a;
+        W[2] = a * x[1];
+    }
 };
 
 // Van der Pol as in the reference example (examples/VanDerPol/main.cpp:41-42):
@@ -146,6 +155,14 @@ struct ModelVdPPetsc {
         gx[0] = mul_rn(w1, mul_right_in(c));
         gx[1] = w[0] + mul_rn(w1, mul_right_in(mul_rn(al, mu)));
         gp[0] = mul_rn(w1, mul_right_in(ax - x[0]));
+    }
+    static constexpr int kVjpW = 1, kVjpAdd = 1;
+    __host__ __device__ __forceinline__ static void vjp_weights(const double *x, const double *p, double *W)
+    {
+        const double a = 1.0 - x[0] * x[0];
+        W[0] = p[0] * (-2.0 * x[0] * x[1] - 1.0);
+        W[1] = p[0] * a;
+        W[2] = a * x[1] - x[0];
     }
 };
 
@@ -206,6 +223,15 @@ struct ModelDHO {
         gp[0] = mul_rn(w1, mul_right_in(mul_rn(mul_m2(om), x0) + mul_rn(mul_m2(ze), x1)));
         gp[1] = mul_rn(w1, mul_right_in(mul_rn(mul_m2(om), x1)));
     }
+    static constexpr int kVjpW = 1, kVjpAdd = 1;
+    __host__ __device__ __forceinline__ static void vjp_weights(const double *x, const double *p, double *W)
+    {
+        const double om = p[0], ze = p[1];
+        W[0] = -om * om;
+        W[1] = -2.0 * ze * om;
+        W[2] = -2.0 * om * x[0] - 2.0 * ze * x[1];
+        W[3] = -2.0 * om * x[1];
+    }
 };
 
 // Exponential decay y' = -k y; p = (k).  Its discrete adjoint has a closed
@@ -236,6 +262,12 @@ struct ModelDecay {
         const MulR wr = mul_right(w[0], r);
         gx[0] = mul_rn(mul_neg(mul_left(p[0], r)), wr);
         gp[0] = mul_rn(mul_neg(mul_left(x[0], r)), wr);
+    }
+    static constexpr int kVjpW = 0, kVjpAdd = -1;
+    __host__ __device__ __forceinline__ static void vjp_weights(const double *x, const double *p, double *W)
+    {
+        W[0] = -p[0];
+        W[1] = -x[0];
     }
 };
 

@@ -89,10 +89,26 @@ void fill_fixed_glv5(KernelSet &k);
 void fill_fixed_glv10(KernelSet &k);
 
 // Further FP64 sweeps of a built-in one-thread model (fp64_path in va_api.cu
-// chooses): products on the integer pipe (va_step64.cuh).  Null: not compiled.
+// chooses): products on the integer pipe (va_step64.cuh) and teams of g lanes
+// per instance (va_team64.cuh).  Null: not compiled.
+struct TeamKernels {
+    int g;
+    const void *fwd, *bwd, *bwd2; // bwd2: two-level backward
+};
+constexpr int kTeams = 4;
 struct Fp64Kernels {
     const void *int_fwd[kTableaux], *int_bwd[kTableaux];
+    TeamKernels team[kTableaux][kTeams]; // widest first
 };
+// the team sweeps (va_inst_team_fp64.cu, va_inst_team_rkf78_fp64.cu)
+void fill_team_vdp(Fp64Kernels &k);
+void fill_team_vdp_petsc(Fp64Kernels &k);
+void fill_team_dho(Fp64Kernels &k);
+void fill_team_decay(Fp64Kernels &k);
+void fill_team_rkf78_vdp(Fp64Kernels &k);
+void fill_team_rkf78_vdp_petsc(Fp64Kernels &k);
+void fill_team_rkf78_dho(Fp64Kernels &k);
+void fill_team_rkf78_decay(Fp64Kernels &k);
 const Fp64Kernels *fp64_kernels(int model); // null: none for the model
 
 // Shared-matrix GLV: bundles of kBundleNB instances per CTA of N threads

@@ -1,0 +1,926 @@
+// FP64 sweeps for small batches: one instance is carried by a team of G lanes.
+//
+// An FP64 instruction takes its SM quadrant's FP64 unit for 64 cycles however
+// many lanes are active and however independent its neighbours are
+// (va_int64.cuh), so with one warp on a quadrant the time of a step is its
+// FP64 instruction count: a lane that carries an instance alone issues ~230
+// of them per attempt of a 5(4) pair (two components) while the other 31
+// lanes, or the other quadrants, have nothing to do.  A team spreads what is
+// independent: lane l keeps the running sums of one (row, component) pair,
+// the rows being the stages X_1 .. X_{s-1}, the new state, the error estimate
+// and the error's denominator; a stage's slope K_j, once known to every lane,
+// is then added to all rows with one product and one sum.  The right-hand
+// side and the controller run on every lane alike.  ~60 FP64 instructions per
+// attempt (G = 16) instead of ~230, and the same bits: every (row, component)
+// sum takes the terms of form_stage / attempt_pair in their order.
+//
+// The backward step is spread the same way: the rows are the stage values'
+// recompute, then K-bar_0 .. K-bar_{s-1}, lambda and mu; where a model gives
+// its VJP as weights, those of all stages are formed at once, a lane a stage:
+// ~80 FP64 instructions per step instead of ~290 (127 without the weights).
+//
+// Measured: one Van der Pol instance 4.4 ms (a lane, FP64 products) -> 2.0 ms;
+// 1,216 instances 6.2 -> 2.5 ms; Fehlberg 7(8), 600 instances 9.5 -> 2.5 ms;
+// two-level backward, 600 instances 11.2 -> 3.6 ms.  What is left is the
+// latency of a step's chain (right-hand side, one product and one sum per
+// stage, the shuffles between them, the step factor): the FP64 unit is busy
+// about half the time.
+#pragma once
+
+#include "va_group.cuh"
+
+namespace va {
+
+// Rows of the forward sums.  Order (rank): y_new, error, X_{s-1} .. X_1,
+// error denominator; a fixed-step tableau has no error rows.  Slot
+// rank * N + i is kept by lane slot % G as its accumulator slot / G.
+template <class Tab, int N, int G>
+struct TeamRows {
+    static constexpr int NS = Tab::S;
+    static constexpr int E = Tab::FIXED ? 0 : 1;
+    static constexpr int R = NS + 2 * E;
+    static constexpr int Q = (R * N + G - 1) / G;
+    static constexpr int rank_b = 0, rank_e = 1, rank_d = R - 1;
+    __host__ __device__ static constexpr int rank_x(int m) { return E + NS - m; }
+    // weight of K_j in the row (the denominator's 1 |K_0|)
+    __host__ __device__ static constexpr double coef(int rank, int j)
+    {
+        if (rank == rank_b)
+            return j < NS ? Tab::b(j) : 0.0;
+        if (E && rank == rank_e) {
+            if constexpr (!Tab::FIXED)
+                return j < NS ? Tab::e(j) : Tab::E_NEW;
+            return 0.0;
+        }
+        if (E && rank == rank_d)
+            return j == 0 ? 1.0 : 0.0;
+        const int m = E + NS - rank;
+        return j < m && j < NS ? Tab::a(m, j) : 0.0;
+    }
+    // whether the row takes a term at j: the stages take every j < m (their
+    // zero coefficients included, as form_stage), y_new and the error the
+    // non-zero ones, the denominator its two
+    __host__ __device__ static constexpr bool used(int rank, int j)
+    {
+        if (rank == rank_b || (E && rank == rank_e))
+            return coef(rank, j) != 0.0;
+        if (E && rank == rank_d)
+            return j <= 1;
+        return j < E + NS - rank;
+    }
+    __host__ __device__ static constexpr bool any_used(int q, int j)
+    {
+        for (int s = q * G; s < (q + 1) * G && s < R * N; s++)
+            if (used(s / N, j))
+                return true;
+        return false;
+    }
+    __host__ __device__ static constexpr bool has(int q, int rank)
+    {
+        for (int i = 0; i < N; i++)
+            if ((rank * N + i) / G == q)
+                return true;
+        return false;
+    }
+};
+
+// The rows' weights by lane, read once per kernel.
+template <class Tab, int N, int G>
+struct TeamForwardTable {
+    using Rows = TeamRows<Tab, N, G>;
+    static constexpr int J = Tab::FIXED ? Tab::S : Tab::S + 1, W = Rows::Q * G;
+    double c[J][W];
+    unsigned use[W];
+    __host__ __device__ constexpr TeamForwardTable() : c(), use()
+    {
+        for (int s = 0; s < Rows::R * N; s++)
+            for (int j = 0; j < J; j++) {
+                c[j][s] = Rows::coef(s / N, j);
+                use[s] |= Rows::used(s / N, j) ? 1u << j : 0u;
+            }
+    }
+};
+template <class Tab, int N, int G>
+__device__ constexpr TeamForwardTable<Tab, N, G> kTeamForward{};
+
+// v[i] for a lane-dependent i without a local array
+template <int N>
+__device__ __forceinline__ double pick(const double (&v)[N], int i)
+{
+    double r = v[0];
+#pragma unroll
+    for (int k = 1; k < N; k++)
+        r = i == k ? v[k] : r;
+    return r;
+}
+
+// A lane's part of the forward sums: its rows' coefficients, and which of
+// them it holds.
+template <class M, class Tab, int G>
+struct TeamForward {
+    static constexpr int N = M::N, NS = Tab::S;
+    using Rows = TeamRows<Tab, N, G>;
+    static constexpr int Q = Rows::Q, J = Tab::FIXED ? NS : NS + 1;
+    double c[J][Q];
+    int comp[Q];
+    unsigned use[Q];      // bit j: the row takes a term at j
+    bool err[Q], den[Q];  // the error row, its denominator
+    LaneGroup<G> team;
+
+    __device__ __forceinline__ TeamForward()
+    {
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+            const int s = team.index + G * q;
+            comp[q] = s % N;
+            use[q] = kTeamForward<Tab, N, G>.use[s];
+            err[q] = Rows::E && s / N == Rows::rank_e;
+            den[q] = Rows::E && s / N == Rows::rank_d;
+#pragma unroll
+            for (int j = 0; j < J; j++)
+                c[j][q] = kTeamForward<Tab, N, G>.c[j][s];
+        }
+    }
+
+    // component i of a row, to every lane
+    __device__ __forceinline__ double row(const double (&acc)[Q], int rank, int i) const
+    {
+        const int s = rank * N + i;
+        return shfl(acc[s / G], team.base + s % G, team.mask);
+    }
+
+    // acc += (c_j dt) K_j for every row that takes the term
+    __device__ __forceinline__ void add(double (&acc)[Q], int j, const double (&K)[N], double dt, double atol,
+                                        double rtol) const
+    {
+#pragma unroll
+        for (int q = 0; q < Q; q++)
+            if (Rows::any_used(q, j)) {
+                double w = c[j][q] * dt, k = pick<N>(K, comp[q]), s = acc[q];
+                const bool dq = Rows::E && Rows::has(q, Rows::rank_d);
+                if (dq && j == 1) { // the denominator's atol + rtol (|y| + |dt K_0|)
+                    w = den[q] ? rtol : w;
+                    k = den[q] ? s : k;
+                    s = den[q] ? atol : s;
+                }
+                double term = w * k;
+                if (dq && j == 0)
+                    term = den[q] ? fabs(term) : term;
+                s = s + term;
+                // rows that must not take the term: y_new and the error where
+                // their weight is zero, the denominator; a finished stage is
+                // not read again
+                const bool keep = Rows::has(q, Rows::rank_b) || (Rows::E && Rows::has(q, Rows::rank_e)) || dq;
+                acc[q] = !keep || (use[q] >> j & 1u) ? s : acc[q];
+            }
+    }
+
+    // attempt_pair / step_fixed, the results on every lane
+    __device__ __forceinline__ double attempt(const double (&y)[N], const double (&k0)[N], const double (&p)[M::P],
+                                              double t, double dt, double atol, double rtol, double (&ynew)[N],
+                                              double (&knew)[N]) const
+    {
+        double acc[Q];
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+            acc[q] = pick<N>(y, comp[q]);
+            if (Rows::E && Rows::has(q, Rows::rank_d))
+                acc[q] = den[q] ? fabs(acc[q]) : acc[q];
+            if (Rows::E && Rows::has(q, Rows::rank_e))
+                acc[q] = err[q] ? -0.0 : acc[q]; // -0 + x = x: the first term
+        }
+        add(acc, 0, k0, dt, atol, rtol);
+#pragma unroll
+        for (int m = 1; m < NS; m++) {
+            double X[N], K[N];
+#pragma unroll
+            for (int i = 0; i < N; i++)
+                X[i] = row(acc, Rows::rank_x(m), i);
+            M::template rhs<double>(X, p, t + Tab::c(m) * dt, K);
+            add(acc, m, K, dt, atol, rtol);
+        }
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            ynew[i] = row(acc, Rows::rank_b, i);
+        if constexpr (Tab::FIXED) {
+            return 0.0;
+        } else {
+            if constexpr (Tab::FSAL) {
+                M::template rhs<double>(ynew, p, t + dt, knew);
+                add(acc, NS, knew, dt, atol, rtol);
+            }
+            double worst = 0.0;
+            if constexpr (Q == 1) {
+                // every lane forms the quotient of its own component, the
+                // error rows' ones are those of the components
+                const int from = team.base + (Rows::rank_e * N + comp[0]) % G;
+                const int dfrom = team.base + (Rows::rank_d * N + comp[0]) % G;
+                const double e = shfl(acc[0], from, team.mask), d = shfl(acc[0], dfrom, team.mask);
+                const double r = quotient64(fabs(e), d);
+#pragma unroll
+                for (int i = 0; i < N; i++)
+                    worst = worse(worst, shfl(r, team.base + i, team.mask));
+            } else {
+#pragma unroll
+                for (int i = 0; i < N; i++)
+                    worst = worse(worst, quotient64(fabs(row(acc, Rows::rank_e, i)), row(acc, Rows::rank_d, i)));
+            }
+            return worst;
+        }
+    }
+    // the larger, a NaN kept
+    __device__ __forceinline__ static double worse(double a, double b)
+    {
+        return is_nan64(a) ? a : is_nan64(b) ? b : max_nonneg64(a, b);
+    }
+};
+
+template <class M, class = void>
+struct HasVjpWeights : std::false_type {
+};
+template <class M>
+struct HasVjpWeights<M, std::void_t<decltype(M::kVjpW)>> : std::true_type {
+};
+
+template <class Tab, int N, int P, int G>
+struct TeamBackwardTable {
+    static constexpr int NS = Tab::S, SLOTS = N + P + NS * N, W = (SLOTS + G - 1) / G * G;
+    static constexpr int XSLOTS = (NS - 1) * N, XW = XSLOTS ? (XSLOTS + G - 1) / G * G : G;
+    double ca[NS][W], cb[W], cx[NS][XW];
+    __host__ __device__ constexpr TeamBackwardTable() : ca(), cb(), cx()
+    {
+        for (int s = N + P; s < SLOTS; s++) {
+            const int k = (s - N - P) / N;
+            cb[s] = Tab::b(k);
+            for (int m = k + 1; m < NS; m++)
+                ca[m][s] = Tab::a(m, k);
+        }
+        for (int s = 0; s < XSLOTS; s++)
+            for (int j = 0; j < NS - 1 - s / N; j++)
+                cx[j][s] = Tab::a(NS - 1 - s / N, j);
+    }
+};
+template <class Tab, int N, int P, int G>
+__device__ constexpr TeamBackwardTable<Tab, N, P, G> kTeamBackward{};
+
+// Rows of the backward sums.  Slots: lambda (N), mu (P), then K-bar_k
+// component i at N + P + k N + i.
+template <class M, class Tab, int G>
+struct TeamBackward {
+    static constexpr int N = M::N, P = M::PG, NS = Tab::S;
+    static constexpr int SLOTS = N + P + NS * N, Q = (SLOTS + G - 1) / G;
+    static constexpr int XQ = ((NS - 1) * N + G - 1) / G; // stage rows X_{s-1} .. X_1
+    static constexpr int XQ1 = XQ > 0 ? XQ : 1;
+    // Models whose VJP outputs o (gx, then gp) are w[kVjpW] W_o(x), plus w[0]
+    // for o = kVjpAdd: the weights W of all stages are formed at once, lane l
+    // taking stage l, and each lane then forms only its own row's output.
+    static constexpr bool WEIGHTS = HasVjpWeights<M>::value;
+    static constexpr int WQ = (NS + G - 1) / G;
+    double ca[NS][Q]; // a_mk of the lane's K-bar_k
+    double cb[Q];     // b_k
+    double cx[NS][XQ1]; // a_mj of the lane's stage m
+    int kind[Q];      // 0 lambda, 1 mu, 2 K-bar
+    int comp[Q];      // component (lambda, K-bar) or parameter (mu)
+    int xcomp[XQ1];
+    LaneGroup<G> team;
+
+    __device__ __forceinline__ TeamBackward()
+    {
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+            const int s = team.index + G * q;
+            kind[q] = s < N ? 0 : s < N + P ? 1 : 2;
+            comp[q] = s < N ? s : s < N + P ? s - N : (s - N - P) % N;
+            cb[q] = kTeamBackward<Tab, N, P, G>.cb[s];
+#pragma unroll
+            for (int m = 0; m < NS; m++)
+                ca[m][q] = kTeamBackward<Tab, N, P, G>.ca[m][s];
+        }
+#pragma unroll
+        for (int q = 0; q < XQ1; q++) {
+            const int s = team.index + G * q;
+            xcomp[q] = s % N;
+#pragma unroll
+            for (int j = 0; j < NS; j++)
+                cx[j][q] = kTeamBackward<Tab, N, P, G>.cx[j][s];
+        }
+    }
+
+    // Whether accumulator q holds a row that stage m adds to
+    __host__ __device__ static constexpr bool live(int q, int m)
+    {
+        for (int s = q * G; s < (q + 1) * G && s < SLOTS; s++)
+            if (s < N + P || (s - N - P) / N < m)
+                return true;
+        return false;
+    }
+    __host__ __device__ static constexpr bool only_kbar(int q) { return q * G >= N + P; }
+    __host__ __device__ static constexpr bool only_sums(int q, int m)
+    {
+        for (int s = q * G; s < (q + 1) * G && s < SLOTS; s++)
+            if (s >= N + P && (s - N - P) / N < m)
+                return false;
+        return true;
+    }
+
+    // mu into its lanes, at the start of a seed
+    __device__ __forceinline__ void clear(double (&mu)[Q]) const
+    {
+#pragma unroll
+        for (int q = 0; q < Q; q++)
+            mu[q] = 0.0;
+    }
+    __device__ __forceinline__ double param(const double (&mu)[Q], int k) const
+    {
+        return shfl(mu[(N + k) / G], team.base + (N + k) % G, team.mask);
+    }
+
+    // back_step: lam on every lane, mu in its lanes
+    __device__ __forceinline__ void step(const double (&y)[N], double tn, double h, const double (&p)[M::P],
+                                         double (&lam)[N], double (&mu)[Q]) const
+    {
+        double X[NS][N];
+        {
+            double acc[XQ1];
+#pragma unroll
+            for (int q = 0; q < XQ1; q++)
+                acc[q] = pick<N>(y, xcomp[q]);
+#pragma unroll
+            for (int i = 0; i < N; i++)
+                X[0][i] = y[i];
+#pragma unroll
+            for (int m = 0; m < NS - 1; m++) {
+                double K[N];
+                M::template rhs<double>(X[m], p, tn + Tab::c(m) * h, K);
+#pragma unroll
+                for (int q = 0; q < XQ1; q++)
+                    if (q * G < (NS - 1 - m) * N) // a stage after m among them
+                        acc[q] = acc[q] + (cx[m][q] * h) * pick<N>(K, xcomp[q]);
+#pragma unroll
+                for (int i = 0; i < N; i++) {
+                    const int s = (NS - 2 - m) * N + i;
+                    X[m + 1][i] = shfl(acc[s / G], team.base + s % G, team.mask);
+                }
+            }
+        }
+        double acc[Q];
+#pragma unroll
+        for (int q = 0; q < Q; q++) {
+            const double l = pick<N>(lam, comp[q]);
+            acc[q] = (cb[q] * h) * l; // seeds K-bar_k = (b_k h) lambda
+            if (!only_kbar(q))
+                acc[q] = kind[q] == 2 ? acc[q] : kind[q] == 0 ? l : mu[q];
+        }
+double W[WQ][N + P]; // VJP weights of stage team.index + G r
+        if constexpr (WEIGHTS) {
+#pragma unroll
+            for (int r = 0; r < WQ; r++) {
+                double Xl[N];
+#pragma unroll
+                for (int i = 0; i < N; i++) {
+                    Xl[i] = X[G * r][i];
+#pragma unroll
+                    for (int m = G * r + 1; m < NS; m++)
+                        Xl[i] = team.index + G * r == m ? X[m][i] : Xl[i];
+                }
+                M::vjp_weights(Xl, p, W[r]);
+            }
+        }
+#pragma unroll
+        for (int m = NS - 1; m >= 0; m--) {
+            double w[N], gx[N], gp[P], Wm[N + P];
+#pragma unroll
+            for (int i = 0; i < N; i++) {
+                const int s = N + P + m * N + i;
+                w[i] = shfl(acc[s / G], team.base + s % G, team.mask);
+            }
+            if constexpr (WEIGHTS) {
+#pragma unroll
+                for (int o = 0; o < N + P; o++)
+                    Wm[o] = shfl(W[m / G][o], team.base + m % G, team.mask);
+            } else {
+                M::template vjp<double>(w, X[m], p, tn + Tab::c(m) * h, gx, gp);
+            }
+#pragma unroll
+            for (int q = 0; q < Q; q++)
+                if (live(q, m)) {
+                    double g; // the row's VJP output: gx of its component, or gp
+                    if constexpr (WEIGHTS) {
+                        const int o = kind[q] == 1 ? N + comp[q] : comp[q];
+                        g = w[M::kVjpW] * pick<N + P>(Wm, o);
+                        if constexpr (M::kVjpAdd >= 0)
+                            g = o == M::kVjpAdd ? w[0] + g : g;
+                    } else {
+                        g = pick<N>(gx, comp[q]);
+                        if (!only_kbar(q))
+                            g = kind[q] == 1 ? pick<P>(gp, comp[q]) : g;
+                    }
+                    // K-bar_k + (gx a_mk) h; a row k >= m is not read again
+                    double term = only_sums(q, m) ? g : (g * ca[m][q]) * h;
+                    if (!only_kbar(q))
+                        term = kind[q] == 2 ? term : g;
+                    acc[q] = acc[q] + term;
+                }
+        }
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            lam[i] = shfl(acc[i / G], team.base + i % G, team.mask);
+#pragma unroll
+        for (int q = 0; q < Q; q++)
+            mu[q] = acc[q];
+    }
+};
+
+// ------------------------------------------------------------ forward sweep
+
+// forward_kernel with the step spread over a team
+template <class M, class Tab, int G>
+__global__ void __launch_bounds__(256) forward_team_kernel(FwdParams a)
+{
+    constexpr int N = M::N, P = M::P;
+    constexpr int RS = record_doubles(N);
+    const TeamForward<M, Tab, G> tf;
+    const bool first = tf.team.index == 0;
+    const int CH = a.pool.chunk_len;
+
+    int b = -1;
+    double y[N], k0[N], p[P], t = 0.0, t1 = 0.0, dt = 0.0, t_start = 0.0;
+    int count = 0, rej = 0, fails = 0, status = ST_OK, chunk = -1, slot = 0;
+    bool at_top = true;
+
+    auto take = [&](unsigned int *counter) -> int {
+        int v = 0;
+        if (first)
+            v = (int)atomicAdd(counter, 1u);
+        return shfl(v, tf.team.base, tf.team.mask);
+    };
+
+    auto fetch = [&]() -> bool {
+        b = take(&a.ctl->fwd_next);
+        if (b >= a.B)
+            return false;
+        if (a.order)
+            b = a.order[b];
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            y[i] = a.y0[(size_t)b * N + i];
+#pragma unroll
+        for (int k = 0; k < P; k++)
+            p[k] = a.par[(size_t)b * P + k];
+        t = t_start = a.t0[b];
+        t1 = a.t1[b];
+        dt = a.dt0;
+        count = rej = fails = 0;
+        status = ST_OK;
+        at_top = true;
+        slot = 0;
+        chunk = take(&a.ctl->pool_next);
+        if (chunk >= a.pool.n_chunks) {
+            status = ST_CKPT_BUDGET;
+            chunk = -1;
+            if (first)
+                atomicOr(&a.ctl->pool_fail, 1u);
+        } else if (first) {
+            a.pool.chunk_prev[chunk] = -1;
+        }
+        M::template rhs<double>(y, p, t, k0);
+        return true;
+    };
+
+    // Reserve the slot of the next stored record; false if the pool ran out.
+    auto reserve = [&]() -> bool {
+        if (chunk < 0)
+            return false;
+        if (slot == CH) {
+            const int c = take(&a.ctl->pool_next);
+            if (c >= a.pool.n_chunks) {
+                if (first)
+                    atomicOr(&a.ctl->pool_fail, 1u);
+                return false;
+            }
+            if (first)
+                a.pool.chunk_prev[c] = chunk;
+            chunk = c;
+            slot = 0;
+        }
+        return true;
+    };
+    auto write = [&]() {
+        if (first)
+            write_record<N>(record_ptr<RS>(a.pool, chunk, slot), t, dt, y);
+        slot++;
+    };
+
+    auto finish = [&]() {
+        if (status == ST_OK) {
+            if (reserve())
+                write();
+            else
+                status = ST_CKPT_BUDGET;
+#pragma unroll
+            for (int i = 0; i < N; i++)
+                if (!is_finite64(y[i]))
+                    status = ST_NONFINITE;
+        }
+        if (!first)
+            return;
+        if (a.yT) {
+#pragma unroll
+            for (int i = 0; i < N; i++)
+                a.yT[(size_t)b * N + i] = y[i];
+        }
+        a.inst_T[b] = count;
+        a.inst_last[b] = chunk;
+        a.inst_status[b] = status;
+        note_work(a, b, count + rej);
+        if (a.inst_t1)
+            a.inst_t1[b] = t1;
+        if (Tab::FIXED && a.inst_t0)
+            a.inst_t0[b] = t_start;
+        if (a.n_acc_out)
+            a.n_acc_out[b] = count;
+        if (a.n_rej_out)
+            a.n_rej_out[b] = rej;
+        if (a.status_out)
+            a.status_out[b] = status;
+    };
+
+    bool alive = fetch();
+    while (alive) {
+        if (status != ST_OK) {
+            finish();
+            alive = fetch();
+            continue;
+        }
+        if (at_top) {
+            if (Tab::FIXED ? !less_equal_pos64((t + dt) - t1, kDblEps) : !greater_pos64(t1 - t, kDblEps)) {
+                finish();
+                alive = fetch();
+                continue;
+            }
+            if (count >= a.max_steps) {
+                status = ST_MAX_STEPS;
+                continue;
+            }
+            if (a.stride <= 1 || count % a.stride == 0) {
+                if (!reserve()) {
+                    status = ST_CKPT_BUDGET;
+                    continue;
+                }
+                write();
+            }
+            if (!Tab::FIXED && greater_pos64((t + dt) - t1, kDblEps))
+                dt = t1 - t;
+            fails = 0;
+            at_top = false;
+        }
+        double ynew[N], knew[N];
+        const double err = tf.attempt(y, k0, p, t, dt, a.atol, a.rtol, ynew, knew);
+        bool ok;
+        if (is_nan64(err)) {
+            status = ST_NONFINITE;
+            continue;
+        }
+        unsigned int *undecided = first ? &a.ctl->pow_undecided : nullptr;
+        if (greater_nonneg64(err, 1.0)) {
+            dt = decrease_step<Tab, double>(dt, err, a.step_pow, undecided);
+            rej++;
+            ok = false;
+        } else {
+            if constexpr (Tab::FIXED) {
+                t = fixed_time(t_start, count + 1, dt);
+            } else {
+                t += dt;
+                dt = increase_step<Tab, double>(dt, err, a.step_pow, undecided);
+            }
+            accept_state<M, Tab, double>(y, y, k0, ynew, ynew, knew, p, t);
+            ok = true;
+        }
+        if (fails >= a.max_fail) {
+            status = ST_MAX_REJECTS;
+            continue;
+        }
+        fails++;
+        if (ok) {
+            count++;
+            at_top = true;
+        } else if (!positive_finite64(dt)) {
+            status = ST_NONFINITE;
+        }
+    }
+}
+
+// ----------------------------------------------------------- backward sweep
+
+// outputs of an instance without a trajectory
+template <int N, int P>
+__device__ __forceinline__ void team_fail(const AdjParams &a, int b, int st)
+{
+    for (int qq = 0; qq < a.nout; qq++) {
+        const size_t o = ((size_t)b * a.nout + qq);
+        for (int i = 0; i < N; i++)
+            a.dy0[o * N + i] = __longlong_as_double(0x7ff8000000000000ll);
+        for (int k = 0; k < P; k++)
+            a.dpar[o * P + k] = __longlong_as_double(0x7ff8000000000000ll);
+    }
+    if (a.status_out)
+        a.status_out[b] = st;
+}
+
+// lambda_0 and mu of a finished seed (one lane writes)
+template <int N, int P>
+__device__ __forceinline__ void team_store(const AdjParams &a, int b, int q, const double (&lam)[N],
+                                           const double (&mu)[P])
+{
+    const size_t o = ((size_t)b * a.nout + q);
+    bool finite = true;
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        a.dy0[o * N + i] = lam[i];
+        finite = finite && is_finite64(lam[i]);
+    }
+#pragma unroll
+    for (int k = 0; k < P; k++) {
+        const double d = a.mu_direct ? a.mu_direct[o * P + k] : 0.0;
+        a.dpar[o * P + k] = d + mu[k];
+        finite = finite && is_finite64(mu[k]);
+    }
+    if (a.status_out && (q == a.nout - 1 || !finite))
+        a.status_out[b] = finite ? ST_OK : ST_NONFINITE;
+}
+
+// backward_kernel with the step spread over a team
+template <class M, class Tab, int G>
+__global__ void __launch_bounds__(256) backward_team_kernel(AdjParams a)
+{
+    constexpr int N = M::N, P = M::P;
+    constexpr int RS = record_doubles(N);
+    const TeamBackward<M, Tab, G> tb;
+    const bool first = tb.team.index == 0;
+    const int CH = a.pool.chunk_len;
+
+    int b = -1, q = 0, j = -1, chunk = -1, slot = 0, T = 0, last = -1;
+    double lam[N], mu[TeamBackward<M, Tab, G>::Q], t_next = 0.0, p[P];
+
+    auto start_seed = [&]() {
+        chunk = last;
+        slot = T % CH;
+        double yTl[N];
+        read_record<N>(record_ptr<RS>(a.pool, chunk, slot), t_next, yTl);
+        const size_t o = ((size_t)b * a.nout + q);
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            lam[i] = a.cost == 0 ? 2.0 * yTl[i] : a.cost == 1 ? 1.0 : a.lambdaT[o * N + i];
+        tb.clear(mu);
+        if (first)
+            note_lambda<N>(a, b, q, T, lam);
+        j = T - 1;
+    };
+    auto fetch = [&]() -> bool {
+        for (;;) {
+            int w = 0;
+            if (first)
+                w = (int)atomicAdd(&a.ctl->adj_next, 1u);
+            w = shfl(w, tb.team.base, tb.team.mask);
+            if (w >= a.B)
+                return false;
+            b = a.order ? a.order[w] : w;
+            const int st = a.inst_status[b];
+            if (st != ST_OK) {
+                if (first)
+                    team_fail<N, P>(a, b, st);
+                continue;
+            }
+#pragma unroll
+            for (int k = 0; k < P; k++)
+                p[k] = a.par[(size_t)b * P + k];
+            T = a.inst_T[b];
+            last = a.inst_last[b];
+            q = 0;
+            start_seed();
+            return true;
+        }
+    };
+
+    bool alive = fetch();
+    while (alive) {
+        if (j < 0) {
+            double m[P];
+#pragma unroll
+            for (int k = 0; k < P; k++)
+                m[k] = tb.param(mu, k);
+            if (first)
+                team_store<N, P>(a, b, q, lam, m);
+            if (q + 1 < a.nout) {
+                q++;
+                start_seed();
+            } else {
+                alive = fetch();
+            }
+            continue;
+        }
+        if (slot == 0) {
+            chunk = a.pool.chunk_prev[chunk];
+            slot = CH - 1;
+        } else {
+            slot--;
+        }
+        double y[N], tn;
+        read_record<N>(record_ptr<RS>(a.pool, chunk, slot), tn, y);
+        tb.step(y, tn, t_next - tn, p, lam, mu);
+        if (first)
+            note_lambda<N>(a, b, q, j, lam);
+        t_next = tn;
+        j--;
+    }
+}
+
+// --------------------------------------------- backward sweep, two levels
+
+// backward_kernel_2level with both phases spread over a team; the segment's
+// records lie in the team's scratch (one lane writes, all read).
+template <class M, class Tab, int G>
+__global__ void __launch_bounds__(256) backward_team_kernel_2level(AdjParams a)
+{
+    constexpr int N = M::N, P = M::P;
+    constexpr int RS = record_doubles(N);
+    const TeamForward<M, Tab, G> tf;
+    const TeamBackward<M, Tab, G> tb;
+    const bool first = tb.team.index == 0;
+    const int CH = a.pool.chunk_len, SK = a.stride;
+    double *scr = a.scratch + ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G * (SK + 1) * RS;
+
+    int b = -1, q = 0, T = 0, R = 0, k = 0, last = -1, chunk = -1, slot = 0, L = 0, done = 0, jb = 0, fails = 0;
+    int head = 0;           // step index of the segment's first record
+    double t_start = 0.0;   // t_0 (fixed-step tableaux)
+    int phase = 0;          // 0: re-integrate segment k, 1: back-step through it
+    double lam[N], mu[TeamBackward<M, Tab, G>::Q], t = 0.0, dt = 0.0, t1 = 0.0, y[N], t_end = 0.0, y_end[N];
+    double p[P], k0[N];
+    bool at_top = true;
+
+    auto keep = [&](int n) { // record n of the segment
+        __syncwarp(tb.team.mask);
+        if (first) {
+            double *r = scr + (size_t)n * RS;
+            r[0] = t;
+#pragma unroll
+            for (int i = 0; i < N; i++)
+                r[2 + i] = y[i];
+        }
+        __syncwarp(tb.team.mask);
+    };
+    auto begin_segment = [&]() {
+        if (slot == 0) {
+            chunk = a.pool.chunk_prev[chunk];
+            slot = CH - 1;
+        } else {
+            slot--;
+        }
+        const double *r = record_ptr<RS>(a.pool, chunk, slot);
+        read_record<N>(r, t, y);
+        dt = r[1];
+        head = k * SK;
+        L = (k == R - 2) ? T - head : SK;
+        keep(0);
+        M::template rhs<double>(y, p, t, k0);
+        done = 0;
+        fails = 0;
+        at_top = true;
+        phase = 0;
+    };
+    auto start_seed = [&]() {
+        chunk = last;
+        slot = (R - 1) % CH;
+        read_record<N>(record_ptr<RS>(a.pool, chunk, slot), t_end, y_end);
+        const size_t o = ((size_t)b * a.nout + q);
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            lam[i] = a.cost == 0 ? 2.0 * y_end[i] : a.cost == 1 ? 1.0 : a.lambdaT[o * N + i];
+        tb.clear(mu);
+        if (first)
+            note_lambda<N>(a, b, q, T, lam);
+        k = R - 2;
+        if (k >= 0)
+            begin_segment();
+    };
+    auto fetch = [&]() -> bool {
+        for (;;) {
+            int w = 0;
+            if (first)
+                w = (int)atomicAdd(&a.ctl->adj_next, 1u);
+            w = shfl(w, tb.team.base, tb.team.mask);
+            if (w >= a.B)
+                return false;
+            b = a.order ? a.order[w] : w;
+            const int st = a.inst_status[b];
+            if (st != ST_OK) {
+                if (first)
+                    team_fail<N, P>(a, b, st);
+                continue;
+            }
+#pragma unroll
+            for (int kk = 0; kk < P; kk++)
+                p[kk] = a.par[(size_t)b * P + kk];
+            T = a.inst_T[b];
+            R = (T + SK - 1) / SK + 1;
+            last = a.inst_last[b];
+            t1 = a.inst_t1[b];
+            if constexpr (Tab::FIXED)
+                t_start = a.inst_t0[b];
+            q = 0;
+            start_seed();
+            return true;
+        }
+    };
+
+    bool alive = fetch();
+    while (alive) {
+        if (k < 0) {
+            double m[P];
+#pragma unroll
+            for (int kk = 0; kk < P; kk++)
+                m[kk] = tb.param(mu, kk);
+            if (first)
+                team_store<N, P>(a, b, q, lam, m);
+            if (q + 1 < a.nout) {
+                q++;
+                start_seed();
+            } else {
+                alive = fetch();
+            }
+            continue;
+        }
+        if (phase == 0) {
+            // one attempt of the forward controller, as forward_team_kernel does
+            if (at_top) {
+                if (!Tab::FIXED && greater_pos64((t + dt) - t1, kDblEps))
+                    dt = t1 - t;
+                fails = 0;
+                at_top = false;
+            }
+            double ynew[N], knew[N];
+            const double err = tf.attempt(y, k0, p, t, dt, a.atol, a.rtol, ynew, knew);
+            if (is_nan64(err) || fails >= a.max_fail) {
+                if (first)
+                    team_fail<N, P>(a, b, ST_RECOMPUTE_MISMATCH);
+                alive = fetch();
+                continue;
+            }
+            fails++;
+            unsigned int *undecided = first ? &a.ctl->pow_undecided : nullptr;
+            if (greater_nonneg64(err, 1.0)) {
+                dt = decrease_step<Tab, double>(dt, err, a.step_pow, undecided);
+                continue;
+            }
+            if constexpr (Tab::FIXED) {
+                t = fixed_time(t_start, head + done + 1, dt);
+            } else {
+                t += dt;
+                dt = increase_step<Tab, double>(dt, err, a.step_pow, undecided);
+            }
+            accept_state<M, Tab, double>(y, y, k0, ynew, ynew, knew, p, t);
+            at_top = true;
+            done++;
+            keep(done);
+            if (done == L) {
+                // the re-integration must land exactly on the next checkpoint
+                bool same = t == t_end;
+#pragma unroll
+                for (int i = 0; i < N; i++)
+                    same = same && y[i] == y_end[i];
+                if (!same) {
+                    if (first)
+                        team_fail<N, P>(a, b, ST_RECOMPUTE_MISMATCH);
+                    alive = fetch();
+                    continue;
+                }
+                phase = 1;
+                jb = L - 1;
+            }
+            continue;
+        }
+        // phase 1: back_step through the segment, last step first
+        const double *r = scr + (size_t)jb * RS;
+        double yj[N];
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            yj[i] = r[2 + i];
+        const double tn = r[0];
+        tb.step(yj, tn, r[RS] - tn, p, lam, mu);
+        if (first)
+            note_lambda<N>(a, b, q, head + jb, lam);
+        jb--;
+        if (jb < 0) {
+            // the segment's start becomes the next segment's end
+            t_end = tn;
+#pragma unroll
+            for (int i = 0; i < N; i++)
+                y_end[i] = yj[i];
+            k--;
+            if (k >= 0)
+                begin_segment();
+        }
+    }
+}
+
+} // namespace va
