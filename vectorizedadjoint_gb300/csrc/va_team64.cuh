@@ -660,8 +660,18 @@ __global__ void __launch_bounds__(256) backward_team_kernel(AdjParams a)
     const int CH = a.pool.chunk_len;
 
     int b = -1, q = 0, j = -1, chunk = -1, slot = 0, T = 0, last = -1;
-    double lam[N], mu[TeamBackward<M, Tab, G>::Q], t_next = 0.0, p[P];
+    double lam[N], mu[TeamBackward<M, Tab, G>::Q], t_next = 0.0, p[P], t_ahead = 0.0, y_ahead[N];
 
+    // the record before the walk's, into t_ahead, y_ahead
+    auto ahead = [&]() {
+        if (slot == 0) {
+            chunk = a.pool.chunk_prev[chunk];
+            slot = CH - 1;
+        } else {
+            slot--;
+        }
+        read_record<N>(record_ptr<RS>(a.pool, chunk, slot), t_ahead, y_ahead);
+    };
     auto start_seed = [&]() {
         chunk = last;
         slot = T % CH;
@@ -675,6 +685,8 @@ __global__ void __launch_bounds__(256) backward_team_kernel(AdjParams a)
         if (first)
             note_lambda<N>(a, b, q, T, lam);
         j = T - 1;
+        if (j >= 0)
+            ahead();
     };
     auto fetch = [&]() -> bool {
         for (;;) {
@@ -719,14 +731,13 @@ __global__ void __launch_bounds__(256) backward_team_kernel(AdjParams a)
             }
             continue;
         }
-        if (slot == 0) {
-            chunk = a.pool.chunk_prev[chunk];
-            slot = CH - 1;
-        } else {
-            slot--;
-        }
-        double y[N], tn;
-        read_record<N>(record_ptr<RS>(a.pool, chunk, slot), tn, y);
+        double y[N];
+        const double tn = t_ahead;
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            y[i] = y_ahead[i];
+        if (j > 0)
+            ahead(); // the next record's load runs beside this step
         tb.step(y, tn, t_next - tn, p, lam, mu);
         if (first)
             note_lambda<N>(a, b, q, j, lam);
