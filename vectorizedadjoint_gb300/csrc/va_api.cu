@@ -61,6 +61,7 @@ struct va_handle {
     const void *sw_fwd = nullptr, *sw_bwd = nullptr, *sw_bwd2 = nullptr;
     int lanes = 1;
     int bps = 0; // resident blocks per SM of the default launch shape (0: the occupancy limit)
+    bool default_shape = true; // neither given by the caller nor tuned
     int N = 0, P = 0;
     int RS = 0; // doubles per checkpoint record at the current stride (record_layout)
     bool stages_on = true; // opt.stage_records, cleared by the automatic checkpoint ladder
@@ -613,6 +614,15 @@ cudaError_t launch(const va_handle *h, const void *fn, int grid, int block, void
     return cudaLaunchKernel(fn, dim3(grid), dim3(block), args, smem, s);
 }
 
+// Lanes of one warp per quadrant for the sweeps of one lane per instance in
+// their default launch shape, which keep only those busy when the order finds
+// that the longest instance sets the pace; 0: no such decision (a shape that
+// the caller gave or the autotuner measured stands).
+int rest_lanes(const va_handle *h)
+{
+    return h->ks && h->ks->tpi == 1 && h->lanes == 1 && h->default_shape ? 128 * h->sm_count : 0;
+}
+
 va_status enqueue_forward(va_handle *h, const double *y0, const double *params, const double *t0,
                           const double *t1, double *yT, int32_t *n_acc, int32_t *n_rej,
                           int32_t *status, cudaStream_t s)
@@ -673,9 +683,11 @@ va_status enqueue_forward(va_handle *h, const double *y0, const double *params, 
         h->fwd_grid = grid_for(h, fn, h->fwd_block, a.B);
     if (h->order_fwd) {
         const int *valid = h->inst_work + a.B;
-        va::OrderArgs o{a.B, nullptr, t0, t1, h->inst_work, valid, h->order_work, h->order_fwd};
+        va::OrderArgs o{a.B, nullptr, t0, t1, h->inst_work, valid, h->order_work, h->order_fwd, nullptr, rest_lanes(h)};
         VA_CUDA(h, va::enqueue_order(o, s));
         a.order = h->order_fwd;
+        a.one_warp = o.lanes ? va::order_one_warp(h->order_work) : nullptr;
+        a.sms = h->sm_count;
         a.inst_work = h->inst_work;
         a.work_valid = h->inst_work + a.B;
     }
@@ -709,9 +721,11 @@ va_status enqueue_backward(va_handle *h, const double *params, const double *lam
         // +3%); the lane groups sort by their own step counts (GLV-10: the
         // reused order made the backward 11% slower)
         const int *reuse = h->ks->tpi == 1 ? h->order_fwd : nullptr;
-        va::OrderArgs o{a.B, h->inst_T, nullptr, nullptr, nullptr, nullptr, h->order_work, h->order_bwd, reuse};
+        va::OrderArgs o{a.B, h->inst_T, nullptr, nullptr, nullptr, nullptr, h->order_work, h->order_bwd, reuse, rest_lanes(h)};
         VA_CUDA(h, va::enqueue_order(o, s));
         a.order = h->order_bwd;
+        a.one_warp = o.lanes ? va::order_one_warp(h->order_work) : nullptr;
+        a.sms = h->sm_count;
     }
     if (h->bks && h->stride > 1) {
         // two-level: segments re-run from the strided checkpoints, in bundles
@@ -856,6 +870,7 @@ void apply_shape(va_handle *h, const TunedShape &t)
     }
     const void *ffn = fwd_kernel(h);
     const void *bfn = bwd_kernel(h);
+    h->default_shape = false;
     h->fwd_block = t.fb;
     h->fwd_grid = grid_of(h, ffn, t.fb, t.fbps);
     h->bwd_block = t.bb;
@@ -1173,6 +1188,7 @@ va_status create_handle(const va_problem *prob, const va_options *opt, const va:
     h->P = P;
     h->chunk_len = o.chunk_len > 0 ? o.chunk_len : 64;
     record_layout(h);
+    h->default_shape = o.block_size <= 0 && o.blocks_per_sm <= 0;
     if (o.block_size > 0) {
         h->fwd_block = h->bwd_block = o.block_size;
     }
@@ -1696,7 +1712,7 @@ va_status va_autotune(va_handle *h, int32_t cost, const double *y0, const double
     cudaStream_t s = (cudaStream_t)stream;
     // the launch shape before tuning, restored if a candidate run fails
     const int prev[4] = {h->fwd_block, h->fwd_grid, h->bwd_block, h->bwd_grid};
-    const bool prev_alt = h->bundle_alt;
+    const bool prev_alt = h->bundle_alt, prev_default = h->default_shape;
     AutotuneEvents ev;
     st = autotune_sweep(h, cost, y0, params, t0, t1, s, ev, t);
     if (st != VA_OK) {
@@ -1704,6 +1720,7 @@ va_status va_autotune(va_handle *h, int32_t cost, const double *y0, const double
         h->fwd_grid = prev[1];
         h->bwd_block = prev[2];
         h->bwd_grid = prev[3];
+        h->default_shape = prev_default;
         h->bundle_alt = prev_alt;
         drop_graph(h);
         return st;

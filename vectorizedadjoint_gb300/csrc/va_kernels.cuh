@@ -88,7 +88,18 @@ struct FwdParams {
     int *work_valid; // set to 1 once inst_work holds a sweep's counts (may be null)
     Pool pool;
     Control *ctl;
+    const int *one_warp; // device flag: keep one warp per SM quadrant only (may be null)
+    int sms;             // SMs (blocks b, b + sms, ... share one)
 };
+
+// Whether this warp stays idle: the first four warps of an SM carry the sweep
+// when the flag is set (the order's decision, va_order.cu).
+template <class Params>
+__device__ __forceinline__ bool resting(const Params &a)
+{
+    return a.one_warp && *a.one_warp &&
+           blockIdx.x / (unsigned)a.sms * (blockDim.x / 32) + threadIdx.x / 32 >= 4;
+}
 
 // Record an instance's attempt count for the next forward sweep's order.
 __device__ __forceinline__ void note_work(const FwdParams &a, int b, int attempts)
@@ -128,6 +139,8 @@ struct AdjParams {
     // hist[((b * nout + q) * hist_cap + n) * N + i] for record n < hist_cap
     double *hist;
     int hist_cap;
+    const int *one_warp; // as FwdParams
+    int sms;
 };
 
 __host__ __device__ constexpr int record_doubles(int n) { return (2 + n + 1) & ~1; }
@@ -648,6 +661,8 @@ __global__ void __launch_bounds__(256) forward_kernel(FwdParams a)
     constexpr int N = M::N, P = M::P;
     constexpr int RS = record_doubles(N);
     const int CH = a.pool.chunk_len;
+    if (resting(a))
+        return;
 
     int b = -1;
     double y[N], t = 0.0, t1 = 0.0, dt = 0.0, t_start = 0.0;
@@ -968,6 +983,8 @@ __global__ void __launch_bounds__(256) backward_kernel(AdjParams a)
     constexpr int N = M::N, P = M::P;
     constexpr int RS = record_doubles(N);
     const int CH = a.pool.chunk_len;
+    if (resting(a))
+        return;
 
     int b = -1, q = 0, j = -1, chunk = -1, slot = 0, T = 0, last = -1;
     double lam[N], mu[P], t_next = 0.0;

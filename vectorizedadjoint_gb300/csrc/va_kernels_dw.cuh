@@ -465,6 +465,8 @@ __global__ void __launch_bounds__(256) forward_kernel_dw(FwdParams a)
     constexpr int RS = STAGES ? stage_record_doubles(N, Tab::S) : record_doubles(N);
     const int CH = a.pool.chunk_len;
     const DwTol tol{dword(a.atol), dword(a.rtol)};
+    if (resting(a))
+        return;
 
     int b = -1;
     double t = 0.0, t1 = 0.0, t_start = 0.0;
@@ -808,6 +810,8 @@ __global__ void __launch_bounds__(256) backward_kernel_dw(AdjParams a)
     static_assert(M::PG == M::P, "parameter adjoint covers every parameter");
     constexpr int RS = STAGES ? stage_record_doubles(N, NS) : record_doubles(N);
     const int CH = a.pool.chunk_len;
+    if (resting(a))
+        return;
 
     int b = -1, q = 0, j = -1, chunk = -1, slot = 0, T = 0, last = -1;
     double t_next = 0.0;
