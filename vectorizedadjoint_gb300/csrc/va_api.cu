@@ -615,8 +615,8 @@ cudaError_t launch(const va_handle *h, const void *fn, int grid, int block, void
 }
 
 // Lanes of one warp per quadrant for the sweeps of one lane per instance in
-// their default launch shape, which keep only those busy when the order finds
-// that the longest instance sets the pace; 0: no such decision (a shape that
+// their default launch shape, which keep only as many warps busy as the order
+// finds useful beside the longest instance; 0: no such decision (a shape that
 // the caller gave or the autotuner measured stands).
 int rest_lanes(const va_handle *h)
 {
@@ -686,7 +686,7 @@ va_status enqueue_forward(va_handle *h, const double *y0, const double *params, 
         va::OrderArgs o{a.B, nullptr, t0, t1, h->inst_work, valid, h->order_work, h->order_fwd, nullptr, rest_lanes(h)};
         VA_CUDA(h, va::enqueue_order(o, s));
         a.order = h->order_fwd;
-        a.one_warp = o.lanes ? va::order_one_warp(h->order_work) : nullptr;
+        a.warps = o.lanes ? va::order_warps(h->order_work) : nullptr;
         a.sms = h->sm_count;
         a.inst_work = h->inst_work;
         a.work_valid = h->inst_work + a.B;
@@ -724,7 +724,7 @@ va_status enqueue_backward(va_handle *h, const double *params, const double *lam
         va::OrderArgs o{a.B, h->inst_T, nullptr, nullptr, nullptr, nullptr, h->order_work, h->order_bwd, reuse, rest_lanes(h)};
         VA_CUDA(h, va::enqueue_order(o, s));
         a.order = h->order_bwd;
-        a.one_warp = o.lanes ? va::order_one_warp(h->order_work) : nullptr;
+        a.warps = o.lanes ? va::order_warps(h->order_work) : nullptr;
         a.sms = h->sm_count;
     }
     if (h->bks && h->stride > 1) {

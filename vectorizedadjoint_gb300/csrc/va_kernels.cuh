@@ -88,17 +88,17 @@ struct FwdParams {
     int *work_valid; // set to 1 once inst_work holds a sweep's counts (may be null)
     Pool pool;
     Control *ctl;
-    const int *one_warp; // device flag: keep one warp per SM quadrant only (may be null)
+    const int *warps;    // device int: warps per SM quadrant to keep busy (may be null: all)
     int sms;             // SMs (blocks b, b + sms, ... share one)
 };
 
-// Whether this warp stays idle: the first four warps of an SM carry the sweep
-// when the flag is set (the order's decision, va_order.cu).
+// Whether this warp stays idle: beyond the warps per quadrant that the order
+// found useful (va_order.cu).
 template <class Params>
 __device__ __forceinline__ bool resting(const Params &a)
 {
-    return a.one_warp && *a.one_warp &&
-           blockIdx.x / (unsigned)a.sms * (blockDim.x / 32) + threadIdx.x / 32 >= 4;
+    return a.warps &&
+           (int)(blockIdx.x / (unsigned)a.sms * (blockDim.x / 32) + threadIdx.x / 32) >= 4 * *a.warps;
 }
 
 // Record an instance's attempt count for the next forward sweep's order.
@@ -139,7 +139,7 @@ struct AdjParams {
     // hist[((b * nout + q) * hist_cap + n) * N + i] for record n < hist_cap
     double *hist;
     int hist_cap;
-    const int *one_warp; // as FwdParams
+    const int *warps; // as FwdParams
     int sms;
 };
 

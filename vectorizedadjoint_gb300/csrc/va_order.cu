@@ -29,7 +29,9 @@
 // ms with one warp, 6.44 with four; FP64 27.0 against 32.1 with two;
 // Van der Pol (lengths within 2x of the mean) 262,144 instances 8.25 ms with
 // one warp, 5.11 with four; 20,000 instances, which fill one warp per
-// quadrant, 1.06 against 1.23.
+// quadrant, 1.06 against 1.23; 65,536 instances (sum = 1.9 longest x lanes)
+// 2.31 with one warp, 1.57 with two, 1.90 with four.  So the sweep keeps
+// ceil(sum / (1.25 longest lanes)) warps per quadrant busy.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -57,8 +59,8 @@ __device__ __forceinline__ int count_bucket(int n) { return n < kBuckets ? (n < 
 // work[2 kBuckets]: 1 when the last forward order came from step counts
 constexpr int kCountedFlag = 2 * kBuckets;
 
-// work[2 kBuckets + 1]: one warp per quadrant is enough
-constexpr int kOneWarpFlag = kCountedFlag + 1;
+// work[2 kBuckets + 1]: warps per quadrant to keep busy
+constexpr int kWarpsSlot = kCountedFlag + 1;
 
 // the backward reuses the forward's order when that one was count-based
 __device__ __forceinline__ bool reusing(const OrderArgs &a) { return a.reuse && a.work[kCountedFlag] == 1; }
@@ -146,7 +148,8 @@ __global__ void order_scan(OrderArgs a)
                 s1 += sum[w];
                 m1 = fmaxf(m1, top[w]);
             }
-            a.work[kOneWarpFlag] = s1 <= 1.25f * m1 * (float)a.lanes ? 1 : 0;
+            const float w = m1 > 0.0f ? ceilf(s1 / (1.25f * m1 * (float)a.lanes)) : 1.0f;
+            a.work[kWarpsSlot] = w < 64.0f ? max(1, (int)w) : 64;
         }
     }
 }
@@ -184,7 +187,7 @@ __global__ void __launch_bounds__(1024) order_scatter(OrderArgs a)
 } // namespace
 
 size_t order_work_ints() { return 2 * kBuckets + 2; }
-const int *order_one_warp(const int *work) { return work + kOneWarpFlag; }
+const int *order_warps(const int *work) { return work + kWarpsSlot; }
 
 cudaError_t enqueue_order(const OrderArgs &a, cudaStream_t s)
 {
