@@ -205,14 +205,14 @@ const void *bwd_kernel(const va_handle *h)
 // (4 per SM), since a second warp on a quadrant would share its FP64 unit.
 // Forward + backward, Van der Pol T = 20, ms with teams of 16 / 8 / 4 / 2 lanes
 // and with one lane (integer products):
-//     B = 1,216   2.50 / 3.16 / 3.99 / 5.03   5.11
-//     B = 2,400   3.67 / 3.18 / 3.99 / 5.04   5.11
-//     B = 4,800   6.57 / 4.74 / 4.00 / 5.02   5.05
-//     B = 9,600   9.42 / 8.39 / 6.25 / 5.06   5.20
-//     B = 19,000  16.9 / 12.3 / 10.2 / 8.15   5.77
-// Fehlberg 7(8) (32 / 16 / 8 lanes, one lane with FP64 products): 600: 2.52 /
-// 3.18 / 3.94, 9.52; 1,200: 3.93 / 3.22 / 3.96, 9.61; 5,003: 8.53 / 7.74 / 6.45,
-// 9.79; 9,600: 14.5 / 9.58 / 7.31, 9.84; 19,000: 28.4 / 18.0 / 12.1, 9.87 -- its
+//     B = 1,216   1.96 / 2.72 / 3.51 / 4.67   4.60
+//     B = 2,400   2.79 / 2.72 / 3.50 / 4.68   4.83
+//     B = 4,800   5.25 / 3.95 / 3.51 / 4.69   4.85
+//     B = 9,600   7.44 / 7.67 / 5.47 / 4.66   5.18
+//     B = 19,000  13.3 / 10.8 / 10.2 / 7.70   5.20
+// Fehlberg 7(8) (32 / 16 / 8 lanes, one lane with FP64 products): 600: 1.88 /
+// 2.52 / 3.27, 9.38; 1,200: 2.82 / 2.53 / 3.27, 9.63; 5,003: 6.58 / 5.53 / 5.24,
+// 9.82; 9,600: 10.6 / 7.68 / 6.57, 9.80; 19,000: 20.6 / 15.0 / 11.7, 9.85 -- its
 // narrowest team serves up to four warps per quadrant.
 //
 // Larger batches: products on the integer pipe for the 5(4) pairs

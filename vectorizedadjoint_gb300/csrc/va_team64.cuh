@@ -14,14 +14,17 @@
 // attempt (G = 16) instead of ~230, and the same bits: every (row, component)
 // sum takes the terms of form_stage / attempt_pair in their order.
 //
-// The backward step is spread the same way: the rows are the stage values'
-// recompute, then K-bar_0 .. K-bar_{s-1}, lambda and mu; where a model gives
-// its VJP as weights, those of all stages are formed at once, a lane a stage:
-// ~80 FP64 instructions per step instead of ~290 (127 without the weights).
+// The backward sweep is spread twice.  What a back step needs from the forward
+// trajectory -- the stage values recomputed from y_n with h_n, and the VJP's
+// weights at them -- does not depend on lambda, so a team forms it for G steps
+// at once, a lane a step (~170 FP64 instructions for G steps of a 5(4) pair).
+// The chain through lambda is then ~33 FP64 instructions per step, its rows
+// (lambda, mu, K-bar_0 .. K-bar_{s-1}) spread over the lanes.
 //
-// Measured: one Van der Pol instance 4.4 ms (a lane, FP64 products) -> 2.0 ms;
-// 1,216 instances 6.2 -> 2.5 ms; Fehlberg 7(8), 600 instances 9.5 -> 2.5 ms;
-// two-level backward, 600 instances 11.2 -> 3.6 ms.  What is left is the
+// Measured, forward + backward: one Van der Pol instance 4.4 ms (a lane, FP64
+// products) -> 2.0 ms with the recompute spread over rows -> 1.5 ms over steps;
+// 1,216 instances 6.2 -> 2.5 -> 1.96; Fehlberg 7(8), 600 instances 9.5 -> 2.5
+// -> 1.9; two-level backward, 600 instances 11.2 -> 3.6 -> 2.9.  What is left is the
 // latency of a step's chain (right-hand side, one product and one sum per
 // stage, the shuffles between them, the step factor): the FP64 unit is busy
 // about half the time.
@@ -235,19 +238,11 @@ struct TeamForward {
     }
 };
 
-template <class M, class = void>
-struct HasVjpWeights : std::false_type {
-};
-template <class M>
-struct HasVjpWeights<M, std::void_t<decltype(M::kVjpW)>> : std::true_type {
-};
-
 template <class Tab, int N, int P, int G>
 struct TeamBackwardTable {
     static constexpr int NS = Tab::S, SLOTS = N + P + NS * N, W = (SLOTS + G - 1) / G * G;
-    static constexpr int XSLOTS = (NS - 1) * N, XW = XSLOTS ? (XSLOTS + G - 1) / G * G : G;
-    double ca[NS][W], cb[W], cx[NS][XW];
-    __host__ __device__ constexpr TeamBackwardTable() : ca(), cb(), cx()
+    double ca[NS][W], cb[W];
+    __host__ __device__ constexpr TeamBackwardTable() : ca(), cb()
     {
         for (int s = N + P; s < SLOTS; s++) {
             const int k = (s - N - P) / N;
@@ -255,33 +250,23 @@ struct TeamBackwardTable {
             for (int m = k + 1; m < NS; m++)
                 ca[m][s] = Tab::a(m, k);
         }
-        for (int s = 0; s < XSLOTS; s++)
-            for (int j = 0; j < NS - 1 - s / N; j++)
-                cx[j][s] = Tab::a(NS - 1 - s / N, j);
     }
 };
 template <class Tab, int N, int P, int G>
 __device__ constexpr TeamBackwardTable<Tab, N, P, G> kTeamBackward{};
 
 // Rows of the backward sums.  Slots: lambda (N), mu (P), then K-bar_k
-// component i at N + P + k N + i.
+// component i at N + P + k N + i.  The model gives its VJP outputs o (gx, then
+// gp) as w[kVjpW] W_o(x), plus w[0] for o = kVjpAdd (vjp_weights).
 template <class M, class Tab, int G>
 struct TeamBackward {
     static constexpr int N = M::N, P = M::PG, NS = Tab::S;
     static constexpr int SLOTS = N + P + NS * N, Q = (SLOTS + G - 1) / G;
-    static constexpr int XQ = ((NS - 1) * N + G - 1) / G; // stage rows X_{s-1} .. X_1
-    static constexpr int XQ1 = XQ > 0 ? XQ : 1;
-    // Models whose VJP outputs o (gx, then gp) are w[kVjpW] W_o(x), plus w[0]
-    // for o = kVjpAdd: the weights W of all stages are formed at once, lane l
-    // taking stage l, and each lane then forms only its own row's output.
-    static constexpr bool WEIGHTS = HasVjpWeights<M>::value;
-    static constexpr int WQ = (NS + G - 1) / G;
+    using Weights = double[NS][N + P];
     double ca[NS][Q]; // a_mk of the lane's K-bar_k
     double cb[Q];     // b_k
-    double cx[NS][XQ1]; // a_mj of the lane's stage m
     int kind[Q];      // 0 lambda, 1 mu, 2 K-bar
     int comp[Q];      // component (lambda, K-bar) or parameter (mu)
-    int xcomp[XQ1];
     LaneGroup<G> team;
 
     __device__ __forceinline__ TeamBackward()
@@ -295,14 +280,6 @@ struct TeamBackward {
 #pragma unroll
             for (int m = 0; m < NS; m++)
                 ca[m][q] = kTeamBackward<Tab, N, P, G>.ca[m][s];
-        }
-#pragma unroll
-        for (int q = 0; q < XQ1; q++) {
-            const int s = team.index + G * q;
-            xcomp[q] = s % N;
-#pragma unroll
-            for (int j = 0; j < NS; j++)
-                cx[j][q] = kTeamBackward<Tab, N, P, G>.cx[j][s];
         }
     }
 
@@ -335,34 +312,25 @@ struct TeamBackward {
         return shfl(mu[(N + k) / G], team.base + (N + k) % G, team.mask);
     }
 
-    // back_step: lam on every lane, mu in its lanes
-    __device__ __forceinline__ void step(const double (&y)[N], double tn, double h, const double (&p)[M::P],
-                                         double (&lam)[N], double (&mu)[Q]) const
+    // VJP weights of every stage of this lane's step (back_step's recompute)
+    __device__ __forceinline__ static void weights(const double (&y)[N], double tn, double h, const double (&p)[M::P],
+                                                   Weights &W)
     {
-        double X[NS][N];
-        {
-            double acc[XQ1];
+        double X[N], K[NS][N];
 #pragma unroll
-            for (int q = 0; q < XQ1; q++)
-                acc[q] = pick<N>(y, xcomp[q]);
-#pragma unroll
-            for (int i = 0; i < N; i++)
-                X[0][i] = y[i];
-#pragma unroll
-            for (int m = 0; m < NS - 1; m++) {
-                double K[N];
-                M::template rhs<double>(X[m], p, tn + Tab::c(m) * h, K);
-#pragma unroll
-                for (int q = 0; q < XQ1; q++)
-                    if (q * G < (NS - 1 - m) * N) // a stage after m among them
-                        acc[q] = acc[q] + (cx[m][q] * h) * pick<N>(K, xcomp[q]);
-#pragma unroll
-                for (int i = 0; i < N; i++) {
-                    const int s = (NS - 2 - m) * N + i;
-                    X[m + 1][i] = shfl(acc[s / G], team.base + s % G, team.mask);
-                }
-            }
+        for (int m = 0; m < NS; m++) {
+            form_stage<Tab, N, double>(m, y, y, K, h, h, X);
+            if (m < NS - 1)
+                M::template rhs<double>(X, p, tn + Tab::c(m) * h, K[m]);
+            M::vjp_weights(X, p, W[m]);
         }
+    }
+
+    // back_step with the weights that lane `from` of the team holds and its
+    // step's h: lam on every lane, mu in its lanes
+    __device__ __forceinline__ void step(const Weights &W, int from, double h, double (&lam)[N], double (&mu)[Q]) const
+    {
+        const int src = team.base + from;
         double acc[Q];
 #pragma unroll
         for (int q = 0; q < Q; q++) {
@@ -371,50 +339,25 @@ struct TeamBackward {
             if (!only_kbar(q))
                 acc[q] = kind[q] == 2 ? acc[q] : kind[q] == 0 ? l : mu[q];
         }
-double W[WQ][N + P]; // VJP weights of stage team.index + G r
-        if constexpr (WEIGHTS) {
-#pragma unroll
-            for (int r = 0; r < WQ; r++) {
-                double Xl[N];
-#pragma unroll
-                for (int i = 0; i < N; i++) {
-                    Xl[i] = X[G * r][i];
-#pragma unroll
-                    for (int m = G * r + 1; m < NS; m++)
-                        Xl[i] = team.index + G * r == m ? X[m][i] : Xl[i];
-                }
-                M::vjp_weights(Xl, p, W[r]);
-            }
-        }
 #pragma unroll
         for (int m = NS - 1; m >= 0; m--) {
-            double w[N], gx[N], gp[P], Wm[N + P];
+            double w[N], Wm[N + P];
 #pragma unroll
             for (int i = 0; i < N; i++) {
                 const int s = N + P + m * N + i;
                 w[i] = shfl(acc[s / G], team.base + s % G, team.mask);
             }
-            if constexpr (WEIGHTS) {
 #pragma unroll
-                for (int o = 0; o < N + P; o++)
-                    Wm[o] = shfl(W[m / G][o], team.base + m % G, team.mask);
-            } else {
-                M::template vjp<double>(w, X[m], p, tn + Tab::c(m) * h, gx, gp);
-            }
+            for (int o = 0; o < N + P; o++)
+                Wm[o] = shfl(W[m][o], src, team.mask);
 #pragma unroll
             for (int q = 0; q < Q; q++)
                 if (live(q, m)) {
-                    double g; // the row's VJP output: gx of its component, or gp
-                    if constexpr (WEIGHTS) {
-                        const int o = kind[q] == 1 ? N + comp[q] : comp[q];
-                        g = w[M::kVjpW] * pick<N + P>(Wm, o);
-                        if constexpr (M::kVjpAdd >= 0)
-                            g = o == M::kVjpAdd ? w[0] + g : g;
-                    } else {
-                        g = pick<N>(gx, comp[q]);
-                        if (!only_kbar(q))
-                            g = kind[q] == 1 ? pick<P>(gp, comp[q]) : g;
-                    }
+                    // the row's VJP output: gx of its component, or gp
+                    const int o = kind[q] == 1 ? N + comp[q] : comp[q];
+                    double g = w[M::kVjpW] * pick<N + P>(Wm, o);
+                    if constexpr (M::kVjpAdd >= 0)
+                        g = o == M::kVjpAdd ? w[0] + g : g;
                     // K-bar_k + (gx a_mk) h; a row k >= m is not read again
                     double term = only_sums(q, m) ? g : (g * ca[m][q]) * h;
                     if (!only_kbar(q))
@@ -649,29 +592,43 @@ __device__ __forceinline__ void team_store(const AdjParams &a, int b, int q, con
         a.status_out[b] = finite ? ST_OK : ST_NONFINITE;
 }
 
-// backward_kernel with the step spread over a team
+// backward_kernel with the steps spread over a team
 template <class M, class Tab, int G>
 __global__ void __launch_bounds__(256) backward_team_kernel(AdjParams a)
 {
     constexpr int N = M::N, P = M::P;
     constexpr int RS = record_doubles(N);
-    const TeamBackward<M, Tab, G> tb;
-    const bool first = tb.team.index == 0;
+    using TB = TeamBackward<M, Tab, G>;
+    const TB tb;
+    const int me = tb.team.index;
+    const bool first = me == 0;
     const int CH = a.pool.chunk_len;
 
     int b = -1, q = 0, j = -1, chunk = -1, slot = 0, T = 0, last = -1;
-    double lam[N], mu[TeamBackward<M, Tab, G>::Q], t_next = 0.0, p[P], t_ahead = 0.0, y_ahead[N];
+    int ready = 0, pos = 0; // steps whose weights the lanes hold, and the next of them
+    double lam[N], mu[TB::Q], t_next = 0.0, p[P], h = 0.0;
+    typename TB::Weights W;
 
-    // the record before the walk's, into t_ahead, y_ahead
-    auto ahead = [&]() {
-        if (slot == 0) {
-            chunk = a.pool.chunk_prev[chunk];
-            slot = CH - 1;
-        } else {
-            slot--;
+    // weights of the steps j, j - 1, .., a lane a step
+    auto prepare = [&]() {
+        ready = j + 1 < G ? j + 1 : G;
+        pos = 0;
+        int c = chunk, s = slot - 1 - (me < ready ? me : ready - 1);
+        while (s < 0) {
+            c = a.pool.chunk_prev[c];
+            s += CH;
         }
-        read_record<N>(record_ptr<RS>(a.pool, chunk, slot), t_ahead, y_ahead);
+        double y[N], tn;
+        read_record<N>(record_ptr<RS>(a.pool, c, s), tn, y);
+        const double above = __shfl_up_sync(tb.team.mask, tn, 1, G);
+        h = (first ? t_next : above) - tn;
+        // the walk and the time go on from the block's last record
+        t_next = shfl(tn, tb.team.base + ready - 1, tb.team.mask);
+        chunk = shfl(c, tb.team.base + ready - 1, tb.team.mask);
+        slot = shfl(s, tb.team.base + ready - 1, tb.team.mask);
+        TB::weights(y, tn, h, p, W);
     };
+
     auto start_seed = [&]() {
         chunk = last;
         slot = T % CH;
@@ -685,8 +642,7 @@ __global__ void __launch_bounds__(256) backward_team_kernel(AdjParams a)
         if (first)
             note_lambda<N>(a, b, q, T, lam);
         j = T - 1;
-        if (j >= 0)
-            ahead();
+        ready = pos = 0;
     };
     auto fetch = [&]() -> bool {
         for (;;) {
@@ -731,17 +687,12 @@ __global__ void __launch_bounds__(256) backward_team_kernel(AdjParams a)
             }
             continue;
         }
-        double y[N];
-        const double tn = t_ahead;
-#pragma unroll
-        for (int i = 0; i < N; i++)
-            y[i] = y_ahead[i];
-        if (j > 0)
-            ahead(); // the next record's load runs beside this step
-        tb.step(y, tn, t_next - tn, p, lam, mu);
+        if (pos == ready)
+            prepare();
+        tb.step(W, pos, shfl(h, tb.team.base + pos, tb.team.mask), lam, mu);
         if (first)
             note_lambda<N>(a, b, q, j, lam);
-        t_next = tn;
+        pos++;
         j--;
     }
 }
@@ -766,7 +717,9 @@ __global__ void __launch_bounds__(256) backward_team_kernel_2level(AdjParams a)
     double t_start = 0.0;   // t_0 (fixed-step tableaux)
     int phase = 0;          // 0: re-integrate segment k, 1: back-step through it
     double lam[N], mu[TeamBackward<M, Tab, G>::Q], t = 0.0, dt = 0.0, t1 = 0.0, y[N], t_end = 0.0, y_end[N];
-    double p[P], k0[N];
+    double p[P], k0[N], h = 0.0;
+    int ready = 0, pos = 0; // phase 1: as backward_team_kernel
+    typename TeamBackward<M, Tab, G>::Weights W;
     bool at_top = true;
 
     auto keep = [&](int n) { // record n of the segment
@@ -907,26 +860,34 @@ __global__ void __launch_bounds__(256) backward_team_kernel_2level(AdjParams a)
                 }
                 phase = 1;
                 jb = L - 1;
+                ready = pos = 0;
             }
             continue;
         }
         // phase 1: back_step through the segment, last step first
-        const double *r = scr + (size_t)jb * RS;
-        double yj[N];
+        if (pos == ready) {
+            ready = jb + 1 < G ? jb + 1 : G;
+            pos = 0;
+            const int me = tb.team.index;
+            const double *r = scr + (size_t)(jb - (me < ready ? me : ready - 1)) * RS;
+            double yj[N];
 #pragma unroll
-        for (int i = 0; i < N; i++)
-            yj[i] = r[2 + i];
-        const double tn = r[0];
-        tb.step(yj, tn, r[RS] - tn, p, lam, mu);
+            for (int i = 0; i < N; i++)
+                yj[i] = r[2 + i];
+            h = r[RS] - r[0];
+            TeamBackward<M, Tab, G>::weights(yj, r[0], h, p, W);
+        }
+        tb.step(W, pos, shfl(h, tb.team.base + pos, tb.team.mask), lam, mu);
+        pos++;
         if (first)
             note_lambda<N>(a, b, q, head + jb, lam);
         jb--;
         if (jb < 0) {
             // the segment's start becomes the next segment's end
-            t_end = tn;
+            t_end = scr[0];
 #pragma unroll
             for (int i = 0; i < N; i++)
-                y_end[i] = yj[i];
+                y_end[i] = scr[2 + i];
             k--;
             if (k >= 0)
                 begin_segment();
