@@ -56,10 +56,10 @@ struct va_handle {
     int sm_count = 0;
     const va::KernelSet *ks = nullptr;
     const va::ModelKernels *user = nullptr; // a device model compiled outside the library
-    // FP64 sweeps in the place of the table's (fp64_path): every-step sweeps
-    // and the two-level backward; the lanes that carry one instance in them
-    const void *sw_fwd = nullptr, *sw_bwd = nullptr, *sw_bwd2 = nullptr;
-    int lanes = 1;
+    // FP64 sweeps (fp64_path): one lane per instance in the place of the table's,
+    // and teams of lanes for smaller loads, widest first
+    const void *sw_fwd = nullptr, *sw_bwd = nullptr;
+    std::vector<va::TeamKernel> teams[va::kFp64Sweeps];
     int bps = 0; // resident blocks per SM of the default launch shape (0: the occupancy limit)
     bool default_shape = true; // neither given by the caller nor tuned
     int N = 0, P = 0;
@@ -83,6 +83,7 @@ struct va_handle {
     double *s_lam = nullptr, *s_mu = nullptr;
 
     int fwd_block = 128, fwd_grid = 0, bwd_block = 128, bwd_grid = 0;
+    int fwd_team_block = 0, fwd_team_grid = 0, bwd_team_block = 0, bwd_team_grid = 0; // of the last team launched
     bool forward_done = false;
     bool ladder_settled = false; // ckpt_stride = -1: va_gradient ran the memory ladder once
     std::string err;
@@ -199,52 +200,33 @@ const void *bwd_kernel(const va_handle *h)
     return h->sw_bwd ? h->sw_bwd : h->ks->bwd[h->opt.tableau][h->opt.precision];
 }
 
-// FP64 sweeps of the built-in one-thread models, by the batch size.
+// FP64 sweeps of the built-in one-thread models.
 //
-// Teams (va_team64.cuh): the widest whose warps do not outnumber the quadrants
-// (4 per SM), since a second warp on a quadrant would share its FP64 unit.
-// Forward + backward, Van der Pol T = 20, ms with teams of 16 / 8 / 4 / 2 lanes
-// and with one lane (integer products):
-//     B = 1,216   1.96 / 2.72 / 3.51 / 4.67   4.60
-//     B = 2,400   2.79 / 2.72 / 3.50 / 4.68   4.83
-//     B = 4,800   5.25 / 3.95 / 3.51 / 4.69   4.85
-//     B = 9,600   7.44 / 7.67 / 5.47 / 4.66   5.18
-//     B = 19,000  13.3 / 10.8 / 10.2 / 7.70   5.20
-// Fehlberg 7(8) (32 / 16 / 8 lanes, one lane with FP64 products): 600: 1.88 /
-// 2.52 / 3.27, 9.38; 1,200: 2.82 / 2.53 / 3.27, 9.63; 5,003: 6.58 / 5.53 / 5.24,
-// 9.82; 9,600: 10.6 / 7.68 / 6.57, 9.80; 19,000: 20.6 / 15.0 / 11.7, 9.85 -- its
-// narrowest team serves up to four warps per quadrant.
+// Teams of lanes (va_team64.cuh) for small loads: the limits and what they
+// were measured against stand where the teams are listed
+// (va_inst_team_fp64.cu, va_inst_team_rkf78_fp64.cu).
 //
-// Larger batches: products on the integer pipe for the 5(4) pairs
-// (va_step64.cuh); Van der Pol with 65,536 instances 9.2 ms against 19.6 ms
-// with FP64 products.  Fehlberg 7(8) and the two-level backward keep the FP64
-// products there: their code is too long for the instruction caches that way
-// (16.1 against 9.8 ms with 5,003 instances, 24.7 against 14.0 ms with 9,001).
-// One block per SM, of 256 threads (two warps on each quadrant to overlap
-// integer and FP64 work) when the batch fills them, else of 128; more resident
-// warps only spread the instruction fetch: 65,536 instances 9.2 ms with 256 x
-// 1, 10.7 with 128 x 2, 12.3 with 128 x 4 and with 128 x 1; 30,000 instances
-// 7.0 ms with 256 x 1, 6.8 with 128 x 1.
+// One lane per instance for larger ones, with the products on the integer pipe
+// for the 5(4) pairs (va_step64.cuh): Van der Pol with 65,536 instances 9.2 ms
+// against 19.6 ms with FP64 products.  Fehlberg 7(8) and the two-level backward
+// keep the FP64 products there: their code is too long for the instruction
+// caches that way (16.1 against 9.8 ms with 5,003 instances, 24.7 against 14.0
+// ms with 9,001).  One block per SM, of 256 threads (two warps on each quadrant
+// to overlap integer and FP64 work) when the batch fills them, else of 128;
+// more resident warps only spread the instruction fetch: 65,536 instances
+// 9.2 ms with 256 x 1, 10.7 with 128 x 2, 12.3 with 128 x 4 and with 128 x 1;
+// 30,000 instances 7.0 ms with 256 x 1, 6.8 with 128 x 1.
 void fp64_path(va_handle *h)
 {
-    h->lanes = h->ks ? h->ks->tpi : 1;
     const va::Fp64Kernels *k = h->user || !h->ks ? nullptr : va::fp64_kernels(h->prob.model);
     if (!k || h->opt.precision != VA_PREC_FP64)
         return;
     const int t = h->opt.tableau;
-    const int64_t lanes = 128LL * h->sm_count; // one warp on every quadrant
-    if (h->opt.block_size <= 0 || h->opt.block_size % 32 == 0) { // a team's lanes share a warp
-        for (const va::TeamKernels &w : k->team[t]) {
-            const int per_quadrant = t == VA_TAB_RKF78 && w.g == 8 ? 4 : 1;
-            if (w.g && (int64_t)h->prob.batch * w.g <= per_quadrant * lanes) {
-                h->lanes = w.g;
-                h->sw_fwd = w.fwd;
-                h->sw_bwd = w.bwd;
-                h->sw_bwd2 = w.bwd2;
-                return;
-            }
-        }
-    }
+    if (h->opt.block_size <= 0 || h->opt.block_size % 32 == 0) // a team's lanes share a warp
+        for (int w = 0; w < va::kFp64Sweeps; w++)
+            for (const va::TeamKernel &c : k->team[t][w])
+                if (c.fn)
+                    h->teams[w].push_back(c);
     if (!k->int_fwd[t])
         return;
     h->sw_fwd = k->int_fwd[t];
@@ -263,7 +245,7 @@ int grid_for(va_handle *h, const void *fn, int block, int instances)
     int bps = h->opt.blocks_per_sm > 0 ? std::min(h->opt.blocks_per_sm, occ) : occ;
     if (h->bps > 0)
         bps = std::min(bps, h->bps);
-    long need = ((long)instances * h->lanes + block - 1) / block;
+    long need = ((long)instances * h->ks->tpi + block - 1) / block;
     long g = (long)h->sm_count * bps;
     return (int)std::max(1L, std::min(g, need));
 }
@@ -512,15 +494,14 @@ int bundle_grid(va_handle *h)
 constexpr int kTwoLevelBlock = 64, kTwoLevelBlocksPerSm = 4;
 constexpr int kTwoLevelGroupBlock = 256, kTwoLevelGroupBlocksPerSm = 2;
 
-// Teams (sw_bwd2): the same blocks, kTwoLevelBlock / lanes instances each.
+// Teams of lanes: the same blocks, kTwoLevelBlock / lanes instances each (no
+// more scratch than one lane per instance).
 int two_level_block(const va_handle *h) { return h->ks->tpi > 1 ? kTwoLevelGroupBlock : kTwoLevelBlock; }
 
 // instances one block of the two-level backward carries at once
 int two_level_per_block(const va_handle *h)
 {
     const int g = h->ks->tpi;
-    if (h->sw_bwd2)
-        return kTwoLevelBlock / h->lanes;
     return g > 1 ? kTwoLevelGroupBlock / 32 * (32 / g) : kTwoLevelBlock;
 }
 
@@ -614,13 +595,66 @@ cudaError_t launch(const va_handle *h, const void *fn, int grid, int block, void
     return cudaLaunchKernel(fn, dim3(grid), dim3(block), args, smem, s);
 }
 
-// Lanes of one warp per quadrant for the sweeps of one lane per instance in
-// their default launch shape, which keep only as many warps busy as the order
-// finds useful beside the longest instance; 0: no such decision (a shape that
-// the caller gave or the autotuner measured stands).
-int rest_lanes(const va_handle *h)
+// SMs for the resting rule of the sweeps of one lane per instance: their
+// default launch shape only (one that the caller gave or the autotuner
+// measured stands)
+int rest_sms(const va_handle *h)
 {
-    return h->ks && h->ks->tpi == 1 && h->lanes == 1 && h->default_shape ? 128 * h->sm_count : 0;
+    return h->ks && h->ks->tpi == 1 && h->default_shape ? h->sm_count : 0;
+}
+
+// Launches the sweep's teams.  By the batch's load, decided on the device:
+// every team whose turn can come (the load is at most the batch size) is
+// launched, and all but one return at once (~2 us each); one_lane tells
+// whether the one-lane sweep can take the batch too, and `a` is then set up
+// for it.  With a launch shape from the caller, or without an order: the one
+// that suits a load of 0.55 B, in that shape.
+template <class Params>
+va_status launch_teams(va_handle *h, int sweep, Params &a, cudaStream_t s, bool &one_lane)
+{
+    const std::vector<va::TeamKernel> &teams = h->teams[sweep];
+    one_lane = true;
+    if (teams.empty())
+        return VA_OK;
+    const int64_t B = h->prob.batch;
+    const float quads = 4.0f * (float)h->sm_count;
+    const bool two_level = sweep == va::FP64_TWO_LEVEL;
+    const bool given = h->opt.block_size > 0 || h->opt.blocks_per_sm > 0;
+    const bool decide = a.load && !given;
+    const int rest = a.rest_sms;
+    a.rest_sms = 0;
+    float from = 0.0f;
+    for (const va::TeamKernel &t : teams) {
+        const float to = t.per_quad * quads;
+        if (!decide && 0.55f * (float)B > to)
+            continue;
+        const int block = two_level ? kTwoLevelBlock : h->opt.block_size > 0 ? h->opt.block_size : 128;
+        int bps = two_level ? kTwoLevelBlocksPerSm : t.bps;
+        if (given && !two_level) {
+            bps = std::max(1, occupancy_of(h, t.fn, block));
+            if (h->opt.blocks_per_sm > 0)
+                bps = std::min(bps, h->opt.blocks_per_sm);
+        }
+        const int64_t need = (B * t.lanes + block - 1) / block;
+        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)h->sm_count * bps));
+        const bool last = !decide || (float)B <= to;
+        a.load_from = from;
+        a.load_to = decide && !(last && from == 0.0f) ? (last ? 3.0e38f : to) : 0.0f;
+        VA_CUDA(h, launch(h, t.fn, grid, block, &a, s));
+        if (!two_level && (last || !decide)) { // what va_get_launch reports
+            (sweep == va::FP64_FORWARD ? h->fwd_team_block : h->bwd_team_block) = block;
+            (sweep == va::FP64_FORWARD ? h->fwd_team_grid : h->bwd_team_grid) = grid;
+        }
+        if (last) {
+            one_lane = false;
+            return VA_OK;
+        }
+        from = to;
+    }
+    a.load_from = from;
+    a.load_to = decide ? 3.0e38f : 0.0f;
+    a.rest_sms = rest;
+    return VA_OK;
 }
 
 va_status enqueue_forward(va_handle *h, const double *y0, const double *params, const double *t0,
@@ -683,15 +717,19 @@ va_status enqueue_forward(va_handle *h, const double *y0, const double *params, 
         h->fwd_grid = grid_for(h, fn, h->fwd_block, a.B);
     if (h->order_fwd) {
         const int *valid = h->inst_work + a.B;
-        va::OrderArgs o{a.B, nullptr, t0, t1, h->inst_work, valid, h->order_work, h->order_fwd, nullptr, rest_lanes(h)};
+        va::OrderArgs o{a.B, nullptr, t0, t1, h->inst_work, valid, h->order_work, h->order_fwd, nullptr};
         VA_CUDA(h, va::enqueue_order(o, s));
         a.order = h->order_fwd;
-        a.warps = o.lanes ? va::order_warps(h->order_work) : nullptr;
-        a.sms = h->sm_count;
+        a.load = va::order_load(h->order_work);
+        a.rest_sms = rest_sms(h);
         a.inst_work = h->inst_work;
         a.work_valid = h->inst_work + a.B;
     }
     VA_CUDA(h, cudaMemsetAsync(h->ctl, 0, sizeof(va::Control), s));
+    bool one_lane;
+    const va_status st = launch_teams(h, va::FP64_FORWARD, a, s, one_lane);
+    if (st != VA_OK || !one_lane)
+        return st;
     VA_CUDA(h, launch(h, fn, h->fwd_grid, h->fwd_block, &a, s));
     return VA_OK;
 }
@@ -721,11 +759,11 @@ va_status enqueue_backward(va_handle *h, const double *params, const double *lam
         // +3%); the lane groups sort by their own step counts (GLV-10: the
         // reused order made the backward 11% slower)
         const int *reuse = h->ks->tpi == 1 ? h->order_fwd : nullptr;
-        va::OrderArgs o{a.B, h->inst_T, nullptr, nullptr, nullptr, nullptr, h->order_work, h->order_bwd, reuse, rest_lanes(h)};
+        va::OrderArgs o{a.B, h->inst_T, nullptr, nullptr, nullptr, nullptr, h->order_work, h->order_bwd, reuse};
         VA_CUDA(h, va::enqueue_order(o, s));
         a.order = h->order_bwd;
-        a.warps = o.lanes ? va::order_warps(h->order_work) : nullptr;
-        a.sms = h->sm_count;
+        a.load = va::order_load(h->order_work);
+        a.rest_sms = rest_sms(h);
     }
     if (h->bks && h->stride > 1) {
         // two-level: segments re-run from the strided checkpoints, in bundles
@@ -821,8 +859,11 @@ va_status enqueue_backward(va_handle *h, const double *params, const double *lam
         a.max_fail = h->opt.max_rejects;
         a.step_pow = h->opt.step_pow;
         VA_CUDA(h, cudaMemsetAsync(&h->ctl->adj_next, 0, sizeof(unsigned int), s));
-        VA_CUDA(h, launch(h, h->sw_bwd2 ? h->sw_bwd2 : h->ks->bwd2[h->opt.tableau][h->opt.precision],
-                          two_level_grid(h), two_level_block(h),
+        bool one_lane;
+        const va_status st = launch_teams(h, va::FP64_TWO_LEVEL, a, s, one_lane);
+        if (st != VA_OK || !one_lane)
+            return st;
+        VA_CUDA(h, launch(h, h->ks->bwd2[h->opt.tableau][h->opt.precision], two_level_grid(h), two_level_block(h),
                           &a, s));
         return VA_OK;
     }
@@ -832,6 +873,10 @@ va_status enqueue_backward(va_handle *h, const double *params, const double *lam
     if (h->bwd_grid <= 0)
         h->bwd_grid = grid_for(h, fn, h->bwd_block, a.B);
     VA_CUDA(h, cudaMemsetAsync(&h->ctl->adj_next, 0, sizeof(unsigned int), s));
+    bool one_lane;
+    const va_status st = launch_teams(h, va::FP64_BACKWARD, a, s, one_lane);
+    if (st != VA_OK || !one_lane)
+        return st;
     VA_CUDA(h, launch(h, fn, h->bwd_grid, h->bwd_block, &a, s));
     return VA_OK;
 }
@@ -858,7 +903,7 @@ struct TunedShape {
 int grid_of(va_handle *h, const void *fn, int block, int bps)
 {
     const int occ = std::max(1, occupancy_of(h, fn, block));
-    const long need = ((long)h->prob.batch * h->lanes + block - 1) / block;
+    const long need = ((long)h->prob.batch * h->ks->tpi + block - 1) / block;
     return (int)std::max(1L, std::min((long)h->sm_count * std::min(bps, occ), need));
 }
 
@@ -1520,13 +1565,13 @@ va_status va_get_launch(const va_handle *h, int32_t *fwd_block, int32_t *fwd_gri
     if (!h)
         return VA_BAD_ARGS;
     if (fwd_block)
-        *fwd_block = h->fwd_block;
+        *fwd_block = h->fwd_team_grid ? h->fwd_team_block : h->fwd_block;
     if (fwd_grid)
-        *fwd_grid = h->fwd_grid;
+        *fwd_grid = h->fwd_team_grid ? h->fwd_team_grid : h->fwd_grid;
     if (bwd_block)
-        *bwd_block = h->bwd_block;
+        *bwd_block = h->bwd_team_grid ? h->bwd_team_block : h->bwd_block;
     if (bwd_grid)
-        *bwd_grid = h->bwd_grid;
+        *bwd_grid = h->bwd_team_grid ? h->bwd_team_grid : h->bwd_grid;
     return VA_OK;
 }
 

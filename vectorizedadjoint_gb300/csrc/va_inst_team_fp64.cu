@@ -7,29 +7,46 @@
 
 namespace va {
 
-template <class M, class Tab, int G>
-static TeamKernels team()
+// Limits: where the next narrower team, or one lane with integer products, is
+// measured faster (forward + backward, ms; load = 0.55 B for Van der Pol T = 20,
+// 0.11 B for the oscillators with horizons to 50).
+//     Van der Pol, 16 / 8 / 4 / 2 lanes, one lane:
+//     B = 1,216   1.96 / 2.72 / 3.51 / 4.67   4.60
+//     B = 2,400   2.79 / 2.72 / 3.50 / 4.68   4.83
+//     B = 4,800   5.25 / 3.95 / 3.51 / 4.69   4.85
+//     B = 9,600   7.44 / 7.67 / 5.47 / 4.66   5.18
+//     B = 19,000  13.3 / 10.8 / 10.2 / 7.70   5.20
+//     oscillators (teams of 16 in two blocks per SM, the others in one):
+//     B = 5,000   10.5 / 12.1 / 15.0 / 19.5   25.0
+//     B = 19,000  12.8 / 13.7 / 15.7 / 21.0   25.6
+// The oscillators gain from wide teams at loads where Van der Pol no longer
+// does (their steps are cheaper beside the fixed part of an attempt); the
+// limits lie between the two.
+// Two-level backward alone, Van der Pol (16 / 8 / 4 / 2, one lane): 4,800: 4.7 /
+// 7.2 / 7.1 / 9.3, 11.1; 9,001: 8.4 / 7.8 / 11.6 / 9.7, 11.0; 12,000: 11.2 / 10.3 /
+// 11.8 / 13.1, 12.5.
+template <class M, class Tab>
+static void fill(TeamKernel (&t)[kFp64Sweeps][kTeams])
 {
-    return {G, (const void *)forward_team_kernel<M, Tab, G>, (const void *)backward_team_kernel<M, Tab, G>,
-            (const void *)backward_team_kernel_2level<M, Tab, G>};
+    t[FP64_FORWARD][0] = {(const void *)forward_team_kernel<M, Tab, 16>, 16, 2, 4.0f};
+    t[FP64_FORWARD][1] = {(const void *)forward_team_kernel<M, Tab, 4>, 4, 1, 6.6f};
+    t[FP64_FORWARD][2] = {(const void *)forward_team_kernel<M, Tab, 2>, 2, 1, 13.0f};
+    t[FP64_BACKWARD][0] = {(const void *)backward_team_kernel<M, Tab, 16>, 16, 2, 4.0f};
+    t[FP64_BACKWARD][1] = {(const void *)backward_team_kernel<M, Tab, 4>, 4, 1, 6.6f};
+    t[FP64_BACKWARD][2] = {(const void *)backward_team_kernel<M, Tab, 2>, 2, 1, 13.0f};
+    t[FP64_TWO_LEVEL][0] = {(const void *)backward_team_kernel_2level<M, Tab, 16>, 16, 2, 6.6f};
+    t[FP64_TWO_LEVEL][1] = {(const void *)backward_team_kernel_2level<M, Tab, 8>, 8, 2, 12.3f};
 }
-
 template <class M>
-static void fill(Fp64Kernels &k)
+static void fill_model(Fp64Kernels &k)
 {
-    k.team[0][0] = team<M, TabDopri5, 16>();
-    k.team[0][1] = team<M, TabDopri5, 8>();
-    k.team[0][2] = team<M, TabDopri5, 4>();
-    k.team[0][3] = team<M, TabDopri5, 2>();
-    k.team[1][0] = team<M, TabCK54, 16>();
-    k.team[1][1] = team<M, TabCK54, 8>();
-    k.team[1][2] = team<M, TabCK54, 4>();
-    k.team[1][3] = team<M, TabCK54, 2>();
+    fill<M, TabDopri5>(k.team[0]);
+    fill<M, TabCK54>(k.team[1]);
 }
 
-void fill_team_vdp(Fp64Kernels &k) { fill<ModelVdP>(k); }
-void fill_team_vdp_petsc(Fp64Kernels &k) { fill<ModelVdPPetsc>(k); }
-void fill_team_dho(Fp64Kernels &k) { fill<ModelDHO>(k); }
-void fill_team_decay(Fp64Kernels &k) { fill<ModelDecay>(k); }
+void fill_team_vdp(Fp64Kernels &k) { fill_model<ModelVdP>(k); }
+void fill_team_vdp_petsc(Fp64Kernels &k) { fill_model<ModelVdPPetsc>(k); }
+void fill_team_dho(Fp64Kernels &k) { fill_model<ModelDHO>(k); }
+void fill_team_decay(Fp64Kernels &k) { fill_model<ModelDecay>(k); }
 
 } // namespace va

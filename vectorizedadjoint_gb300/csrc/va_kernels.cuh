@@ -88,17 +88,26 @@ struct FwdParams {
     int *work_valid; // set to 1 once inst_work holds a sweep's counts (may be null)
     Pool pool;
     Control *ctl;
-    const int *warps;    // device int: warps per SM quadrant to keep busy (may be null: all)
-    int sms;             // SMs (blocks b, b + sms, ... share one)
+    const float *load;   // the batch's load (va_order.cu; device float, may be null: no decisions)
+    float load_from, load_to; // run only for load_from < load <= load_to (load_to 0: any)
+    int rest_sms;        // SMs (blocks b, b + rest_sms, ... share one) for resting, 0: no rest
 };
 
-// Whether this warp stays idle: beyond the warps per quadrant that the order
-// found useful (va_order.cu).
+// Whether another sweep of the same launch takes this batch.
+template <class Params>
+__device__ __forceinline__ bool gated_off(const Params &a)
+{
+    return a.load && a.load_to > 0.0f && !(*a.load > a.load_from && *a.load <= a.load_to);
+}
+// Whether this warp stays idle: beyond the warps per quadrant that are useful
+// beside the longest instance.
 template <class Params>
 __device__ __forceinline__ bool resting(const Params &a)
 {
-    return a.warps &&
-           (int)(blockIdx.x / (unsigned)a.sms * (blockDim.x / 32) + threadIdx.x / 32) >= 4 * *a.warps;
+    if (!a.load || !a.rest_sms)
+        return false;
+    const float warps = fmaxf(1.0f, ceilf(*a.load / (1.25f * 128.0f * (float)a.rest_sms)));
+    return (float)(blockIdx.x / (unsigned)a.rest_sms * (blockDim.x / 32) + threadIdx.x / 32) >= 4.0f * warps;
 }
 
 // Record an instance's attempt count for the next forward sweep's order.
@@ -139,8 +148,9 @@ struct AdjParams {
     // hist[((b * nout + q) * hist_cap + n) * N + i] for record n < hist_cap
     double *hist;
     int hist_cap;
-    const int *warps; // as FwdParams
-    int sms;
+    const float *load; // as FwdParams
+    float load_from, load_to;
+    int rest_sms;
 };
 
 __host__ __device__ constexpr int record_doubles(int n) { return (2 + n + 1) & ~1; }
@@ -661,7 +671,7 @@ __global__ void __launch_bounds__(256) forward_kernel(FwdParams a)
     constexpr int N = M::N, P = M::P;
     constexpr int RS = record_doubles(N);
     const int CH = a.pool.chunk_len;
-    if (resting(a))
+    if (gated_off(a) || resting(a))
         return;
 
     int b = -1;
@@ -983,7 +993,7 @@ __global__ void __launch_bounds__(256) backward_kernel(AdjParams a)
     constexpr int N = M::N, P = M::P;
     constexpr int RS = record_doubles(N);
     const int CH = a.pool.chunk_len;
-    if (resting(a))
+    if (gated_off(a) || resting(a))
         return;
 
     int b = -1, q = 0, j = -1, chunk = -1, slot = 0, T = 0, last = -1;
@@ -1110,6 +1120,8 @@ __global__ void __launch_bounds__(256) backward_kernel_2level(AdjParams a)
     constexpr int N = M::N, P = M::P;
     constexpr int RS = record_doubles(N);
     const int CH = a.pool.chunk_len, SK = a.stride;
+    if (gated_off(a))
+        return;
     double *scr = a.scratch + ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * (SK + 1) * RS;
 
     int b = -1, q = 0, T = 0, R = 0, k = 0, last = -1, chunk = -1, slot = 0, L = 0, done = 0, jb = 0, fails = 0;

@@ -465,7 +465,7 @@ __global__ void __launch_bounds__(256) forward_kernel_dw(FwdParams a)
     constexpr int RS = STAGES ? stage_record_doubles(N, Tab::S) : record_doubles(N);
     const int CH = a.pool.chunk_len;
     const DwTol tol{dword(a.atol), dword(a.rtol)};
-    if (resting(a))
+    if (gated_off(a) || resting(a))
         return;
 
     int b = -1;
@@ -810,7 +810,7 @@ __global__ void __launch_bounds__(256) backward_kernel_dw(AdjParams a)
     static_assert(M::PG == M::P, "parameter adjoint covers every parameter");
     constexpr int RS = STAGES ? stage_record_doubles(N, NS) : record_doubles(N);
     const int CH = a.pool.chunk_len;
-    if (resting(a))
+    if (gated_off(a) || resting(a))
         return;
 
     int b = -1, q = 0, j = -1, chunk = -1, slot = 0, T = 0, last = -1;

@@ -18,20 +18,20 @@
 // second sort, and the backward then visits the checkpoint chunks in the
 // order the forward allocated them (the caller decides; one-thread models).
 //
-// The sort also decides how many warps a one-thread sweep keeps busy.  More
-// warps per SM quadrant raise the throughput (1.9x with four, double-word
-// Van der Pol) but slow each of them by more, and with uneven lengths the
-// sweep ends with its longest instance.  One warp per quadrant finishes the
-// whole batch in max(longest, sum of lengths / lanes) steps of the fastest
-// kind; when the second is not above the first, the longest instance sets the
-// pace and every other resident warp only delays it.  Measured, forward +
-// backward: 65,536 double-word oscillators (lengths to 1,737, mean ~190) 5.15
-// ms with one warp, 6.44 with four; FP64 27.0 against 32.1 with two;
-// Van der Pol (lengths within 2x of the mean) 262,144 instances 8.25 ms with
-// one warp, 5.11 with four; 20,000 instances, which fill one warp per
-// quadrant, 1.06 against 1.23; 65,536 instances (sum = 1.9 longest x lanes)
-// 2.31 with one warp, 1.57 with two, 1.90 with four.  So the sweep keeps
-// ceil(sum / (1.25 longest lanes)) warps per quadrant busy.
+// The sort also leaves the batch's load, sum(length) / max(length), by which
+// the one-thread sweeps choose on the device how many warps they keep busy
+// (resting) and how many lanes carry an instance (gated_off): with uneven
+// lengths the longest instance sets the pace, and whatever shares its SM
+// quadrant only delays it.  More warps per quadrant raise the throughput
+// (1.9x with four, double-word Van der Pol) but slow each of them by more.
+// One warp per quadrant finishes a batch in max(1, load / lanes) times its
+// longest instance; the sweeps keep ceil(load / (1.25 lanes)) warps per
+// quadrant.  Measured, forward + backward: 65,536 double-word oscillators
+// (lengths to 1,737, mean ~190: load 0.4 lanes) 5.15 ms with one warp, 6.44
+// with four; FP64 27.0 against 32.1 with two; Van der Pol (mean 0.55 of the
+// longest) 20,000 instances (0.6) 1.06 with one, 1.23 with four; 65,536 (1.9)
+// 2.31 with one, 1.57 with two, 1.90 with four; 262,144 (7.4) 8.25 with one,
+// 5.11 with four.
 #include <cuda_runtime.h>
 
 #include <cstdint>
@@ -59,8 +59,8 @@ __device__ __forceinline__ int count_bucket(int n) { return n < kBuckets ? (n < 
 // work[2 kBuckets]: 1 when the last forward order came from step counts
 constexpr int kCountedFlag = 2 * kBuckets;
 
-// work[2 kBuckets + 1]: warps per quadrant to keep busy
-constexpr int kWarpsSlot = kCountedFlag + 1;
+// work[2 kBuckets + 1]: the load (a float)
+constexpr int kLoadSlot = kCountedFlag + 1;
 
 // the backward reuses the forward's order when that one was count-based
 __device__ __forceinline__ bool reusing(const OrderArgs &a) { return a.reuse && a.work[kCountedFlag] == 1; }
@@ -125,32 +125,31 @@ __global__ void order_scan(OrderArgs a)
     const bool prev = a.prev_work && a.prev_valid && *a.prev_valid;
     if (t == 0 && !a.steps) // a forward order: say whether it came from counts
         a.work[kCountedFlag] = prev ? 1 : 0;
-    if (a.lanes > 0) {
-        __shared__ float sum[32], top[32];
-        const bool counted = a.steps || prev;
-        float s1 = 0.0f, m1 = 0.0f;
-        for (int j = 0; j < 4; j++) {
-            const float l = v[j] ? bucket_length(counted, kBuckets - 1 - (t * 4 + j)) : 0.0f;
-            s1 += l * (float)v[j];
-            m1 = fmaxf(m1, l);
+    __shared__ float sum[32], top[32];
+    const bool counted = a.steps || prev;
+    float s1 = 0.0f, m1 = 0.0f;
+    for (int j = 0; j < 4; j++) {
+        const float l = v[j] ? bucket_length(counted, kBuckets - 1 - (t * 4 + j)) : 0.0f;
+        s1 += l * (float)v[j];
+        m1 = fmaxf(m1, l);
+    }
+    for (int o = 16; o; o >>= 1) {
+        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+        m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+    }
+    if ((t & 31) == 0) {
+        sum[t >> 5] = s1;
+        top[t >> 5] = m1;
+    }
+    __syncthreads();
+    if (t == 0) {
+        for (int w = 1; w < 32; w++) {
+            s1 += sum[w];
+            m1 = fmaxf(m1, top[w]);
         }
-        for (int o = 16; o; o >>= 1) {
-            s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-            m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
-        }
-        if ((t & 31) == 0) {
-            sum[t >> 5] = s1;
-            top[t >> 5] = m1;
-        }
-        __syncthreads();
-        if (t == 0) {
-            for (int w = 1; w < 32; w++) {
-                s1 += sum[w];
-                m1 = fmaxf(m1, top[w]);
-            }
-            const float w = m1 > 0.0f ? ceilf(s1 / (1.25f * m1 * (float)a.lanes)) : 1.0f;
-            a.work[kWarpsSlot] = w < 64.0f ? max(1, (int)w) : 64;
-        }
+        // at most one per instance, at least one instance's (a batch of length 0 too)
+        const float load = m1 > 0.0f ? s1 / m1 : 1.0f;
+        a.work[kLoadSlot] = __float_as_int(fminf(fmaxf(load, 1.0f), (float)a.B));
     }
 }
 
@@ -187,7 +186,7 @@ __global__ void __launch_bounds__(1024) order_scatter(OrderArgs a)
 } // namespace
 
 size_t order_work_ints() { return 2 * kBuckets + 2; }
-const int *order_warps(const int *work) { return work + kWarpsSlot; }
+const float *order_load(const int *work) { return reinterpret_cast<const float *>(work + kLoadSlot); }
 
 cudaError_t enqueue_order(const OrderArgs &a, cudaStream_t s)
 {

@@ -18,14 +18,12 @@ struct OrderArgs {
     int *order;        // [B] output permutation, longest first
     const int *reuse;  // backward: the forward's order, copied instead of sorting when
                        //   that order came from counts (flag in work); may be null
-    int lanes;         // lanes of one warp per SM quadrant over the whole GPU (0: no
-                       //   decision about resident warps, order_warps)
 };
 
 size_t order_work_ints();
-// In `work`, on the device: the warps per quadrant that the sweep should keep
-// busy, set with the order (see va_order.cu).
-const int *order_warps(const int *work);
+// In `work`, on the device: the batch's load, the sum of its instances'
+// lengths in units of the longest, set with the order (see va_order.cu).
+const float *order_load(const int *work);
 cudaError_t enqueue_order(const OrderArgs &a, cudaStream_t s);
 
 } // namespace va

@@ -91,14 +91,17 @@ void fill_fixed_glv10(KernelSet &k);
 // Further FP64 sweeps of a built-in one-thread model (fp64_path in va_api.cu
 // chooses): products on the integer pipe (va_step64.cuh) and teams of g lanes
 // per instance (va_team64.cuh).  Null: not compiled.
-struct TeamKernels {
-    int g;
-    const void *fwd, *bwd, *bwd2; // bwd2: two-level backward
+struct TeamKernel {
+    const void *fn;
+    int lanes;       // per instance
+    int bps;         // resident blocks of 128 threads per SM
+    float per_quad;  // highest load, per SM quadrant, that the team takes
 };
-constexpr int kTeams = 4;
+enum { FP64_FORWARD = 0, FP64_BACKWARD = 1, FP64_TWO_LEVEL = 2, kFp64Sweeps = 3 };
+constexpr int kTeams = 3;
 struct Fp64Kernels {
     const void *int_fwd[kTableaux], *int_bwd[kTableaux];
-    TeamKernels team[kTableaux][kTeams]; // widest first
+    TeamKernel team[kTableaux][kFp64Sweeps][kTeams]; // widest first
 };
 // the team sweeps (va_inst_team_fp64.cu, va_inst_team_rkf78_fp64.cu)
 void fill_team_vdp(Fp64Kernels &k);

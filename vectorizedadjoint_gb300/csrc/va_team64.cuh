@@ -382,6 +382,8 @@ __global__ void __launch_bounds__(256) forward_team_kernel(FwdParams a)
 {
     constexpr int N = M::N, P = M::P;
     constexpr int RS = record_doubles(N);
+    if (gated_off(a))
+        return;
     const TeamForward<M, Tab, G> tf;
     const bool first = tf.team.index == 0;
     const int CH = a.pool.chunk_len;
@@ -599,6 +601,8 @@ __global__ void __launch_bounds__(256) backward_team_kernel(AdjParams a)
     constexpr int N = M::N, P = M::P;
     constexpr int RS = record_doubles(N);
     using TB = TeamBackward<M, Tab, G>;
+    if (gated_off(a))
+        return;
     const TB tb;
     const int me = tb.team.index;
     const bool first = me == 0;
@@ -706,6 +710,8 @@ __global__ void __launch_bounds__(256) backward_team_kernel_2level(AdjParams a)
 {
     constexpr int N = M::N, P = M::P;
     constexpr int RS = record_doubles(N);
+    if (gated_off(a))
+        return;
     const TeamForward<M, Tab, G> tf;
     const TeamBackward<M, Tab, G> tb;
     const bool first = tb.team.index == 0;
