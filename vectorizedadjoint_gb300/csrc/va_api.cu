@@ -218,7 +218,7 @@ const void *bwd_kernel(const va_handle *h)
 // 30,000 instances 7.0 ms with 256 x 1, 6.8 with 128 x 1.
 void fp64_path(va_handle *h)
 {
-    const va::Fp64Kernels *k = h->user || !h->ks ? nullptr : va::fp64_kernels(h->prob.model);
+    const va::Fp64Kernels *k = h->user || !h->ks ? nullptr : va::fp64_kernels(h->prob.model, h->N);
     if (!k || h->opt.precision != VA_PREC_FP64)
         return;
     const int t = h->opt.tableau;
@@ -229,9 +229,11 @@ void fp64_path(va_handle *h)
                     h->teams[w].push_back(c);
     if (!k->int_fwd[t])
         return;
-    h->sw_fwd = k->int_fwd[t];
-    h->sw_bwd = k->int_bwd[t];
-    if (h->opt.block_size <= 0 && h->opt.blocks_per_sm <= 0) {
+    if (h->prob.batch >= k->int_fwd_min)
+        h->sw_fwd = k->int_fwd[t];
+    if (h->prob.batch >= k->int_bwd_min)
+        h->sw_bwd = k->int_bwd[t];
+    if (h->ks->tpi == 1 && h->opt.block_size <= 0 && h->opt.blocks_per_sm <= 0) {
         h->fwd_block = h->bwd_block = h->prob.batch > 256 * h->sm_count ? 256 : 128;
         h->bps = 1;
     }

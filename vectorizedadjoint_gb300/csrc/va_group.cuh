@@ -90,37 +90,93 @@ struct ModelGLVLane {
         }
     }
 
-    // f_i = x_i (r_i + sum_j A_ij x_j)
+    // r_i + sum_j A_ij x_j
     template <class S>
-    __device__ __forceinline__ static void rhs(const S *x, const S *p, S t, S *f)
+    __device__ __forceinline__ static S rate(const S *x, const S *p)
     {
-        (void)t;
         const LaneGroup<NN> G;
         S acc = S(0);
 #pragma unroll
         for (int j = 0; j < NN; j++)
             acc = madd(p[1 + j], shfl(x[0], G.base + j, G.mask), acc);
-        f[0] = x[0] * (p[0] + acc);
+        return p[0] + acc;
+    }
+    // f_i = x_i (r_i + sum_j A_ij x_j)
+    template <class S>
+    __device__ __forceinline__ static void rhs(const S *x, const S *p, S t, S *f)
+    {
+        (void)t;
+        f[0] = x[0] * rate<S>(x, p);
     }
 
     // gx_k = w_k s_k + sum_i A_ik w_i x_i ; gr_k = w_k x_k ; gA_kj = w_k x_k x_j
+    // at a point whose rate is known: the recompute of a back step forms the
+    // rates of its stages (all but the last), a sixth of the step's FP64
+    // instructions at N = 5
+    template <class S>
+    __device__ __forceinline__ static void vjp_rate(const S *w, const S *x, S s, const S *p, S *gx, S *gp)
+    {
+        const LaneGroup<NN> G;
+        const S v = w[0] * x[0];
+#pragma unroll
+        for (int j = 0; j < NN; j++)
+            gp[1 + j] = v * shfl(x[0], G.base + j, G.mask);
+        S g = w[0] * s;
+#pragma unroll
+        for (int j = 0; j < NN; j++)
+            g = madd(p[1 + NN + j], shfl(v, G.base + j, G.mask), g);
+        gx[0] = g;
+        gp[0] = v;
+    }
     template <class S>
     __device__ __forceinline__ static void vjp(const S *w, const S *x, const S *p, S t, S *gx, S *gp)
     {
         (void)t;
+        vjp_rate<S>(w, x, rate<S>(x, p), p, gx, gp);
+    }
+
+    // the same with the products on the integer pipe (va_step64.cuh): the
+    // factors that cross lanes are exchanged unpacked
+    static constexpr bool kProducts64 = true;
+    __device__ __forceinline__ static MulR from_lane(const MulR &v, int src, unsigned mask)
+    {
+        return {__shfl_sync(mask, v.h, src), __shfl_sync(mask, v.l, src), __shfl_sync(mask, v.e, src)};
+    }
+    // 0 + v
+    __device__ __forceinline__ static double from_zero(double v) { return f64_bits(v) == 1ull << 63 ? 0.0 : v; }
+    __device__ __forceinline__ static void rhs64(const double *x, const double *p, double *f, MulRange &r)
+    {
         const LaneGroup<NN> G;
-        const S v = w[0] * x[0];
-        S s = S(0);
+        const MulR xr = mul_right(x[0], r);
+        double acc = 0.0;
 #pragma unroll
         for (int j = 0; j < NN; j++) {
-            const S xj = shfl(x[0], G.base + j, G.mask);
-            s = madd(p[1 + j], xj, s);
-            gp[1 + j] = v * xj;
+            const double term = mul_rn(mul_left_in(p[1 + j]), from_lane(xr, G.base + j, G.mask));
+            acc = j == 0 ? from_zero(term) : term + acc;
         }
-        S g = w[0] * (p[0] + s);
+        f[0] = mul_rn(mul_left_in(p[0] + acc), xr);
+    }
+    __device__ __forceinline__ static void vjp64(const double *w, const double *x, const double *p, double *gx,
+                                                 double *gp, MulRange &r)
+    {
+        const LaneGroup<NN> G;
+        const MulR xr = mul_right(x[0], r);
+        const MulL wl = mul_left(w[0], r);
+        const double v = mul_rn(wl, xr);
+        const MulL vl = mul_left_in(v);
+        const MulR vr = mul_right_in(v);
+        double s = 0.0;
+#pragma unroll
+        for (int j = 0; j < NN; j++) {
+            const MulR xj = from_lane(xr, G.base + j, G.mask);
+            const double term = mul_rn(mul_left_in(p[1 + j]), xj);
+            s = j == 0 ? from_zero(term) : term + s;
+            gp[1 + j] = mul_rn(vl, xj);
+        }
+        double g = mul_rn(wl, mul_right_in(p[0] + s));
 #pragma unroll
         for (int j = 0; j < NN; j++)
-            g = madd(p[1 + NN + j], shfl(v, G.base + j, G.mask), g);
+            g = mul_rn(mul_left_in(p[1 + NN + j]), from_lane(vr, G.base + j, G.mask)) + g;
         gx[0] = g;
         gp[0] = v;
     }
@@ -159,7 +215,7 @@ __device__ __forceinline__ void accept_state_group(double (&y)[1], S (&ys)[1], S
 
 // ------------------------------------------------------------ forward sweep
 
-template <class M, class Tab, class S>
+template <class M, class Tab, class S, bool INT64 = false>
 __global__ void __launch_bounds__(256) forward_group_kernel(FwdParams a)
 {
     constexpr int G = M::TPI, NT = M::NTOT, PT = M::PTOT, P = M::P;
@@ -304,7 +360,7 @@ __global__ void __launch_bounds__(256) forward_group_kernel(FwdParams a)
         double ynew[1];
         S ynew_s[1], knew[1];
         const double err = group_max<G>(
-            attempt<M, Tab, S>(y, ys, k0, p, t, dt, a.atol, a.rtol, ynew, ynew_s, knew), mask);
+            attempt<M, Tab, S, INT64>(y, ys, k0, p, t, dt, a.atol, a.rtol, ynew, ynew_s, knew), mask);
         bool ok;
         if (is_nan64(err)) {
             status = ST_NONFINITE;
@@ -340,7 +396,7 @@ __global__ void __launch_bounds__(256) forward_group_kernel(FwdParams a)
 
 // ----------------------------------------------------------- backward sweep
 
-template <class M, class Tab, class S>
+template <class M, class Tab, class S, bool INT64 = false>
 __global__ void __launch_bounds__(256) backward_group_kernel(AdjParams a)
 {
     constexpr int G = M::TPI, NT = M::NTOT, PT = M::PTOT, P = M::P, PG = M::PG;
@@ -437,7 +493,7 @@ __global__ void __launch_bounds__(256) backward_group_kernel(AdjParams a)
         const double tn = r[0];
         double y[1] = {r[2 + li]};
         const double h = t_next - tn;
-        back_step<M, Tab, S>(y, tn, h, p, lam, mu);
+        back_step<M, Tab, S, INT64>(y, tn, h, p, lam, mu);
         note_lambda_lane(a, b, q, j, NT, li, lam[0]);
         t_next = tn;
         j--;

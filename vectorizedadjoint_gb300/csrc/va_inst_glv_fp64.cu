@@ -15,6 +15,34 @@ static void fill(KernelSet &k)
     k.bwd[1][0] = (const void *)backward_group_kernel<M, TabCK54, double>;
 }
 
+// With the products on the integer pipe (va_step64.cuh).  Forward, 16,384
+// instances: N = 10 3.96 -> 2.85 ms, N = 5 1.70 -> 1.21; 777 instances: N = 10
+// 0.88 -> 0.71, N = 5 the same.  Backward, 16,384 instances: N = 5 3.16 -> 2.52;
+// N = 10 needs more registers than there are (9.1 -> 9.3), and with few warps
+// the longer code loses for both (777 instances, N = 5: 1.04 -> 1.41).
+// (one instance, N = 10: 0.48 -> 0.51 forward.)
+constexpr int kTwoWarps5 = 2 * 608 * 6; // groups of 5 that fill two warps per quadrant of 152 SMs
+template <int NN>
+static Fp64Kernels make_int()
+{
+    using M = ModelGLVLane<NN>;
+    Fp64Kernels k{};
+    k.int_fwd[0] = (const void *)forward_group_kernel<M, TabDopri5, double, true>;
+    k.int_fwd[1] = (const void *)forward_group_kernel<M, TabCK54, double, true>;
+    if constexpr (NN == 5) {
+        k.int_bwd[0] = (const void *)backward_group_kernel<M, TabDopri5, double, true>;
+        k.int_bwd[1] = (const void *)backward_group_kernel<M, TabCK54, double, true>;
+    }
+    k.int_fwd_min = NN == 5 ? kTwoWarps5 : 32;
+    k.int_bwd_min = kTwoWarps5;
+    return k;
+}
+const Fp64Kernels *fp64_kernels_glv(int n)
+{
+    static const Fp64Kernels k5 = make_int<5>(), k10 = make_int<10>();
+    return n == 5 ? &k5 : n == 10 ? &k10 : nullptr;
+}
+
 void fill_fp64_glv5(KernelSet &k) { fill<5>(k); }
 void fill_fp64_glv10(KernelSet &k) { fill<10>(k); }
 

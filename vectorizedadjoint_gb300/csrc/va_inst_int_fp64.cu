@@ -21,7 +21,7 @@ static Fp64Kernels make(void (*team)(Fp64Kernels &), void (*rkf78)(Fp64Kernels &
     return k;
 }
 
-const Fp64Kernels *fp64_kernels(int model)
+const Fp64Kernels *fp64_kernels(int model, int n)
 {
     static const Fp64Kernels vdp = make<ModelVdP>(fill_team_vdp, fill_team_rkf78_vdp),
                              petsc = make<ModelVdPPetsc>(fill_team_vdp_petsc, fill_team_rkf78_vdp_petsc),
@@ -30,7 +30,8 @@ const Fp64Kernels *fp64_kernels(int model)
     return model == VA_MODEL_VDP ? &vdp
          : model == VA_MODEL_VDP_PETSC ? &petsc
          : model == VA_MODEL_DHO ? &dho
-         : model == VA_MODEL_DECAY ? &decay : nullptr;
+         : model == VA_MODEL_DECAY ? &decay
+         : model == VA_MODEL_GLV ? fp64_kernels_glv(n) : nullptr;
 }
 
 } // namespace va

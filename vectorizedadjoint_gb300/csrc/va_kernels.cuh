@@ -841,6 +841,15 @@ __global__ void __launch_bounds__(256) forward_kernel(FwdParams a)
 
 // ----------------------------------------------------------- backward sweep
 
+// Models that share a part of f between the right-hand side and the VJP at the
+// same point (rate, vjp_rate: the lane-group Lotka-Volterra model).
+template <class M, class S, class = void>
+struct HasRate : std::false_type {
+};
+template <class M, class S>
+struct HasRate<M, S, std::void_t<decltype(M::template rate<S>(nullptr, nullptr))>> : std::true_type {
+};
+
 // One back_prop_step (backpropagation.hpp:160-229) for step n with state y_n,
 // start time tn and h = t_{n+1} - t_n.  lam: in lambda_{n+1}, out lambda_n.
 template <class M, class Tab, class S>
@@ -856,12 +865,25 @@ __host__ __device__ __forceinline__ void back_step_general(const double (&y)[M::
     for (int i = 0; i < N; i++)
         ys[i] = from_d<S>(y[i]);
     const S shh = from_d<S>(h);
+    constexpr bool RATE = HasRate<M, S>::value;
+    S rate[NS];
     // recompute the stages from y_n (compute_intermediate_states, :24-64)
 #pragma unroll
     for (int m = 0; m < NS; m++) {
         form_stage<Tab, N, S>(m, y, ys, K, h, shh, X[m]);
-        M::template rhs<S>(X[m], p, from_d<S>(tn + Tab::c(m) * h), K[m]);
+        if constexpr (RATE) {
+            rate[m] = M::template rate<S>(X[m], p);
+            K[m][0] = X[m][0] * rate[m];
+        } else {
+            M::template rhs<S>(X[m], p, from_d<S>(tn + Tab::c(m) * h), K[m]);
+        }
     }
+    auto vjp = [&](int m, const S (&w)[N], S (&gx)[N], S (&gp)[P]) {
+        if constexpr (RATE)
+            M::template vjp_rate<S>(w, X[m], rate[m], p, gx, gp);
+        else
+            M::template vjp<S>(w, X[m], p, from_d<S>(tn + Tab::c(m) * h), gx, gp);
+    };
     S Kbar[NS][N];
     if constexpr (std::is_same<S, double>::value) {
         // seeds: ybar = lambda, Kbar_m = (b_m h) lambda  (:178-184)
@@ -877,7 +899,7 @@ __host__ __device__ __forceinline__ void back_step_general(const double (&y)[M::
 #pragma unroll
         for (int m = NS - 1; m >= 0; m--) {
             S gx[N], gp[P];
-            M::template vjp<S>(Kbar[m], X[m], p, S(tn + Tab::c(m) * h), gx, gp);
+            vjp(m, Kbar[m], gx, gp);
 #pragma unroll
             for (int i = 0; i < N; i++) {
                 ybar[i] += gx[i];
@@ -912,7 +934,7 @@ __host__ __device__ __forceinline__ void back_step_general(const double (&y)[M::
 #pragma unroll
         for (int m = NS - 1; m >= 0; m--) {
             S gx[N], gp[P];
-            M::template vjp<S>(Kbar[m], X[m], p, from_d<S>(tn + Tab::c(m) * h), gx, gp);
+            vjp(m, Kbar[m], gx, gp);
 #pragma unroll
             for (int i = 0; i < N; i++) {
                 dx[i] = m == NS - 1 ? gx[i] : dx[i] + gx[i];

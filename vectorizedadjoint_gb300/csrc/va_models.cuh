@@ -81,12 +81,12 @@ struct ModelVdP {
     {
         const double a = 1.0 - mul_rn(mul_left(x[0], r), mul_right_in(x[0]));
         f[0] = x[1];
-        f[1] = mul_rn(mul_left_in(mul_rn(mul_left_in(a), mul_right(p[0], r))), mul_right(x[1], r)) - x[0];
+        f[1] = mul_rn(mul_left_in(mul_rn(mul_left_in(a), mul_right_in(p[0]))), mul_right(x[1], r)) - x[0];
     }
     __host__ __device__ __forceinline__ static void vjp64(const double *w, const double *x, const double *p,
                                                           double *gx, double *gp, MulRange &r)
     {
-        const MulR x1 = mul_right(x[1], r), mu = mul_right(p[0], r);
+        const MulR x1 = mul_right(x[1], r), mu = mul_right_in(p[0]);
         const MulL w1 = mul_left(w[1], r), x0 = mul_left(x[0], r);
         const double a = 1.0 - mul_rn(x0, mul_right_in(x[0]));
         const MulL al = mul_left_in(a);
@@ -141,12 +141,12 @@ struct ModelVdPPetsc {
     {
         const double a = 1.0 - mul_rn(mul_left(x[0], r), mul_right_in(x[0]));
         f[0] = x[1];
-        f[1] = mul_rn(mul_left_in(mul_rn(mul_left_in(a), mul_right(x[1], r)) - x[0]), mul_right(p[0], r));
+        f[1] = mul_rn(mul_left_in(mul_rn(mul_left_in(a), mul_right(x[1], r)) - x[0]), mul_right_in(p[0]));
     }
     __host__ __device__ __forceinline__ static void vjp64(const double *w, const double *x, const double *p,
                                                           double *gx, double *gp, MulRange &r)
     {
-        const MulR x1 = mul_right(x[1], r), mu = mul_right(p[0], r);
+        const MulR x1 = mul_right(x[1], r), mu = mul_right_in(p[0]);
         const MulL w1 = mul_left(w[1], r), x0 = mul_left(x[0], r);
         const double a = 1.0 - mul_rn(x0, mul_right_in(x[0]));
         const MulL al = mul_left_in(a);
@@ -207,7 +207,7 @@ struct ModelDHO {
     static constexpr bool kProducts64 = true;
     __host__ __device__ __forceinline__ static void rhs64(const double *x, const double *p, double *f, MulRange &r)
     {
-        const MulL om = mul_left(p[0], r), ze = mul_left(p[1], r);
+        const MulL om = mul_left_in(p[0]), ze = mul_left_in(p[1]);
         const MulR omr = mul_right_in(p[0]);
         const double k = mul_rn(mul_neg(om), omr), c = mul_rn(mul_m2(ze), omr); // -om om, -2 ze om
         f[0] = x[1];
@@ -216,7 +216,7 @@ struct ModelDHO {
     __host__ __device__ __forceinline__ static void vjp64(const double *w, const double *x, const double *p,
                                                           double *gx, double *gp, MulRange &r)
     {
-        const MulL om = mul_left(p[0], r), ze = mul_left(p[1], r), w1 = mul_left(w[1], r);
+        const MulL om = mul_left_in(p[0]), ze = mul_left_in(p[1]), w1 = mul_left(w[1], r);
         const MulR omr = mul_right_in(p[0]), x0 = mul_right(x[0], r), x1 = mul_right(x[1], r);
         gx[0] = mul_rn(w1, mul_right_in(mul_rn(mul_neg(om), omr)));
         gx[1] = w[0] + mul_rn(w1, mul_right_in(mul_rn(mul_m2(ze), omr)));
@@ -254,13 +254,13 @@ struct ModelDecay {
     static constexpr bool kProducts64 = true;
     __host__ __device__ __forceinline__ static void rhs64(const double *x, const double *p, double *f, MulRange &r)
     {
-        f[0] = mul_rn(mul_neg(mul_left(p[0], r)), mul_right(x[0], r));
+        f[0] = mul_rn(mul_neg(mul_left_in(p[0])), mul_right(x[0], r));
     }
     __host__ __device__ __forceinline__ static void vjp64(const double *w, const double *x, const double *p,
                                                           double *gx, double *gp, MulRange &r)
     {
         const MulR wr = mul_right(w[0], r);
-        gx[0] = mul_rn(mul_neg(mul_left(p[0], r)), wr);
+        gx[0] = mul_rn(mul_neg(mul_left_in(p[0])), wr);
         gp[0] = mul_rn(mul_neg(mul_left(x[0], r)), wr);
     }
     static constexpr int kVjpW = 0, kVjpAdd = -1;

@@ -101,6 +101,7 @@ enum { FP64_FORWARD = 0, FP64_BACKWARD = 1, FP64_TWO_LEVEL = 2, kFp64Sweeps = 3 
 constexpr int kTeams = 3;
 struct Fp64Kernels {
     const void *int_fwd[kTableaux], *int_bwd[kTableaux];
+    int int_fwd_min, int_bwd_min; // smallest batches they take
     TeamKernel team[kTableaux][kFp64Sweeps][kTeams]; // widest first
 };
 // the team sweeps (va_inst_team_fp64.cu, va_inst_team_rkf78_fp64.cu)
@@ -112,7 +113,8 @@ void fill_team_rkf78_vdp(Fp64Kernels &k);
 void fill_team_rkf78_vdp_petsc(Fp64Kernels &k);
 void fill_team_rkf78_dho(Fp64Kernels &k);
 void fill_team_rkf78_decay(Fp64Kernels &k);
-const Fp64Kernels *fp64_kernels(int model); // null: none for the model
+const Fp64Kernels *fp64_kernels(int model, int n); // null: none for the model
+const Fp64Kernels *fp64_kernels_glv(int n);
 
 // Shared-matrix GLV: bundles of kBundleNB instances per CTA of N threads
 // (FP64, FP32); the double-word sweeps take bundles of kBundleNBdw, whose

@@ -43,6 +43,17 @@ template <class M>
 struct HasProducts64<M, std::void_t<decltype(M::kProducts64)>> : std::bool_constant<M::kProducts64> {
 };
 
+// the model's parameters into the range, once per step (rhs64 and vjp64 take
+// them as noted)
+template <class M>
+__host__ __device__ __forceinline__ void note_params64(const double (&p)[M::P], MulRange &r)
+{
+    if constexpr (HasProducts64<M>::value) {
+#pragma unroll
+        for (int k = 0; k < M::P; k++)
+            r.note(f64_hi(p[k]), f64_lo(p[k]));
+    }
+}
 template <class M>
 __host__ __device__ __forceinline__ void model_rhs64(const double *x, const double *p, double t, double *f,
                                                      MulRange &r)
@@ -128,6 +139,7 @@ __host__ __device__ __forceinline__ bool attempt64(const double (&y)[M::N], cons
 {
     constexpr int N = M::N, NS = Tab::S;
     MulRange r;
+    note_params64<M>(p, r);
     const MulR h = mul_right(dt, r);
     MulL K[NS][N];
     bool neg_zero = false;
@@ -210,6 +222,7 @@ __host__ __device__ __forceinline__ bool back_step64(const double (&y)[M::N], do
 {
     constexpr int N = M::N, P = M::PG, NS = Tab::S;
     MulRange r;
+    note_params64<M>(p, r);
     const MulR h = mul_right(hh, r);
     double X[NS][N];
     bool neg_zero = false;
