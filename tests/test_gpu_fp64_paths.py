@@ -119,3 +119,24 @@ def test_choice_by_load(oracle, cuda, tab, stride, even, B):
     for r in res[1:]:
         for a, b in zip(r, res[0]):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("N,B", [(5, 7), (5, 7400), (10, 7), (10, 300)])
+@pytest.mark.parametrize("tab", ["dopri5", "ck54"])
+def test_lotka_volterra_special_values_bit_exact(oracle, cuda, N, B, tab):
+    """Lane groups with integer products (N = 10 forward always, N = 5 where the batch fills two warps per quadrant): zero
+    and huge entries of A, r and x on some lanes only, beside ordinary groups of the same warp."""
+    rng = np.random.default_rng(N + B)
+    A = rng.normal(0, 0.1, (B, N, N))
+    A[:, np.arange(N), np.arange(N)] = -1.0
+    r, y0, t1 = rng.uniform(0.5, 1.5, (B, N)), rng.uniform(0.1, 1.0, (B, N)), np.full(B, 2.0)
+    A[0][np.arange(N) != np.arange(N)[:, None]] = 0.0
+    y0[1, 2], r[1, 0] = 0.0, -0.0
+    y0[2, 1] = 1e-100
+    A[3, 1, 2] = 1e-90
+    y0[4] = 0.0
+    A[5, 0, 3], y0[5, 3] = -1e80, 1e-79
+    y0[6, 0] = np.inf
+    p = np.concatenate([r, A.reshape(B, N * N)], 1)
+    NP["glv"] = N + N * N
+    check(oracle, "glv", tab, y0, p, t1, sorted({*range(7), B // 2, B - 1}))

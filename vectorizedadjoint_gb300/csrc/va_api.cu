@@ -207,7 +207,7 @@ const void *bwd_kernel(const va_handle *h)
 // (va_inst_team_fp64.cu, va_inst_team_rkf78_fp64.cu).
 //
 // One lane per instance for larger ones, with the products on the integer pipe
-// for the 5(4) pairs (va_step64.cuh): Van der Pol with 65,536 instances 9.2 ms
+// for the 5(4) pairs (va_step64.cuh): Van der Pol with 65,536 instances 8.4 ms
 // against 19.6 ms with FP64 products.  Fehlberg 7(8) and the two-level backward
 // keep the FP64 products there: their code is too long for the instruction
 // caches that way (16.1 against 9.8 ms with 5,003 instances, 24.7 against 14.0

@@ -7,6 +7,14 @@
 // are bound by the FP64 instruction count at every batch size.  A product in
 // integers issues in ~45 cycles beside the sums.
 //
+// Not every product: with all of them in integers the FP64 unit waits for the
+// integer pipe and the instruction fetch.  Left to the FP64 unit: the forward's
+// right-hand side of the one-lane models (a chain of products, short of
+// independent work; 65,536 Van der Pol instances forward 3.94 -> 3.81 ms) and
+// the second product of each K-bar term (backward 5.22 -> 4.58; the recompute's
+// right-hand sides as well 4.99, the coefficients c h as well 5.1; the error's
+// terms of one component 4.17 forward).
+//
 // The operations and their order are those of attempt_pair, step_fixed and
 // back_step; every sum is the FP64 instruction and every product the
 // correctly rounded one, so the results have the same bits.  A coefficient
@@ -54,11 +62,11 @@ __host__ __device__ __forceinline__ void note_params64(const double (&p)[M::P], 
             r.note(f64_hi(p[k]), f64_lo(p[k]));
     }
 }
-template <class M>
+template <class M, bool FORWARD = false>
 __host__ __device__ __forceinline__ void model_rhs64(const double *x, const double *p, double t, double *f,
                                                      MulRange &r)
 {
-    if constexpr (HasProducts64<M>::value) {
+    if constexpr (HasProducts64<M>::value && !(FORWARD && M::kForwardRhsFp64)) {
         (void)t;
         M::rhs64(x, p, f, r);
     } else {
@@ -153,7 +161,7 @@ __host__ __device__ __forceinline__ bool attempt64(const double (&y)[M::N], cons
     for (int m = 1; m < NS; m++) {
         double X[N], f[N];
         form_stage64<Tab, N>(m, y, K, h, X);
-        model_rhs64<M>(X, p, t + Tab::c(m) * dt, f, r);
+        model_rhs64<M, true>(X, p, t + Tab::c(m) * dt, f, r);
 #pragma unroll
         for (int i = 0; i < N; i++)
             K[m][i] = mul_left(f[i], r);
@@ -186,7 +194,7 @@ __host__ __device__ __forceinline__ bool attempt64(const double (&y)[M::N], cons
                 first = false;
             }
         if constexpr (Tab::FSAL) {
-            model_rhs64<M>(ynew, p, t + dt, knew, r);
+            model_rhs64<M, true>(ynew, p, t + dt, knew, r);
             const MulR c = coef_right(Tab::E_NEW, h);
 #pragma unroll
             for (int i = 0; i < N; i++)
@@ -277,7 +285,7 @@ __host__ __device__ __forceinline__ bool back_step64(const double (&y)[M::N], do
             for (int k = 0; k < NS - 1; k++)
                 if (k < m) {
                     if (Tab::a(m, k) != 0.0)
-                        Kbar[k][i] += mul_rn(mul_left_in(mul_rn(g, mul_right_in(Tab::a(m, k)))), h);
+                        Kbar[k][i] += mul_rn(g, mul_right_in(Tab::a(m, k))) * hh;
                     else
                         Kbar[k][i] = add_zero64(Kbar[k][i], g.e ^ h.e);
                 }
