@@ -496,8 +496,7 @@ int bundle_grid(va_handle *h)
 constexpr int kTwoLevelBlock = 64, kTwoLevelBlocksPerSm = 4;
 constexpr int kTwoLevelGroupBlock = 256, kTwoLevelGroupBlocksPerSm = 2;
 
-// Teams of lanes: the same blocks, kTwoLevelBlock / lanes instances each (no
-// more scratch than one lane per instance).
+// Teams of lanes: the same blocks, kTwoLevelBlock / lanes instances each.
 int two_level_block(const va_handle *h) { return h->ks->tpi > 1 ? kTwoLevelGroupBlock : kTwoLevelBlock; }
 
 // instances one block of the two-level backward carries at once
@@ -515,6 +514,13 @@ int two_level_grid(va_handle *h)
     return (int)std::max(1L, std::min(need, (long)h->sm_count * bps));
 }
 
+// blocks of a team sweep
+int team_grid(const va_handle *h, const va::TeamKernel &t, int block, int bps)
+{
+    const int64_t need = ((int64_t)h->prob.batch * t.lanes + block - 1) / block;
+    return (int)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)h->sm_count * bps));
+}
+
 // doubles of re-integration scratch the two-level backward needs
 size_t two_level_scratch_doubles(va_handle *h)
 {
@@ -523,7 +529,12 @@ size_t two_level_scratch_doubles(va_handle *h)
     const size_t carriers = (size_t)two_level_grid(h) * two_level_per_block(h);
     if (h->ks->tpi > 1)
         return carriers * (size_t)va::group_scratch_doubles(h->N, h->stride);
-    return carriers * (h->stride + 1) * scratch_record_doubles(h);
+    size_t records = carriers * (h->stride + 1);
+    for (const va::TeamKernel &t : h->teams[va::FP64_TWO_LEVEL]) {
+        const size_t teams = (size_t)team_grid(h, t, kTwoLevelBlock, kTwoLevelBlocksPerSm) * (kTwoLevelBlock / t.lanes);
+        records = std::max(records, teams * va::team_segments(t.lanes, h->stride) * (h->stride + 1));
+    }
+    return records * scratch_record_doubles(h);
 }
 
 // Scratch for the current stride; never called during stream capture.
@@ -627,7 +638,9 @@ va_status launch_teams(va_handle *h, int sweep, Params &a, cudaStream_t s, bool 
     a.rest_sms = 0;
     float from = 0.0f;
     for (const va::TeamKernel &t : teams) {
-        const float to = t.per_quad * quads;
+        float to = t.per_quad * quads;
+        if (two_level && h->stride > 16)
+            to *= 256.0f / ((float)h->stride * (float)h->stride);
         if (!decide && 0.55f * (float)B > to)
             continue;
         const int block = two_level ? kTwoLevelBlock : h->opt.block_size > 0 ? h->opt.block_size : 128;
@@ -637,8 +650,7 @@ va_status launch_teams(va_handle *h, int sweep, Params &a, cudaStream_t s, bool 
             if (h->opt.blocks_per_sm > 0)
                 bps = std::min(bps, h->opt.blocks_per_sm);
         }
-        const int64_t need = (B * t.lanes + block - 1) / block;
-        const int grid = (int)std::max<int64_t>(1, std::min<int64_t>(need, (int64_t)h->sm_count * bps));
+        const int grid = team_grid(h, t, block, bps);
         const bool last = !decide || (float)B <= to;
         a.load_from = from;
         a.load_to = decide && !(last && from == 0.0f) ? (last ? 3.0e38f : to) : 0.0f;

@@ -22,9 +22,11 @@ namespace va {
 // The oscillators gain from wide teams at loads where Van der Pol no longer
 // does (their steps are cheaper beside the fixed part of an attempt); the
 // limits lie between the two.
-// Two-level backward alone, Van der Pol (16 / 8 / 4 / 2, one lane): 4,800: 4.7 /
-// 7.2 / 7.1 / 9.3, 11.1; 9,001: 8.4 / 7.8 / 11.6 / 9.7, 11.0; 12,000: 11.2 / 10.3 /
-// 11.8 / 13.1, 12.5.
+// Two-level backward alone, Van der Pol, stride 16 (32 / 16 / 8 lanes, one
+// lane): 200: 0.73 / 1.11, 11.2; 1,200: 1.16 / 1.21, 11.3; 9,001: 5.97 / 4.69 /
+// 5.34, 11.0; 30,000: 16.2 (16 lanes), 22.3; 100,000: 63.6 / 54.9, 37.4.  Longer
+// segments are fewer to share out, and launch_teams lowers the limits for them
+// (stride 50, ~250 steps: 9,001 instances 7.7 with 16 lanes, 7.3 with one).
 template <class M, class Tab>
 static void fill(TeamKernel (&t)[kFp64Sweeps][kTeams])
 {
@@ -34,8 +36,8 @@ static void fill(TeamKernel (&t)[kFp64Sweeps][kTeams])
     t[FP64_BACKWARD][0] = {(const void *)backward_team_kernel<M, Tab, 16>, 16, 2, 4.0f};
     t[FP64_BACKWARD][1] = {(const void *)backward_team_kernel<M, Tab, 4>, 4, 1, 6.6f};
     t[FP64_BACKWARD][2] = {(const void *)backward_team_kernel<M, Tab, 2>, 2, 1, 13.0f};
-    t[FP64_TWO_LEVEL][0] = {(const void *)backward_team_kernel_2level<M, Tab, 16>, 16, 2, 6.6f};
-    t[FP64_TWO_LEVEL][1] = {(const void *)backward_team_kernel_2level<M, Tab, 8>, 8, 2, 12.3f};
+    t[FP64_TWO_LEVEL][0] = {(const void *)backward_team_kernel_2level<M, Tab, 32>, 32, 2, 0.75f};
+    t[FP64_TWO_LEVEL][1] = {(const void *)backward_team_kernel_2level<M, Tab, 16>, 16, 2, 50.0f};
 }
 template <class M>
 static void fill_model(Fp64Kernels &k)

@@ -97,6 +97,16 @@ struct TeamKernel {
     int bps;         // resident blocks of 128 threads per SM
     float per_quad;  // highest load, per SM quadrant, that the team takes
 };
+// Segments that a team of g lanes re-integrates at once in the two-level
+// backward: a lane each, but no more than ~1,024 scratch records per team.
+#ifdef __CUDACC__
+__host__ __device__
+#endif
+inline int team_segments(int g, int stride)
+{
+    const int n = 1024 / stride;
+    return n < 1 ? 1 : n < g ? n : g;
+}
 enum { FP64_FORWARD = 0, FP64_BACKWARD = 1, FP64_TWO_LEVEL = 2, kFp64Sweeps = 3 };
 constexpr int kTeams = 3;
 struct Fp64Kernels {

@@ -24,13 +24,15 @@
 // Measured, forward + backward: one Van der Pol instance 4.4 ms (a lane, FP64
 // products) -> 2.0 ms with the recompute spread over rows -> 1.5 ms over steps;
 // 1,216 instances 6.2 -> 2.5 -> 1.96; Fehlberg 7(8), 600 instances 9.5 -> 2.5
-// -> 1.9; two-level backward, 600 instances 11.2 -> 3.6 -> 2.9.  What is left is the
+// -> 1.9; two-level backward, 600 instances 11.2 -> 3.6 -> 2.9, and 0.8
+// with a segment a lane.  What is left is the
 // latency of a step's chain (right-hand side, one product and one sum per
 // stage, the shuffles between them, the step factor): the FP64 unit is busy
 // about half the time.
 #pragma once
 
 #include "va_group.cuh"
+#include "va_registry.h"
 
 namespace va {
 
@@ -703,61 +705,127 @@ __global__ void __launch_bounds__(256) backward_team_kernel(AdjParams a)
 
 // --------------------------------------------- backward sweep, two levels
 
-// backward_kernel_2level with both phases spread over a team; the segment's
-// records lie in the team's scratch (one lane writes, all read).
+// backward_kernel_2level with a team per instance.  The segments between
+// checkpoints are re-integrated G at once, a lane a segment (each from its own
+// checkpoint, one lane's attempt of forward_kernel: the same bits), into the
+// lanes' scratch; the back steps then run through all of them, last first,
+// their recompute G steps at once as in backward_team_kernel.  Spreading one
+// segment's attempts over the team instead (forward_team_kernel's step) took
+// ~60 FP64 instructions per step of one instance, a lane a segment ~260 / G.
 template <class M, class Tab, int G>
 __global__ void __launch_bounds__(256) backward_team_kernel_2level(AdjParams a)
 {
     constexpr int N = M::N, P = M::P;
     constexpr int RS = record_doubles(N);
+    using TB = TeamBackward<M, Tab, G>;
     if (gated_off(a))
         return;
-    const TeamForward<M, Tab, G> tf;
-    const TeamBackward<M, Tab, G> tb;
-    const bool first = tb.team.index == 0;
+    const TB tb;
+    const unsigned mask = tb.team.mask;
+    const int me = tb.team.index, base = tb.team.base;
+    const bool first = me == 0;
     const int CH = a.pool.chunk_len, SK = a.stride;
-    double *scr = a.scratch + ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G * (SK + 1) * RS;
+    const int segs = team_segments(G, SK);
+    const size_t seg_doubles = (size_t)(SK + 1) * RS;
+    // lane l's segment: team_scr + l seg_doubles, l < segs
+    double *team_scr = a.scratch + ((size_t)blockIdx.x * blockDim.x + threadIdx.x) / G * segs * seg_doubles;
 
-    int b = -1, q = 0, T = 0, R = 0, k = 0, last = -1, chunk = -1, slot = 0, L = 0, done = 0, jb = 0, fails = 0;
-    int head = 0;           // step index of the segment's first record
-    double t_start = 0.0;   // t_0 (fixed-step tableaux)
-    int phase = 0;          // 0: re-integrate segment k, 1: back-step through it
-    double lam[N], mu[TeamBackward<M, Tab, G>::Q], t = 0.0, dt = 0.0, t1 = 0.0, y[N], t_end = 0.0, y_end[N];
-    double p[P], k0[N], h = 0.0;
-    int ready = 0, pos = 0; // phase 1: as backward_team_kernel
-    typename TeamBackward<M, Tab, G>::Weights W;
-    bool at_top = true;
+    int b = -1, q = 0, j = -1, T = 0, R = 0, last = -1, chunk = -1, slot = 0;
+    int top = 0, low = 0;   // the lanes hold the segments top, top - 1, .. of steps low .. j
+    int ready = 0, pos = 0; // as backward_team_kernel
+    double lam[N], mu[TB::Q], t1 = 0.0, t_start = 0.0, t_end = 0.0, y_end[N], p[P], h = 0.0;
+    typename TB::Weights W;
 
-    auto keep = [&](int n) { // record n of the segment
-        __syncwarp(tb.team.mask);
-        if (first) {
-            double *r = scr + (size_t)n * RS;
-            r[0] = t;
+    // Re-integrates the segments that end with step j; false: one of them did
+    // not land on its next checkpoint.
+    auto reintegrate = [&]() -> bool {
+        top = j / SK;
+        const int cnt = top + 1 < segs ? top + 1 : segs;
+        low = (top - cnt + 1) * SK;
+        bool run = me < cnt;
+        const int at = run ? me : cnt - 1, first_step = (top - at) * SK;
+        const int L = j + 1 - first_step < SK ? j + 1 - first_step : SK;
+        int c = chunk, s = slot - 1 - at; // the walk is on checkpoint top + 1
+        while (s < 0) {
+            c = a.pool.chunk_prev[c];
+            s += CH;
+        }
+        const double *r = record_ptr<RS>(a.pool, c, s);
+        double t, y[N], dt = r[1], te, ye[N];
+        read_record<N>(r, t, y);
+        // the segment's end: the next checkpoint, which the lane above starts from
+        te = __shfl_up_sync(mask, t, 1, G);
+        te = first ? t_end : te;
+#pragma unroll
+        for (int i = 0; i < N; i++) {
+            const double v = __shfl_up_sync(mask, y[i], 1, G);
+            ye[i] = first ? y_end[i] : v;
+        }
+        t_end = shfl(t, base + cnt - 1, mask);
+#pragma unroll
+        for (int i = 0; i < N; i++)
+            y_end[i] = shfl(y[i], base + cnt - 1, mask);
+        chunk = shfl(c, base + cnt - 1, mask);
+        slot = shfl(s, base + cnt - 1, mask);
+
+        double *scr = team_scr + me * seg_doubles, k0[N];
+        auto keep = [&](int n) {
+            double *w = scr + (size_t)n * RS;
+            w[0] = t;
 #pragma unroll
             for (int i = 0; i < N; i++)
-                r[2 + i] = y[i];
-        }
-        __syncwarp(tb.team.mask);
-    };
-    auto begin_segment = [&]() {
-        if (slot == 0) {
-            chunk = a.pool.chunk_prev[chunk];
-            slot = CH - 1;
-        } else {
-            slot--;
-        }
-        const double *r = record_ptr<RS>(a.pool, chunk, slot);
-        read_record<N>(r, t, y);
-        dt = r[1];
-        head = k * SK;
-        L = (k == R - 2) ? T - head : SK;
-        keep(0);
+                w[2 + i] = y[i];
+        };
+        __syncwarp(mask); // the back steps have read the segments before
+        if (run)
+            keep(0);
         M::template rhs<double>(y, p, t, k0);
-        done = 0;
-        fails = 0;
-        at_top = true;
-        phase = 0;
+        int done = 0, fails = 0;
+        bool at_top = true, ok = true;
+        while (run) {
+            if (at_top) {
+                if (!Tab::FIXED && greater_pos64((t + dt) - t1, kDblEps))
+                    dt = t1 - t;
+                fails = 0;
+                at_top = false;
+            }
+            double ynew[N], ys[N], knew[N];
+            const double err = attempt<M, Tab, double>(y, y, k0, p, t, dt, a.atol, a.rtol, ynew, ys, knew);
+            if (is_nan64(err) || fails >= a.max_fail) {
+                ok = run = false;
+                continue;
+            }
+            fails++;
+            if (greater_nonneg64(err, 1.0)) {
+                dt = decrease_step<Tab, double>(dt, err, a.step_pow, &a.ctl->pow_undecided);
+                continue;
+            }
+            if constexpr (Tab::FIXED) {
+                t = fixed_time(t_start, first_step + done + 1, dt);
+            } else {
+                t += dt;
+                dt = increase_step<Tab, double>(dt, err, a.step_pow, &a.ctl->pow_undecided);
+            }
+            accept_state<M, Tab, double>(y, y, k0, ynew, ynew, knew, p, t);
+            at_top = true;
+            done++;
+            keep(done);
+            if (done == L) {
+                run = false;
+                ok = t == te;
+#pragma unroll
+                for (int i = 0; i < N; i++)
+                    ok = ok && y[i] == ye[i];
+            }
+        }
+        __syncwarp(mask); // the segments are in place
+        return __all_sync(mask, ok);
     };
+    // step n's record in the lanes' scratch, its successor behind it
+    auto step_record = [&](int n) -> const double * {
+        return team_scr + (top - n / SK) * seg_doubles + (size_t)(n % SK) * RS;
+    };
+
     auto start_seed = [&]() {
         chunk = last;
         slot = (R - 1) % CH;
@@ -769,16 +837,16 @@ __global__ void __launch_bounds__(256) backward_team_kernel_2level(AdjParams a)
         tb.clear(mu);
         if (first)
             note_lambda<N>(a, b, q, T, lam);
-        k = R - 2;
-        if (k >= 0)
-            begin_segment();
+        j = T - 1;
+        low = T;
+        ready = pos = 0;
     };
     auto fetch = [&]() -> bool {
         for (;;) {
             int w = 0;
             if (first)
                 w = (int)atomicAdd(&a.ctl->adj_next, 1u);
-            w = shfl(w, tb.team.base, tb.team.mask);
+            w = shfl(w, base, mask);
             if (w >= a.B)
                 return false;
             b = a.order ? a.order[w] : w;
@@ -805,7 +873,7 @@ __global__ void __launch_bounds__(256) backward_team_kernel_2level(AdjParams a)
 
     bool alive = fetch();
     while (alive) {
-        if (k < 0) {
+        if (j < 0) {
             double m[P];
 #pragma unroll
             for (int kk = 0; kk < P; kk++)
@@ -820,84 +888,28 @@ __global__ void __launch_bounds__(256) backward_team_kernel_2level(AdjParams a)
             }
             continue;
         }
-        if (phase == 0) {
-            // one attempt of the forward controller, as forward_team_kernel does
-            if (at_top) {
-                if (!Tab::FIXED && greater_pos64((t + dt) - t1, kDblEps))
-                    dt = t1 - t;
-                fails = 0;
-                at_top = false;
-            }
-            double ynew[N], knew[N];
-            const double err = tf.attempt(y, k0, p, t, dt, a.atol, a.rtol, ynew, knew);
-            if (is_nan64(err) || fails >= a.max_fail) {
-                if (first)
-                    team_fail<N, P>(a, b, ST_RECOMPUTE_MISMATCH);
-                alive = fetch();
-                continue;
-            }
-            fails++;
-            unsigned int *undecided = first ? &a.ctl->pow_undecided : nullptr;
-            if (greater_nonneg64(err, 1.0)) {
-                dt = decrease_step<Tab, double>(dt, err, a.step_pow, undecided);
-                continue;
-            }
-            if constexpr (Tab::FIXED) {
-                t = fixed_time(t_start, head + done + 1, dt);
-            } else {
-                t += dt;
-                dt = increase_step<Tab, double>(dt, err, a.step_pow, undecided);
-            }
-            accept_state<M, Tab, double>(y, y, k0, ynew, ynew, knew, p, t);
-            at_top = true;
-            done++;
-            keep(done);
-            if (done == L) {
-                // the re-integration must land exactly on the next checkpoint
-                bool same = t == t_end;
-#pragma unroll
-                for (int i = 0; i < N; i++)
-                    same = same && y[i] == y_end[i];
-                if (!same) {
-                    if (first)
-                        team_fail<N, P>(a, b, ST_RECOMPUTE_MISMATCH);
-                    alive = fetch();
-                    continue;
-                }
-                phase = 1;
-                jb = L - 1;
-                ready = pos = 0;
-            }
+        if (j < low && !reintegrate()) {
+            if (first)
+                team_fail<N, P>(a, b, ST_RECOMPUTE_MISMATCH);
+            alive = fetch();
             continue;
         }
-        // phase 1: back_step through the segment, last step first
-        if (pos == ready) {
-            ready = jb + 1 < G ? jb + 1 : G;
+        if (pos == ready) { // weights of the steps j, j - 1, .. that the lanes hold
+            ready = j + 1 - low < G ? j + 1 - low : G;
             pos = 0;
-            const int me = tb.team.index;
-            const double *r = scr + (size_t)(jb - (me < ready ? me : ready - 1)) * RS;
+            const double *r = step_record(j - (me < ready ? me : ready - 1));
             double yj[N];
 #pragma unroll
             for (int i = 0; i < N; i++)
                 yj[i] = r[2 + i];
             h = r[RS] - r[0];
-            TeamBackward<M, Tab, G>::weights(yj, r[0], h, p, W);
+            TB::weights(yj, r[0], h, p, W);
         }
-        tb.step(W, pos, shfl(h, tb.team.base + pos, tb.team.mask), lam, mu);
-        pos++;
+        tb.step(W, pos, shfl(h, base + pos, mask), lam, mu);
         if (first)
-            note_lambda<N>(a, b, q, head + jb, lam);
-        jb--;
-        if (jb < 0) {
-            // the segment's start becomes the next segment's end
-            t_end = scr[0];
-#pragma unroll
-            for (int i = 0; i < N; i++)
-                y_end[i] = scr[2 + i];
-            k--;
-            if (k >= 0)
-                begin_segment();
-        }
+            note_lambda<N>(a, b, q, j, lam);
+        pos++;
+        j--;
     }
 }
 
