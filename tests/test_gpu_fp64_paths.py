@@ -140,3 +140,38 @@ def test_lotka_volterra_special_values_bit_exact(oracle, cuda, N, B, tab):
     p = np.concatenate([r, A.reshape(B, N * N)], 1)
     NP["glv"] = N + N * N
     check(oracle, "glv", tab, y0, p, t1, sorted({*range(7), B // 2, B - 1}))
+
+
+@pytest.mark.parametrize("N", [5, 10])
+@pytest.mark.parametrize("tab", ["dopri5", "ck54"])
+@pytest.mark.parametrize("B", [1, 40, 900])
+def test_lotka_volterra_warps(oracle, cuda, N, tab, B):
+    """A warp per instance against lane groups (a block size that it does not take): several seeds, direct gradients, the
+    adjoint history, fewer resident warps than instances, short chunks, failed instances."""
+    rng = np.random.default_rng(N * 1000 + B)
+    A = rng.normal(0, 0.1, (B, N, N))
+    A[:, np.arange(N), np.arange(N)] = -1.0
+    p = np.concatenate([rng.uniform(0.5, 1.5, (B, N)), A.reshape(B, N * N)], 1)
+    y0, t1 = rng.uniform(0.1, 1.0, (B, N)), rng.uniform(0.0, 8.0, B)
+    if B > 10:
+        p[3, 0], t1[4], y0[5, 1] = np.nan, 0.0, np.inf
+    lam, mud = rng.standard_normal((B, 2, N)), rng.standard_normal((B, 2, N + N * N))
+    res = []
+    for block, bps, chunk in ((0, 0, 0), (64, 1, 3), (96, 0, 0), (224, 0, 0)):
+        s = Solver("glv", N, N + N * N, B, nout=2, tableau=tab, atol=1e-7, rtol=1e-7, block_size=block, blocks_per_sm=bps,
+                   chunk_len=chunk, max_steps=45)
+        s.set_adjoint_history(4)
+        for _ in range(2):
+            f = s.forward(dev(y0), dev(p), dev(np.zeros(B)), dev(t1))
+            g = s.backward(dev(p), dev(lam), dev(mud))
+        res.append([v.cpu().numpy() for v in (f["yT"], f["n_acc"], f["n_rej"], f["status"], g["status"], g["dy0"], g["dp"])])
+        s.close()
+    pb = oracle.problem("glv", tab, N, N + N * N, 1e-7, 1e-7)
+    for b in {0, B - 1}:
+        if res[0][3][b] == 0:
+            fw = oracle.forward(pb, y0[b], p[b], 0.0, t1[b])
+            assert fw["n_acc"] == res[0][1][b]
+            np.testing.assert_array_equal(fw["states"][-1], res[0][0][b])
+    for r in res[1:]:
+        for a, b in zip(r, res[0]):
+            np.testing.assert_array_equal(a, b)

@@ -221,7 +221,7 @@ __global__ void __launch_bounds__(256) forward_group_kernel(FwdParams a)
     constexpr int G = M::TPI, NT = M::NTOT, PT = M::PTOT, P = M::P;
     constexpr int RS = record_doubles(NT);
     const LaneGroup<G> grp;
-    if (!grp.active())
+    if (!grp.active() || gated_off(a))
         return;
     const int li = grp.index, src = grp.base;
     const unsigned mask = grp.mask;
@@ -402,7 +402,7 @@ __global__ void __launch_bounds__(256) backward_group_kernel(AdjParams a)
     constexpr int G = M::TPI, NT = M::NTOT, PT = M::PTOT, P = M::P, PG = M::PG;
     constexpr int RS = record_doubles(NT);
     const LaneGroup<G> grp;
-    if (!grp.active())
+    if (!grp.active() || gated_off(a))
         return;
     const int li = grp.index, src = grp.base;
     const unsigned mask = grp.mask;

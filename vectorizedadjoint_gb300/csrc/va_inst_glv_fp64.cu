@@ -2,6 +2,7 @@
 // they reproduce the CPU oracle bit for bit (see va_inst_small_fp64.cu).
 #include "va_group.cuh"
 #include "va_registry.h"
+#include "va_team_glv64.cuh"
 
 namespace va {
 
@@ -35,6 +36,17 @@ static Fp64Kernels make_int()
     }
     k.int_fwd_min = NN == 5 ? kTwoWarps5 : 32;
     k.int_bwd_min = kTwoWarps5;
+    // A warp per instance (va_team_glv64.cuh); limits where the lane groups are
+    // faster, ms (load ~0.8 B):
+    //     N = 5    forward: 100: 0.32, groups 0.61; 777: 0.48, 0.59; 3,000: 1.15, 0.62
+    //              backward: 0.25, 0.89; 0.38, 0.86; 0.97, 0.91
+    //     N = 10   forward: 0.51, 0.72; 0.79, 0.71; 2.08, 0.79
+    //              backward: 0.54, 1.53; 0.85, 1.51; 2.36, 1.88
+    const float fq = NN == 5 ? 1.5f : 0.95f, bq = NN == 5 ? 3.8f : 2.8f;
+    k.team[0][FP64_FORWARD][0] = {(const void *)forward_glv_warp_kernel<NN, TabDopri5>, 32, 2, fq};
+    k.team[1][FP64_FORWARD][0] = {(const void *)forward_glv_warp_kernel<NN, TabCK54>, 32, 2, fq};
+    k.team[0][FP64_BACKWARD][0] = {(const void *)backward_glv_warp_kernel<NN, TabDopri5>, 32, 2, bq};
+    k.team[1][FP64_BACKWARD][0] = {(const void *)backward_glv_warp_kernel<NN, TabCK54>, 32, 2, bq};
     return k;
 }
 const Fp64Kernels *fp64_kernels_glv(int n)
