@@ -1,7 +1,6 @@
 // Kernels of the tensor-core dA contraction (va_contract.cuh): the factor-row
 // offsets of each instance, the contraction on tcgen05 with tensor-memory
 // accumulators, and the fixed-order sum of the CTA partials.
-#include <cuda_bf16.h>
 #include <cuda_runtime.h>
 
 #include <algorithm>
@@ -53,119 +52,121 @@ __device__ __forceinline__ float dw_abs_hi(double packed) { return fabsf(dw_unpa
 // exponent e with |x| < 2^e for every entry whose leading word is at most m
 __device__ __forceinline__ int bound_exponent(float m) { return m > 0.0f ? ilogbf(m) + 1 : -120; }
 
-__device__ __forceinline__ uint32_t pack_bf16x2(float a, float b)
+// two digits as a bf16 pair: a digit has at most 8 significant bits, so its
+// bf16 is the upper half of its float
+__device__ __forceinline__ uint32_t pack_digits(float a, float b)
 {
-    const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
-    return *reinterpret_cast<const uint32_t *>(&v);
+    return __byte_perm(__float_as_uint(a), __float_as_uint(b), 0x7632);
 }
 
 // One column's 8 consecutive rows (a core-matrix row of 16 bytes) as Q digit
-// planes: vals are packed double-words, e the column's exponent.
-__device__ __forceinline__ void slice_row8(const double (&vals)[8], DigitScale sc, uint8_t *plane0,
-                                           size_t plane_stride)
+// planes: vals are packed double-words, sc the column's scale.
+__device__ __forceinline__ void slice_row8(const double *vals, DigitScale sc, uint8_t *plane0, size_t plane_stride)
 {
-    float d[8][kContractQ];
+    uint32_t q[kContractQ][4];
 #pragma unroll
-    for (int r = 0; r < 8; r++) {
-        const dword w = dw_unpack(vals[r]);
-        split_digits(w.hi, w.lo, sc, d[r]);
+    for (int r = 0; r < 8; r += 2) {
+        const dword w0 = dw_unpack(vals[r]), w1 = dw_unpack(vals[r + 1]);
+        float d0[kContractQ], d1[kContractQ];
+        split_digits_in_place(w0.hi, w0.lo, sc, d0);
+        split_digits_in_place(w1.hi, w1.lo, sc, d1);
+#pragma unroll
+        for (int s = 0; s < kContractQ; s++)
+            q[s][r / 2] = pack_digits(d0[s], d1[s]);
     }
 #pragma unroll
-    for (int s = 0; s < kContractQ; s++) {
-        uint4 q;
-        q.x = pack_bf16x2(d[0][s], d[1][s]);
-        q.y = pack_bf16x2(d[2][s], d[3][s]);
-        q.z = pack_bf16x2(d[4][s], d[5][s]);
-        q.w = pack_bf16x2(d[6][s], d[7][s]);
-        *reinterpret_cast<uint4 *>(plane0 + s * plane_stride) = q;
-    }
+    for (int s = 0; s < kContractQ; s++)
+        *reinterpret_cast<uint4 *>(plane0 + s * plane_stride) = make_uint4(q[s][0], q[s][1], q[s][2], q[s][3]);
 }
+
+// A chunk's column exponents and scales 2^(e - 8) (0 outside the fold's fast
+// range; the column then takes its exponent).
+struct ContractScales {
+    int ev[kContractTileM], ex[kContractTileN];
+    alignas(16) float pv[kContractTileM], px[kContractTileN];
+};
+__device__ __forceinline__ float fold_scale(int e) { return e >= -100 && e <= 100 ? pow2f(e - 8) : 0.0f; }
 
 // Slices chunk c of the CTA's tile into one shared-memory stage and stores
-// the column exponents (e_v[128], e_x[64]).
+// the column exponents.  A warp holds all 64 rows of its columns (8 of v, 4
+// of x), so each factor is read once and a column's maximum is a few
+// shuffles: no barrier between the maximum and the digits.
 __device__ __forceinline__ void slice_chunk(const ContractParams &p, int c, int K, int ti, int tj, uint8_t *stage,
-                                            int *ev, int *ex, float *red, const double *const *xrow)
+                                            ContractScales &sc, const double *const *xrow)
 {
-    const int t = threadIdx.x;
+    const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
     const int k0 = c * kContractKC;
-    // v: column i = t & 127, rows 16 h .. 16 h + 15 (h = t >> 7)
+    const bool whole = k0 + kContractKC <= K;
+    // v: column i, rows 16 h .. 16 h + 15; x: column j, rows 8 q .. 8 q + 7
+    const int i = warp * 8 + (lane & 7), h = lane >> 3;
+    const int j = warp * 4 + (lane & 3), q = lane >> 2;
+    double v[16], x[8];
+    const double *col = p.v + (size_t)(k0 + 16 * h) * kContractN + ti * kContractTileM + i;
+    const int xc = tj * kContractTileN + j;
+    if (whole) {
+#pragma unroll
+        for (int r = 0; r < 16; r++)
+            v[r] = __ldg(col + (size_t)r * kContractN);
+#pragma unroll
+        for (int r = 0; r < 8; r++)
+            x[r] = __ldg(xrow[8 * q + r] + xc);
+    } else {
+#pragma unroll
+        for (int r = 0; r < 16; r++)
+            v[r] = k0 + 16 * h + r < K ? __ldg(col + (size_t)r * kContractN) : 0.0;
+#pragma unroll
+        for (int r = 0; r < 8; r++)
+            x[r] = k0 + 8 * q + r < K ? __ldg(xrow[8 * q + r] + xc) : 0.0;
+    }
+    // v planes [slice][kgroup 8][row 128][8]
     {
-        const int i = t & 127, h = t >> 7;
-        const double *col = p.v + (size_t)ti * kContractTileM + i;
         float m = 0.0f;
 #pragma unroll
-        for (int r = 0; r < 16; r++) {
-            const int k = k0 + 16 * h + r;
-            if (k < K)
-                m = fmaxf(m, dw_abs_hi(__ldg(col + (size_t)k * kContractN)));
+        for (int r = 0; r < 16; r++)
+            m = fmaxf(m, dw_abs_hi(v[r]));
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 8));
+        m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, 16));
+        const int e = bound_exponent(m);
+        if (h == 0) {
+            sc.ev[i] = e;
+            sc.pv[i] = fold_scale(e);
         }
-        red[t] = m;
+        const DigitScale ds = digit_scale(e);
+#pragma unroll
+        for (int g = 0; g < 2; g++)
+            slice_row8(v + 8 * g, ds, stage + (size_t)(2 * h + g) * kVGroupBytes + i * 16, 8 * kVGroupBytes);
     }
-    // x: column j = t & 63, rows 8 q .. 8 q + 7 (q = t >> 6)
+    // x planes [slice][kgroup 8][row 64][8]
     {
-        const int j = t & 63, q = t >> 6;
         float m = 0.0f;
 #pragma unroll
-        for (int r = 0; r < 8; r++) {
-            const int k = k0 + 8 * q + r;
-            if (k < K)
-                m = fmaxf(m, dw_abs_hi(__ldg(xrow[8 * q + r] + tj * kContractTileN + j)));
+        for (int r = 0; r < 8; r++)
+            m = fmaxf(m, dw_abs_hi(x[r]));
+#pragma unroll
+        for (int o = 4; o < 32; o *= 2)
+            m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+        const int e = bound_exponent(m);
+        if (q == 0) {
+            sc.ex[j] = e;
+            sc.px[j] = fold_scale(e);
         }
-        red[kContractThreads + t] = m;
-    }
-    __syncthreads();
-    if (t < 128) {
-        ev[t] = bound_exponent(fmaxf(fmaxf(red[t], red[t + 128]), fmaxf(red[t + 256], red[t + 384])));
-    } else if (t < 192) {
-        const int j = t - 128;
-        float m = 0.0f;
-#pragma unroll
-        for (int q = 0; q < 8; q++)
-            m = fmaxf(m, red[kContractThreads + j + 64 * q]);
-        ex[j] = bound_exponent(m);
-    }
-    __syncthreads();
-    // digits: v planes [slice][kgroup 8][row 128][8] (plane = 16 KB, kgroup = 2 KB)
-    {
-        const int i = t & 127, h = t >> 7;
-        const double *col = p.v + (size_t)ti * kContractTileM + i;
-        const DigitScale sc = digit_scale(ev[i]);
-#pragma unroll
-        for (int g = 0; g < 2; g++) {
-            const int kg = 2 * h + g;
-            double vals[8];
-#pragma unroll
-            for (int r = 0; r < 8; r++) {
-                const int k = k0 + 8 * kg + r;
-                vals[r] = k < K ? __ldg(col + (size_t)k * kContractN) : 0.0;
-            }
-            slice_row8(vals, sc, stage + (size_t)kg * 2048 + i * 16, (size_t)kContractKC * kContractTileM * 2);
-        }
-    }
-    // digits: x planes [slice][kgroup 8][row 64][8] (plane = 8 KB, kgroup = 1 KB)
-    {
-        const int j = t & 63, q = t >> 6;
-        const DigitScale sc = digit_scale(ex[j]);
-        uint8_t *xs = stage + kTileVBytes;
-        {
-            const int kg = q;
-            double vals[8];
-#pragma unroll
-            for (int r = 0; r < 8; r++) {
-                const int k = k0 + 8 * kg + r;
-                vals[r] = k < K ? __ldg(xrow[8 * kg + r] + tj * kContractTileN + j) : 0.0;
-            }
-            slice_row8(vals, sc, xs + (size_t)kg * 1024 + j * 16, (size_t)kContractKC * kContractTileN * 2);
-        }
+        slice_row8(x, digit_scale(e), stage + kTileVBytes + (size_t)q * kXGroupBytes + j * 16, 8 * kXGroupBytes);
     }
 }
 
-// The x-row pointers of chunk c into xrow[64] (rows past K: null, never
-// dereferenced), and a prefetch of the chunk's rows of the CTA's tile into
-// L2 (the factor rows are read once from DRAM; the slicing loads then wait
-// on L2 instead)
+// The x-row pointer that this thread stages of chunk c (threads 0 .. 255:
+// row t & 63; null past K, never dereferenced)
+__device__ __forceinline__ const double *chunk_row(const ContractParams &p, int c, int K)
+{
+    const int kx = c * kContractKC + (threadIdx.x & 63);
+    return threadIdx.x < 256 && kx < K ? p.xp[kx] : nullptr;
+}
+
+// The x-row pointers of chunk c into xrow[64], and a prefetch of the chunk's
+// rows of the CTA's tile into L2 (the factor rows are read once from DRAM;
+// the slicing loads then wait on L2 instead)
 __device__ __forceinline__ void prefetch_chunk(const ContractParams &p, int c, int K, int ti, int tj,
-                                               const double **xrow)
+                                               const double *base, const double **xrow)
 {
     const int t = threadIdx.x;
     // v: 64 rows of 128 doubles, 8 threads a row; x: 64 rows of 64, 4 threads a row
@@ -173,14 +174,10 @@ __device__ __forceinline__ void prefetch_chunk(const ContractParams &p, int c, i
     if (kv < K)
         asm volatile("prefetch.global.L2 [%0];" ::"l"(p.v + (size_t)kv * kContractN + ti * kContractTileM +
                                                       (t & 7) * 16));
-    const int kx = c * kContractKC + (t & 63);
-    if (t < 256) {
-        const double *base = kx < K ? p.xp[kx] : nullptr;
-        if (t < 64)
-            xrow[t] = base;
-        if (base)
-            asm volatile("prefetch.global.L2 [%0];" ::"l"(base + tj * kContractTileN + (t >> 6) * 16));
-    }
+    if (t < 64)
+        xrow[t] = base;
+    if (base)
+        asm volatile("prefetch.global.L2 [%0];" ::"l"(base + tj * kContractTileN + (t >> 6) * 16));
 }
 
 // The 40 MMAs of one chunk: for every group g = s + t the digit pairs
@@ -189,7 +186,7 @@ __device__ __forceinline__ void issue_chunk(uint32_t tmem_acc, const uint8_t *st
 {
     constexpr uint32_t idesc = umma_idesc_bf16(kContractTileM, kContractTileN);
     const uint32_t vbase = smem_u32(stage), xbase = smem_u32(stage + kTileVBytes);
-    constexpr uint32_t vplane = kContractKC * kContractTileM * 2, xplane = kContractKC * kContractTileN * 2;
+    constexpr uint32_t vplane = 8 * kVGroupBytes, xplane = 8 * kXGroupBytes;
 #pragma unroll
     for (int g = 0; g < kContractQ; g++) {
         bool first = true;
@@ -199,8 +196,8 @@ __device__ __forceinline__ void issue_chunk(uint32_t tmem_acc, const uint8_t *st
 #pragma unroll
             for (int kk = 0; kk < kContractKC / 16; kk++) {
                 // K step kk covers kgroups 2kk and 2kk + 1
-                const uint64_t ad = umma_desc(vbase + s * vplane + kk * 2 * 2048, 2048, 128);
-                const uint64_t bd = umma_desc(xbase + tq * xplane + kk * 2 * 1024, 1024, 128);
+                const uint64_t ad = umma_desc(vbase + s * vplane + kk * 2 * kVGroupBytes, kVGroupBytes, 128);
+                const uint64_t bd = umma_desc(xbase + tq * xplane + kk * 2 * kXGroupBytes, kXGroupBytes, 128);
                 umma_bf16(tmem_acc + g * kContractTileN, ad, bd, idesc, first ? 0u : 1u);
                 first = false;
             }
@@ -208,39 +205,64 @@ __device__ __forceinline__ void issue_chunk(uint32_t tmem_acc, const uint8_t *st
     }
 }
 
+// (ah, al) += v + lo
+__device__ __forceinline__ void fold_add(float &ah, float &al, float v, float lo)
+{
+    const float s = ah + v;
+    const float bb = s - ah;
+    const float e = (ah - (s - bb)) + (v - bb);
+    const float l = lo + e;
+    ah = s + l;
+    al = l - (ah - s);
+}
+
 // Folds one chunk's group sums into the double-word accumulators of this
-// thread's row and 32 columns: acc += R_g 2^(e_v + e_x - 8(g + 2)).
-__device__ __forceinline__ void fold_chunk(uint32_t tmem_row, const int *ev, const int *ex, int row, int col0,
+// thread's row and 16 columns.  The digits carry their weights, so group g
+// holds S_g = R_g 2^(-8g), a multiple of 2^(-8g) below 2^(24 - 8g): S_0 + S_1,
+// S_2 + S_3 and the sum of both lose nothing in fast two-sums, and one
+// double-word addition of 2^(e_v + e_x - 16) times the result replaces one
+// per group.
+__device__ __forceinline__ void fold_chunk(uint32_t tmem_row, const ContractScales &sc, int row, int col0,
                                            float (&ah)[kContractFoldCols], float (&al)[kContractFoldCols])
 {
-    constexpr int C = kContractFoldCols;
-    // R_g 2^(esum - 8g) = (R_g 2^(-8g)) 2^esum: two exact multiplications by
-    // normal powers of two when -102 <= esum <= 103 (|R_g| < 2^24, so every
-    // product is a normal float); ldexpf for columns outside that range
-    int esum[C];
-    float p2[C];
-    bool fast = true;
+    constexpr int C = 8;
+    const float pv = sc.pv[row];
 #pragma unroll
-    for (int c = 0; c < C; c++) {
-        esum[c] = ev[row] + ex[col0 + c] - 16;
-        fast = fast && esum[c] >= -102 && esum[c] <= 103;
-        p2[c] = pow2f(min(max(esum[c], -102), 103));
-    }
-#pragma unroll 1
-    for (int g = 0; g < kContractQ; g++) {
-        float R[C];
-        tmem_ld16(tmem_row + g * kContractTileN, R);
-        const float sg = pow2f(-8 * g);
+    for (int c0 = 0; c0 < kContractFoldCols; c0 += C) {
+        float S[kContractQ][C], p2[C];
+        tmem_ld8_groups<kContractQ>(tmem_row + c0, 0, S);
+        float lo = pv, hi = pv;
+#pragma unroll
+        for (int c = 0; c < C; c += 4) {
+            const float4 w = *reinterpret_cast<const float4 *>(&sc.px[col0 + c0 + c]);
+            p2[c] = pv * w.x;
+            p2[c + 1] = pv * w.y;
+            p2[c + 2] = pv * w.z;
+            p2[c + 3] = pv * w.w;
+        }
 #pragma unroll
         for (int c = 0; c < C; c++) {
-            const float v = fast ? (R[c] * sg) * p2[c] : ldexpf(R[c], esum[c] - 8 * g); // exact
-            // double-word accumulation: (ah, al) += v
-            const float s = ah[c] + v;
-            const float bb = s - ah[c];
-            const float e = (ah[c] - (s - bb)) + (v - bb);
-            const float lo = al[c] + e;
-            ah[c] = s + lo;
-            al[c] = lo - (ah[c] - s);
+            lo = fminf(lo, p2[c]);
+            hi = fmaxf(hi, p2[c]);
+        }
+        // every product below is then a normal float
+        if (lo >= 0x1p-70f && hi <= 0x1p100f) {
+#pragma unroll
+            for (int c = 0; c < C; c++) {
+                float s, e, u, f, w, g;
+                fast_two_sum(S[0][c], S[1][c], s, e);
+                fast_two_sum(S[2][c], S[3][c], u, f);
+                fast_two_sum(s, u, w, g);
+                fold_add(ah[c0 + c], al[c0 + c], w * p2[c], al[c0 + c] + (e + f + g) * p2[c]);
+            }
+        } else {
+#pragma unroll
+            for (int c = 0; c < C; c++) {
+                const int esum = sc.ev[row] + sc.ex[col0 + c0 + c] - 16;
+#pragma unroll
+                for (int g = 0; g < kContractQ; g++)
+                    fold_add(ah[c0 + c], al[c0 + c], ldexpf(S[g][c], esum), al[c0 + c]);
+            }
         }
     }
 }
@@ -249,11 +271,9 @@ __device__ __forceinline__ void fold_chunk(uint32_t tmem_row, const int *ev, con
 __global__ void __launch_bounds__(kContractThreads, 1) contract_kernel(ContractParams p)
 {
     extern __shared__ __align__(1024) uint8_t smem[];
-    uint8_t *stages[2] = {smem, smem + kStageBytes};
     uint64_t *done = reinterpret_cast<uint64_t *>(smem + 2 * kStageBytes); // [2]
     uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(done + 2);
-    __shared__ int ev_s[2][kContractTileM], ex_s[2][kContractTileN];
-    __shared__ float red[2 * kContractThreads];
+    __shared__ ContractScales scales[3];             // of chunk idx in idx % 3: see the loop
     __shared__ const double *xrow_s[2][kContractKC]; // x-row pointers of the chunk in each stage
 
     const int t = threadIdx.x, warp = t >> 5, lane = t & 31;
@@ -287,57 +307,70 @@ __global__ void __launch_bounds__(kContractThreads, 1) contract_kernel(ContractP
     for (int c = 0; c < kContractFoldCols; c++)
         ah[c] = al[c] = 0.0f;
 
-    // ok stays uniform across the block (a bounded wait that gave up on any
-    // thread stops the work of all of them at the next barrier)
+    // One barrier a chunk: a thread slices chunk idx, meets the others, and
+    // folds chunk idx - 1 while the MMAs of idx run.  What the next chunk
+    // overwrites is free by then:
+    // - stage and accumulators of idx - 2: every thread has waited for its
+    //   MMAs and folded it before the barrier of idx;
+    // - the scales of idx - 1 are read after that barrier, while a thread that
+    //   is ahead already writes those of idx + 1: three sets;
+    // - the row pointers of idx are read before it: two sets.
+    // ok is uniform in a warp, and in the block from barrier to barrier (a
+    // bounded wait that gave up stops the work of all).
     bool ok = true;
     int issued = 0, waited = 0; // chunks committed / chunks whose commit was awaited
     const int n = c1 - c0;
-    if (n > 0)
-        prefetch_chunk(p, c0, K, ti, tj, xrow_s[0]);
+    const double *base = nullptr;
+    if (n > 0) {
+        prefetch_chunk(p, c0, K, ti, tj, chunk_row(p, c0, K), xrow_s[0]);
+        if (n > 1)
+            base = chunk_row(p, c0 + 1, K);
+    }
     __syncthreads();
+    int cur = 0, last = 2; // idx % 3, (idx - 1) % 3
     for (int idx = 0; idx < n; idx++) {
         const int st = idx & 1;
         if (ok) {
-            slice_chunk(p, c0 + idx, K, ti, tj, stages[st], ev_s[st], ex_s[st], red, xrow_s[st]);
+            slice_chunk(p, c0 + idx, K, ti, tj, smem + st * kStageBytes, scales[cur], xrow_s[st]);
             if (idx + 1 < n)
-                prefetch_chunk(p, c0 + idx + 1, K, ti, tj, xrow_s[st ^ 1]);
+                prefetch_chunk(p, c0 + idx + 1, K, ti, tj, base, xrow_s[st ^ 1]);
+            if (idx + 2 < n)
+                base = chunk_row(p, c0 + idx + 2, K);
         }
         // the digit planes, written by this CTA's threads, feed the tensor core
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         tc_fence_before();
-        __syncthreads();
+        ok = __syncthreads_and(ok) != 0;
         if (ok) {
-            if (t == 0) {
+            if (t == kContractThreads - 32) {
                 tc_fence_after();
-                issue_chunk(tmem + st * kContractQ * kContractTileN, stages[st]);
+                issue_chunk(tmem + st * kContractQ * kContractTileN, smem + st * kStageBytes);
                 umma_commit(&done[st]);
             }
+            __syncwarp();
             issued = idx + 1;
-        }
-        if (idx > 0 && ok) {
-            // the previous chunk's group sums
-            const int pst = st ^ 1;
-            const bool w = mbar_wait_bounded(&done[pst], ((idx - 1) >> 1) & 1, p.error);
-            ok = __syncthreads_and(w) != 0;
-            if (ok) {
-                waited = idx;
-                tc_fence_after();
-                fold_chunk(tmem + lane_addr + pst * kContractQ * kContractTileN + col0, ev_s[pst], ex_s[pst], row,
-                           col0, ah, al);
+            if (idx > 0) {
+                // the previous chunk's group sums
+                const int pst = st ^ 1;
+                ok = __all_sync(0xffffffffu, mbar_wait_bounded(&done[pst], ((idx - 1) >> 1) & 1, p.error)) != 0;
+                if (ok) {
+                    waited = idx;
+                    tc_fence_after();
+                    fold_chunk(tmem + lane_addr + pst * kContractQ * kContractTileN + col0, scales[last], row, col0,
+                               ah, al);
+                }
             }
-            tc_fence_before();
         }
-        __syncthreads();
+        last = cur;
+        cur = cur == 2 ? 0 : cur + 1;
     }
     if (ok && issued == n && n > 0) {
         const int idx = n - 1, st = idx & 1;
-        const bool w = mbar_wait_bounded(&done[st], (idx >> 1) & 1, p.error);
-        ok = __syncthreads_and(w) != 0;
+        ok = __all_sync(0xffffffffu, mbar_wait_bounded(&done[st], (idx >> 1) & 1, p.error)) != 0;
         if (ok) {
             waited = n;
             tc_fence_after();
-            fold_chunk(tmem + lane_addr + st * kContractQ * kContractTileN + col0, ev_s[st], ex_s[st], row, col0,
-                       ah, al);
+            fold_chunk(tmem + lane_addr + st * kContractQ * kContractTileN + col0, scales[last], row, col0, ah, al);
         }
     }
     // after an error: wait (bounded) for the MMAs still in flight before the

@@ -120,23 +120,6 @@ __device__ __forceinline__ void tmem_ld32(uint32_t taddr, float (&v)[32])
         v[c] = __uint_as_float(r[c]);
 }
 
-// 16 consecutive FP32 columns of this thread's tensor-memory lane
-__device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16])
-{
-    uint32_t r[16];
-    asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 "
-                 "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15}, [%16];"
-                 : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]),
-                   "=r"(r[7]), "=r"(r[8]), "=r"(r[9]), "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]),
-                   "=r"(r[14]), "=r"(r[15])
-                 : "r"(taddr)
-                 : "memory");
-    asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-    for (int c = 0; c < 16; c++)
-        v[c] = __uint_as_float(r[c]);
-}
-
 // 8 consecutive FP32 columns of this thread's tensor-memory lane
 __device__ __forceinline__ void tmem_ld8(uint32_t taddr, float (&v)[8])
 {
