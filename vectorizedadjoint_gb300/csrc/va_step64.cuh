@@ -17,10 +17,9 @@
 //
 // The operations and their order are those of attempt_pair, step_fixed and
 // back_step; every sum is the FP64 instruction and every product the
-// correctly rounded one, so the results have the same bits.  A coefficient
-// that is zero adds nothing here (its product with a finite value is a zero,
-// which changes no sum but one that is -0 itself: such a sum is handled as
-// the addition would).
+// correctly rounded one, so the results have the same bits.  For the 5(4)
+// pairs: no a_mj is zero, and a zero b_m or e_m is left out of the sums as it
+// is in attempt_pair.
 //
 // Range.  The products need operands whose significand and exponent can be
 // taken apart (no infinities, NaNs or subnormals) and results that are
@@ -29,7 +28,7 @@
 // before the next one is noted, so with all of them within 2^-240 .. 2^240 (or
 // zero) no product leaves the normal range.  Otherwise the functions return
 // false and the caller takes the step over with FP64 instructions throughout
-// (attempt_pair, step_fixed, back_step): the same result, or the same
+// (attempt_pair, back_step): the same result, or the same
 // infinities and NaNs.
 #pragma once
 
@@ -109,17 +108,7 @@ __host__ __device__ __forceinline__ MulR coef_right(double c, const MulR &h)
     return mul_right_in(mul_rn(mul_left_in(c), h));
 }
 
-template <class Tab>
-constexpr bool zero_in_a()
-{
-    for (int m = 1; m < Tab::S; m++)
-        for (int j = 0; j < m; j++)
-            if (Tab::a(m, j) == 0.0)
-                return true;
-    return false;
-}
-
-// X_m = y + sum_{j<m} (a_mj dt) K_j (form_stage), the non-zero coefficients
+// X_m = y + sum_{j<m} (a_mj dt) K_j (form_stage); the 5(4) pairs have no zero a_mj
 template <class Tab, int N>
 __host__ __device__ __forceinline__ void form_stage64(int m, const double (&y)[N], const MulL (&K)[Tab::S][N],
                                                       const MulR &h, double (&X)[N])
@@ -129,7 +118,7 @@ __host__ __device__ __forceinline__ void form_stage64(int m, const double (&y)[N
         X[i] = y[i];
 #pragma unroll
     for (int j = 0; j < Tab::S - 1; j++)
-        if (j < m && Tab::a(m, j) != 0.0) {
+        if (j < m) {
             const MulR c = coef_right(Tab::a(m, j), h);
 #pragma unroll
             for (int i = 0; i < N; i++)
@@ -137,8 +126,8 @@ __host__ __device__ __forceinline__ void form_stage64(int m, const double (&y)[N
         }
 }
 
-// attempt_pair's (step_fixed's) step for double stages: y_new, k_new and the
-// error norm (0 for a fixed-step tableau).  False: out of range.
+// attempt_pair's step for double stages: y_new, k_new and the error norm.
+// False: out of range.
 template <class M, class Tab>
 __host__ __device__ __forceinline__ bool attempt64(const double (&y)[M::N], const double (&k0)[M::N],
                                                    const double (&p)[M::P], double t, double dt, double atol,
@@ -150,13 +139,9 @@ __host__ __device__ __forceinline__ bool attempt64(const double (&y)[M::N], cons
     note_params64<M>(p, r);
     const MulR h = mul_right(dt, r);
     MulL K[NS][N];
-    bool neg_zero = false;
 #pragma unroll
-    for (int i = 0; i < N; i++) {
+    for (int i = 0; i < N; i++)
         K[0][i] = mul_left(k0[i], r);
-        if (zero_in_a<Tab>()) // no sum starts from -0: skipped zero terms change none
-            neg_zero = neg_zero || f64_bits(y[i]) == 1ull << 63;
-    }
 #pragma unroll
     for (int m = 1; m < NS; m++) {
         double X[N], f[N];
@@ -177,47 +162,37 @@ __host__ __device__ __forceinline__ bool attempt64(const double (&y)[M::N], cons
             for (int i = 0; i < N; i++)
                 ynew[i] = ynew[i] + mul_rn(K[j][i], c);
         }
-    if constexpr (Tab::FIXED) {
-        err = 0.0;
-    } else {
-        double e[N];
-        bool first = true;
+    double e[N];
+    bool first = true;
 #pragma unroll
-        for (int j = 0; j < NS; j++)
-            if (Tab::e(j) != 0.0) {
-                const MulR c = coef_right(Tab::e(j), h);
+    for (int j = 0; j < NS; j++)
+        if (Tab::e(j) != 0.0) {
+            const MulR c = coef_right(Tab::e(j), h);
 #pragma unroll
-                for (int i = 0; i < N; i++) {
-                    const double term = mul_rn(K[j][i], c);
-                    e[i] = first ? term : e[i] + term;
-                }
-                first = false;
+            for (int i = 0; i < N; i++) {
+                const double term = mul_rn(K[j][i], c);
+                e[i] = first ? term : e[i] + term;
             }
-        if constexpr (Tab::FSAL) {
-            model_rhs64<M, true>(ynew, p, t + dt, knew, r);
-            const MulR c = coef_right(Tab::E_NEW, h);
-#pragma unroll
-            for (int i = 0; i < N; i++)
-                e[i] = e[i] + mul_rn(mul_left(knew[i], r), c);
+            first = false;
         }
-        // odeint's rel_error + norm_inf: one quotient per component, then max
-        const MulR ah = {h.h, h.l, h.e & 0x7fffffffu};
-        const MulL rt = mul_left(rtol, r);
-        err = 0.0;
+    if constexpr (Tab::FSAL) {
+        model_rhs64<M, true>(ynew, p, t + dt, knew, r);
+        const MulR c = coef_right(Tab::E_NEW, h);
 #pragma unroll
-        for (int i = 0; i < N; i++) {
-            const MulL ak = {K[0][i].h, K[0][i].l, K[0][i].e & 0x7fffffffu};
-            const double s = fabs(y[i]) + mul_rn(ak, ah);
-            err = max_nonneg64(err, quotient64(fabs(e[i]), atol + mul_rn(rt, mul_right(s, r))));
-        }
+        for (int i = 0; i < N; i++)
+            e[i] = e[i] + mul_rn(mul_left(knew[i], r), c);
     }
-    return !r.beyond(kChainRange) && !neg_zero && !is_nan64(err);
-}
-
-// acc + (a zero with the given sign bit)
-__host__ __device__ __forceinline__ double add_zero64(double acc, uint32_t sign)
-{
-    return f64_bits(acc) == 1ull << 63 && !(sign & 0x80000000u) ? 0.0 : acc;
+    // odeint's rel_error + norm_inf: one quotient per component, then max
+    const MulR ah = {h.h, h.l, h.e & 0x7fffffffu};
+    const MulL rt = mul_left(rtol, r);
+    err = 0.0;
+#pragma unroll
+    for (int i = 0; i < N; i++) {
+        const MulL ak = {K[0][i].h, K[0][i].l, K[0][i].e & 0x7fffffffu};
+        const double s = fabs(y[i]) + mul_rn(ak, ah);
+        err = max_nonneg64(err, quotient64(fabs(e[i]), atol + mul_rn(rt, mul_right(s, r))));
+    }
+    return !r.beyond(kChainRange) && !is_nan64(err);
 }
 
 // back_step for double stages: lambda_n in ybar, mu's new sums in ms.  False:
@@ -233,7 +208,6 @@ __host__ __device__ __forceinline__ bool back_step64(const double (&y)[M::N], do
     note_params64<M>(p, r);
     const MulR h = mul_right(hh, r);
     double X[NS][N];
-    bool neg_zero = false;
     {
         MulL K[NS][N];
 #pragma unroll
@@ -246,11 +220,6 @@ __host__ __device__ __forceinline__ bool back_step64(const double (&y)[M::N], do
                 for (int i = 0; i < N; i++)
                     K[m][i] = mul_left(f[i], r);
             }
-        }
-        if (zero_in_a<Tab>()) {
-#pragma unroll
-            for (int i = 0; i < N; i++)
-                neg_zero = neg_zero || f64_bits(y[i]) == 1ull << 63;
         }
     }
     double Kbar[NS][N];
@@ -283,18 +252,14 @@ __host__ __device__ __forceinline__ bool back_step64(const double (&y)[M::N], do
             const MulL g = mul_left(gx[i], r);
 #pragma unroll
             for (int k = 0; k < NS - 1; k++)
-                if (k < m) {
-                    if (Tab::a(m, k) != 0.0)
-                        Kbar[k][i] += mul_rn(g, mul_right_in(Tab::a(m, k))) * hh;
-                    else
-                        Kbar[k][i] = add_zero64(Kbar[k][i], g.e ^ h.e);
-                }
+                if (k < m)
+                    Kbar[k][i] += mul_rn(g, mul_right_in(Tab::a(m, k))) * hh;
         }
 #pragma unroll
         for (int k = 0; k < P; k++)
             ms[k] += gp[k];
     }
-    return !r.beyond(kChainRange) && !neg_zero;
+    return !r.beyond(kChainRange);
 }
 
 } // namespace va
