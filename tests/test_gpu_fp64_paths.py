@@ -175,3 +175,34 @@ def test_lotka_volterra_warps(oracle, cuda, N, tab, B):
     for r in res[1:]:
         for a, b in zip(r, res[0]):
             np.testing.assert_array_equal(a, b)
+
+
+@pytest.mark.parametrize("model", sorted(NP))
+@pytest.mark.parametrize("tab", ["dopri5", "ck54"])
+@pytest.mark.parametrize("B,nout", [(1, 2), (33, 3), (700, 2), (2500, 5)])
+def test_two_seeds_at_once(cuda, model, tab, B, nout):
+    """Seed rows two at a time against one call per seed row: gradients, status and lambda history, an odd last seed, direct
+    gradients, failed instances, instances without a step, a seed that is not finite."""
+    y0, p, t1 = draw(model, B, B + nout)
+    n, P = y0.shape[1], p.shape[1]
+    if B > 10:
+        p[3, 0], t1[4], y0[5, 0] = np.nan, 0.0, np.inf
+    rng = np.random.default_rng(nout)
+    lam, mud = rng.standard_normal((B, nout, n)), rng.standard_normal((B, nout, P))
+    if B > 10:
+        lam[7, 0, 0], lam[8, nout - 1, 0] = np.inf, np.nan
+    got = []
+    for rows in [range(nout)] + [[k] for k in range(nout)]:
+        s = Solver(model, n, P, B, nout=len(rows), tableau=tab, precision="fp64", atol=1e-6, rtol=1e-6)
+        s.set_adjoint_history(6)
+        s.forward(dev(y0), dev(p), dev(np.zeros(B)), dev(t1))
+        g = s.backward(dev(p), dev(lam[:, rows]), dev(mud[:, rows]))
+        hist = [s.adjoint_history(b)[1] for b in {0, B - 1}]
+        got.append([g[k].cpu().numpy() for k in ("dy0", "dp", "status")] + [hist])
+        s.close()
+    for k in range(nout):
+        for both, one in zip(got[0][:2], got[1 + k][:2]):
+            np.testing.assert_array_equal(both[:, k], one[:, 0])
+        for both, one in zip(got[0][3], got[1 + k][3]):
+            np.testing.assert_array_equal(both[k], one[0])
+    np.testing.assert_array_equal(got[0][2], got[nout][2])  # the last seed row's status

@@ -227,6 +227,8 @@ void fp64_path(va_handle *h)
             for (const va::TeamKernel &c : k->team[t][w])
                 if (c.fn)
                     h->teams[w].push_back(c);
+    if (!h->teams[va::FP64_BACKWARD].empty() && k->pair[t].fn && h->prob.nout > 1)
+        h->teams[va::FP64_BACKWARD].front() = k->pair[t];
     if (!k->int_fwd[t])
         return;
     if (h->prob.batch >= k->int_fwd_min)

@@ -28,8 +28,9 @@ namespace va {
 // segments are fewer to share out, and launch_teams lowers the limits for them
 // (stride 50, ~250 steps: 9,001 instances 7.7 with 16 lanes, 7.3 with one).
 template <class M, class Tab>
-static void fill(TeamKernel (&t)[kFp64Sweeps][kTeams])
+static void fill(TeamKernel (&t)[kFp64Sweeps][kTeams], TeamKernel &pair)
 {
+    pair = {(const void *)backward_team_kernel<M, Tab, 32, 2>, 32, 2, 4.0f};
     t[FP64_FORWARD][0] = {(const void *)forward_team_kernel<M, Tab, 16>, 16, 2, 4.0f};
     t[FP64_FORWARD][1] = {(const void *)forward_team_kernel<M, Tab, 4>, 4, 1, 6.6f};
     t[FP64_FORWARD][2] = {(const void *)forward_team_kernel<M, Tab, 2>, 2, 1, 13.0f};
@@ -42,8 +43,8 @@ static void fill(TeamKernel (&t)[kFp64Sweeps][kTeams])
 template <class M>
 static void fill_model(Fp64Kernels &k)
 {
-    fill<M, TabDopri5>(k.team[0]);
-    fill<M, TabCK54>(k.team[1]);
+    fill<M, TabDopri5>(k.team[0], k.pair[0]);
+    fill<M, TabCK54>(k.team[1], k.pair[1]);
 }
 
 void fill_team_vdp(Fp64Kernels &k) { fill_model<ModelVdP>(k); }

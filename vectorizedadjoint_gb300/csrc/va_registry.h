@@ -113,6 +113,9 @@ struct Fp64Kernels {
     const void *int_fwd[kTableaux], *int_bwd[kTableaux];
     int int_fwd_min, int_bwd_min; // smallest batches they take
     TeamKernel team[kTableaux][kFp64Sweeps][kTeams]; // widest first
+    // two seed rows at once: takes the place of the widest backward team when
+    // there are two or more
+    TeamKernel pair[kTableaux];
 };
 // the team sweeps (va_inst_team_fp64.cu, va_inst_team_rkf78_fp64.cu)
 void fill_team_vdp(Fp64Kernels &k);

@@ -37,29 +37,25 @@
 namespace va {
 
 // Rows of the forward sums.  Order (rank): y_new, error, X_{s-1} .. X_1,
-// error denominator; a fixed-step tableau has no error rows.  Slot
-// rank * N + i is kept by lane slot % G as its accumulator slot / G.
+// error denominator.  Slot rank * N + i is kept by lane slot % G as its
+// accumulator slot / G.
 template <class Tab, int N, int G>
 struct TeamRows {
     static constexpr int NS = Tab::S;
-    static constexpr int E = Tab::FIXED ? 0 : 1;
-    static constexpr int R = NS + 2 * E;
+    static constexpr int R = NS + 2;
     static constexpr int Q = (R * N + G - 1) / G;
     static constexpr int rank_b = 0, rank_e = 1, rank_d = R - 1;
-    __host__ __device__ static constexpr int rank_x(int m) { return E + NS - m; }
+    __host__ __device__ static constexpr int rank_x(int m) { return NS + 1 - m; }
     // weight of K_j in the row (the denominator's 1 |K_0|)
     __host__ __device__ static constexpr double coef(int rank, int j)
     {
         if (rank == rank_b)
             return j < NS ? Tab::b(j) : 0.0;
-        if (E && rank == rank_e) {
-            if constexpr (!Tab::FIXED)
-                return j < NS ? Tab::e(j) : Tab::E_NEW;
-            return 0.0;
-        }
-        if (E && rank == rank_d)
+        if (rank == rank_e)
+            return j < NS ? Tab::e(j) : Tab::E_NEW;
+        if (rank == rank_d)
             return j == 0 ? 1.0 : 0.0;
-        const int m = E + NS - rank;
+        const int m = NS + 1 - rank;
         return j < m && j < NS ? Tab::a(m, j) : 0.0;
     }
     // whether the row takes a term at j: the stages take every j < m (their
@@ -67,11 +63,11 @@ struct TeamRows {
     // non-zero ones, the denominator its two
     __host__ __device__ static constexpr bool used(int rank, int j)
     {
-        if (rank == rank_b || (E && rank == rank_e))
+        if (rank == rank_b || rank == rank_e)
             return coef(rank, j) != 0.0;
-        if (E && rank == rank_d)
+        if (rank == rank_d)
             return j <= 1;
-        return j < E + NS - rank;
+        return j < NS + 1 - rank;
     }
     __host__ __device__ static constexpr bool any_used(int q, int j)
     {
@@ -93,7 +89,7 @@ struct TeamRows {
 template <class Tab, int N, int G>
 struct TeamForwardTable {
     using Rows = TeamRows<Tab, N, G>;
-    static constexpr int J = Tab::FIXED ? Tab::S : Tab::S + 1, W = Rows::Q * G;
+    static constexpr int J = Tab::S + 1, W = Rows::Q * G;
     double c[J][W];
     unsigned use[W];
     __host__ __device__ constexpr TeamForwardTable() : c(), use()
@@ -125,7 +121,7 @@ template <class M, class Tab, int G>
 struct TeamForward {
     static constexpr int N = M::N, NS = Tab::S;
     using Rows = TeamRows<Tab, N, G>;
-    static constexpr int Q = Rows::Q, J = Tab::FIXED ? NS : NS + 1;
+    static constexpr int Q = Rows::Q, J = NS + 1;
     double c[J][Q];
     int comp[Q];
     unsigned use[Q];      // bit j: the row takes a term at j
@@ -139,8 +135,8 @@ struct TeamForward {
             const int s = team.index + G * q;
             comp[q] = s % N;
             use[q] = kTeamForward<Tab, N, G>.use[s];
-            err[q] = Rows::E && s / N == Rows::rank_e;
-            den[q] = Rows::E && s / N == Rows::rank_d;
+            err[q] = s / N == Rows::rank_e;
+            den[q] = s / N == Rows::rank_d;
 #pragma unroll
             for (int j = 0; j < J; j++)
                 c[j][q] = kTeamForward<Tab, N, G>.c[j][s];
@@ -162,7 +158,7 @@ struct TeamForward {
         for (int q = 0; q < Q; q++)
             if (Rows::any_used(q, j)) {
                 double w = c[j][q] * dt, k = pick<N>(K, comp[q]), s = acc[q];
-                const bool dq = Rows::E && Rows::has(q, Rows::rank_d);
+                const bool dq = Rows::has(q, Rows::rank_d);
                 if (dq && j == 1) { // the denominator's atol + rtol (|y| + |dt K_0|)
                     w = den[q] ? rtol : w;
                     k = den[q] ? s : k;
@@ -175,12 +171,12 @@ struct TeamForward {
                 // rows that must not take the term: y_new and the error where
                 // their weight is zero, the denominator; a finished stage is
                 // not read again
-                const bool keep = Rows::has(q, Rows::rank_b) || (Rows::E && Rows::has(q, Rows::rank_e)) || dq;
+                const bool keep = Rows::has(q, Rows::rank_b) || Rows::has(q, Rows::rank_e) || dq;
                 acc[q] = !keep || (use[q] >> j & 1u) ? s : acc[q];
             }
     }
 
-    // attempt_pair / step_fixed, the results on every lane
+    // attempt_pair, the results on every lane
     __device__ __forceinline__ double attempt(const double (&y)[N], const double (&k0)[N], const double (&p)[M::P],
                                               double t, double dt, double atol, double rtol, double (&ynew)[N],
                                               double (&knew)[N]) const
@@ -189,9 +185,9 @@ struct TeamForward {
 #pragma unroll
         for (int q = 0; q < Q; q++) {
             acc[q] = pick<N>(y, comp[q]);
-            if (Rows::E && Rows::has(q, Rows::rank_d))
+            if (Rows::has(q, Rows::rank_d))
                 acc[q] = den[q] ? fabs(acc[q]) : acc[q];
-            if (Rows::E && Rows::has(q, Rows::rank_e))
+            if (Rows::has(q, Rows::rank_e))
                 acc[q] = err[q] ? -0.0 : acc[q]; // -0 + x = x: the first term
         }
         add(acc, 0, k0, dt, atol, rtol);
@@ -207,31 +203,27 @@ struct TeamForward {
 #pragma unroll
         for (int i = 0; i < N; i++)
             ynew[i] = row(acc, Rows::rank_b, i);
-        if constexpr (Tab::FIXED) {
-            return 0.0;
-        } else {
-            if constexpr (Tab::FSAL) {
-                M::template rhs<double>(ynew, p, t + dt, knew);
-                add(acc, NS, knew, dt, atol, rtol);
-            }
-            double worst = 0.0;
-            if constexpr (Q == 1) {
-                // every lane forms the quotient of its own component, the
-                // error rows' ones are those of the components
-                const int from = team.base + (Rows::rank_e * N + comp[0]) % G;
-                const int dfrom = team.base + (Rows::rank_d * N + comp[0]) % G;
-                const double e = shfl(acc[0], from, team.mask), d = shfl(acc[0], dfrom, team.mask);
-                const double r = quotient64(fabs(e), d);
-#pragma unroll
-                for (int i = 0; i < N; i++)
-                    worst = worse(worst, shfl(r, team.base + i, team.mask));
-            } else {
-#pragma unroll
-                for (int i = 0; i < N; i++)
-                    worst = worse(worst, quotient64(fabs(row(acc, Rows::rank_e, i)), row(acc, Rows::rank_d, i)));
-            }
-            return worst;
+        if constexpr (Tab::FSAL) {
+            M::template rhs<double>(ynew, p, t + dt, knew);
+            add(acc, NS, knew, dt, atol, rtol);
         }
+        double worst = 0.0;
+        if constexpr (Q == 1) {
+            // every lane forms the quotient of its own component, the
+            // error rows' ones are those of the components
+            const int from = team.base + (Rows::rank_e * N + comp[0]) % G;
+            const int dfrom = team.base + (Rows::rank_d * N + comp[0]) % G;
+            const double e = shfl(acc[0], from, team.mask), d = shfl(acc[0], dfrom, team.mask);
+            const double r = quotient64(fabs(e), d);
+#pragma unroll
+            for (int i = 0; i < N; i++)
+                worst = worse(worst, shfl(r, team.base + i, team.mask));
+        } else {
+#pragma unroll
+            for (int i = 0; i < N; i++)
+                worst = worse(worst, quotient64(fabs(row(acc, Rows::rank_e, i)), row(acc, Rows::rank_d, i)));
+        }
+        return worst;
     }
     // the larger, a NaN kept
     __device__ __forceinline__ static double worse(double a, double b)
@@ -260,43 +252,47 @@ __device__ constexpr TeamBackwardTable<Tab, N, P, G> kTeamBackward{};
 // Rows of the backward sums.  Slots: lambda (N), mu (P), then K-bar_k
 // component i at N + P + k N + i.  The model gives its VJP outputs o (gx, then
 // gp) as w[kVjpW] W_o(x), plus w[0] for o = kVjpAdd (vjp_weights).
-template <class M, class Tab, int G>
+// SEEDS seed rows at once: H = G / SEEDS lanes each hold a seed's rows, and
+// the weights serve all of them.
+template <class M, class Tab, int G, int SEEDS = 1>
 struct TeamBackward {
+    static constexpr int H = G / SEEDS;
     static constexpr int N = M::N, P = M::PG, NS = Tab::S;
-    static constexpr int SLOTS = N + P + NS * N, Q = (SLOTS + G - 1) / G;
+    static constexpr int SLOTS = N + P + NS * N, Q = (SLOTS + H - 1) / H;
     using Weights = double[NS][N + P];
     double ca[NS][Q]; // a_mk of the lane's K-bar_k
     double cb[Q];     // b_k
     int kind[Q];      // 0 lambda, 1 mu, 2 K-bar
     int comp[Q];      // component (lambda, K-bar) or parameter (mu)
     LaneGroup<G> team;
+    int seed, rows; // the lane's seed of the team's, and the first lane with that seed's rows
 
-    __device__ __forceinline__ TeamBackward()
+    __device__ __forceinline__ TeamBackward() : seed(team.index / H), rows(team.base + team.index / H * H)
     {
 #pragma unroll
         for (int q = 0; q < Q; q++) {
-            const int s = team.index + G * q;
+            const int s = team.index % H + H * q;
             kind[q] = s < N ? 0 : s < N + P ? 1 : 2;
             comp[q] = s < N ? s : s < N + P ? s - N : (s - N - P) % N;
-            cb[q] = kTeamBackward<Tab, N, P, G>.cb[s];
+            cb[q] = kTeamBackward<Tab, N, P, H>.cb[s];
 #pragma unroll
             for (int m = 0; m < NS; m++)
-                ca[m][q] = kTeamBackward<Tab, N, P, G>.ca[m][s];
+                ca[m][q] = kTeamBackward<Tab, N, P, H>.ca[m][s];
         }
     }
 
     // Whether accumulator q holds a row that stage m adds to
     __host__ __device__ static constexpr bool live(int q, int m)
     {
-        for (int s = q * G; s < (q + 1) * G && s < SLOTS; s++)
+        for (int s = q * H; s < (q + 1) * H && s < SLOTS; s++)
             if (s < N + P || (s - N - P) / N < m)
                 return true;
         return false;
     }
-    __host__ __device__ static constexpr bool only_kbar(int q) { return q * G >= N + P; }
+    __host__ __device__ static constexpr bool only_kbar(int q) { return q * H >= N + P; }
     __host__ __device__ static constexpr bool only_sums(int q, int m)
     {
-        for (int s = q * G; s < (q + 1) * G && s < SLOTS; s++)
+        for (int s = q * H; s < (q + 1) * H && s < SLOTS; s++)
             if (s >= N + P && (s - N - P) / N < m)
                 return false;
         return true;
@@ -311,7 +307,7 @@ struct TeamBackward {
     }
     __device__ __forceinline__ double param(const double (&mu)[Q], int k) const
     {
-        return shfl(mu[(N + k) / G], team.base + (N + k) % G, team.mask);
+        return shfl(mu[(N + k) / H], rows + (N + k) % H, team.mask);
     }
 
     // VJP weights of every stage of this lane's step (back_step's recompute)
@@ -329,7 +325,7 @@ struct TeamBackward {
     }
 
     // back_step with the weights that lane `from` of the team holds and its
-    // step's h: lam on every lane, mu in its lanes
+    // step's h: lam on every lane of the seed, mu in its lanes
     __device__ __forceinline__ void step(const Weights &W, int from, double h, double (&lam)[N], double (&mu)[Q]) const
     {
         const int src = team.base + from;
@@ -347,7 +343,7 @@ struct TeamBackward {
 #pragma unroll
             for (int i = 0; i < N; i++) {
                 const int s = N + P + m * N + i;
-                w[i] = shfl(acc[s / G], team.base + s % G, team.mask);
+                w[i] = shfl(acc[s / H], rows + s % H, team.mask);
             }
 #pragma unroll
             for (int o = 0; o < N + P; o++)
@@ -369,7 +365,7 @@ struct TeamBackward {
         }
 #pragma unroll
         for (int i = 0; i < N; i++)
-            lam[i] = shfl(acc[i / G], team.base + i % G, team.mask);
+            lam[i] = shfl(acc[i / H], rows + i % H, team.mask);
 #pragma unroll
         for (int q = 0; q < Q; q++)
             mu[q] = acc[q];
@@ -391,7 +387,7 @@ __global__ void __launch_bounds__(256) forward_team_kernel(FwdParams a)
     const int CH = a.pool.chunk_len;
 
     int b = -1;
-    double y[N], k0[N], p[P], t = 0.0, t1 = 0.0, dt = 0.0, t_start = 0.0;
+    double y[N], k0[N], p[P], t = 0.0, t1 = 0.0, dt = 0.0;
     int count = 0, rej = 0, fails = 0, status = ST_OK, chunk = -1, slot = 0;
     bool at_top = true;
 
@@ -414,7 +410,7 @@ __global__ void __launch_bounds__(256) forward_team_kernel(FwdParams a)
 #pragma unroll
         for (int k = 0; k < P; k++)
             p[k] = a.par[(size_t)b * P + k];
-        t = t_start = a.t0[b];
+        t = a.t0[b];
         t1 = a.t1[b];
         dt = a.dt0;
         count = rej = fails = 0;
@@ -482,8 +478,6 @@ __global__ void __launch_bounds__(256) forward_team_kernel(FwdParams a)
         note_work(a, b, count + rej);
         if (a.inst_t1)
             a.inst_t1[b] = t1;
-        if (Tab::FIXED && a.inst_t0)
-            a.inst_t0[b] = t_start;
         if (a.n_acc_out)
             a.n_acc_out[b] = count;
         if (a.n_rej_out)
@@ -500,7 +494,7 @@ __global__ void __launch_bounds__(256) forward_team_kernel(FwdParams a)
             continue;
         }
         if (at_top) {
-            if (Tab::FIXED ? !less_equal_pos64((t + dt) - t1, kDblEps) : !greater_pos64(t1 - t, kDblEps)) {
+            if (!greater_pos64(t1 - t, kDblEps)) {
                 finish();
                 alive = fetch();
                 continue;
@@ -516,7 +510,7 @@ __global__ void __launch_bounds__(256) forward_team_kernel(FwdParams a)
                 }
                 write();
             }
-            if (!Tab::FIXED && greater_pos64((t + dt) - t1, kDblEps))
+            if (greater_pos64((t + dt) - t1, kDblEps))
                 dt = t1 - t;
             fails = 0;
             at_top = false;
@@ -534,12 +528,8 @@ __global__ void __launch_bounds__(256) forward_team_kernel(FwdParams a)
             rej++;
             ok = false;
         } else {
-            if constexpr (Tab::FIXED) {
-                t = fixed_time(t_start, count + 1, dt);
-            } else {
-                t += dt;
-                dt = increase_step<Tab, double>(dt, err, a.step_pow, undecided);
-            }
+            t += dt;
+            dt = increase_step<Tab, double>(dt, err, a.step_pow, undecided);
             accept_state<M, Tab, double>(y, y, k0, ynew, ynew, knew, p, t);
             ok = true;
         }
@@ -592,25 +582,28 @@ __device__ __forceinline__ void team_store(const AdjParams &a, int b, int q, con
         a.dpar[o * P + k] = d + mu[k];
         finite = finite && is_finite64(mu[k]);
     }
-    if (a.status_out && (q == a.nout - 1 || !finite))
+    if (a.status_out && q == a.nout - 1)
         a.status_out[b] = finite ? ST_OK : ST_NONFINITE;
 }
 
-// backward_kernel with the steps spread over a team
-template <class M, class Tab, int G>
+// backward_kernel with the steps spread over a team, SEEDS seed rows at once.
+// Two seed rows in the halves of a warp, where one half holds a seed's rows
+// (the 5(4) pairs): the recompute serves both, and the chain through lambda is
+// issued once for both.
+template <class M, class Tab, int G, int SEEDS = 1>
 __global__ void __launch_bounds__(256) backward_team_kernel(AdjParams a)
 {
     constexpr int N = M::N, P = M::P;
     constexpr int RS = record_doubles(N);
-    using TB = TeamBackward<M, Tab, G>;
+    using TB = TeamBackward<M, Tab, G, SEEDS>;
     if (gated_off(a))
         return;
     const TB tb;
     const int me = tb.team.index;
-    const bool first = me == 0;
+    const bool first = me == 0, writes = me % TB::H == 0;
     const int CH = a.pool.chunk_len;
 
-    int b = -1, q = 0, j = -1, chunk = -1, slot = 0, T = 0, last = -1;
+    int b = -1, q = 0 /* the team's first seed */, j = -1, chunk = -1, slot = 0, T = 0, last = -1;
     int ready = 0, pos = 0; // steps whose weights the lanes hold, and the next of them
     double lam[N], mu[TB::Q], t_next = 0.0, p[P], h = 0.0;
     typename TB::Weights W;
@@ -640,13 +633,15 @@ __global__ void __launch_bounds__(256) backward_team_kernel(AdjParams a)
         slot = T % CH;
         double yTl[N];
         read_record<N>(record_ptr<RS>(a.pool, chunk, slot), t_next, yTl);
-        const size_t o = ((size_t)b * a.nout + q);
+        // an odd last seed fills the lanes of its successor too
+        const int mine = q + tb.seed < a.nout ? q + tb.seed : a.nout - 1;
+        const size_t o = ((size_t)b * a.nout + mine);
 #pragma unroll
         for (int i = 0; i < N; i++)
             lam[i] = a.cost == 0 ? 2.0 * yTl[i] : a.cost == 1 ? 1.0 : a.lambdaT[o * N + i];
         tb.clear(mu);
-        if (first)
-            note_lambda<N>(a, b, q, T, lam);
+        if (writes && q + tb.seed < a.nout)
+            note_lambda<N>(a, b, q + tb.seed, T, lam);
         j = T - 1;
         ready = pos = 0;
     };
@@ -683,10 +678,10 @@ __global__ void __launch_bounds__(256) backward_team_kernel(AdjParams a)
 #pragma unroll
             for (int k = 0; k < P; k++)
                 m[k] = tb.param(mu, k);
-            if (first)
-                team_store<N, P>(a, b, q, lam, m);
-            if (q + 1 < a.nout) {
-                q++;
+            if (writes && q + tb.seed < a.nout)
+                team_store<N, P>(a, b, q + tb.seed, lam, m);
+            if (q + SEEDS < a.nout) {
+                q += SEEDS;
                 start_seed();
             } else {
                 alive = fetch();
@@ -696,8 +691,8 @@ __global__ void __launch_bounds__(256) backward_team_kernel(AdjParams a)
         if (pos == ready)
             prepare();
         tb.step(W, pos, shfl(h, tb.team.base + pos, tb.team.mask), lam, mu);
-        if (first)
-            note_lambda<N>(a, b, q, j, lam);
+        if (writes && q + tb.seed < a.nout)
+            note_lambda<N>(a, b, q + tb.seed, j, lam);
         pos++;
         j--;
     }
@@ -733,7 +728,7 @@ __global__ void __launch_bounds__(256) backward_team_kernel_2level(AdjParams a)
     int b = -1, q = 0, j = -1, T = 0, R = 0, last = -1, chunk = -1, slot = 0;
     int top = 0, low = 0;   // the lanes hold the segments top, top - 1, .. of steps low .. j
     int ready = 0, pos = 0; // as backward_team_kernel
-    double lam[N], mu[TB::Q], t1 = 0.0, t_start = 0.0, t_end = 0.0, y_end[N], p[P], h = 0.0;
+    double lam[N], mu[TB::Q], t1 = 0.0, t_end = 0.0, y_end[N], p[P], h = 0.0;
     typename TB::Weights W;
 
     // Re-integrates the segments that end with step j; false: one of them did
@@ -784,7 +779,7 @@ __global__ void __launch_bounds__(256) backward_team_kernel_2level(AdjParams a)
         bool at_top = true, ok = true;
         while (run) {
             if (at_top) {
-                if (!Tab::FIXED && greater_pos64((t + dt) - t1, kDblEps))
+                if (greater_pos64((t + dt) - t1, kDblEps))
                     dt = t1 - t;
                 fails = 0;
                 at_top = false;
@@ -800,12 +795,8 @@ __global__ void __launch_bounds__(256) backward_team_kernel_2level(AdjParams a)
                 dt = decrease_step<Tab, double>(dt, err, a.step_pow, &a.ctl->pow_undecided);
                 continue;
             }
-            if constexpr (Tab::FIXED) {
-                t = fixed_time(t_start, first_step + done + 1, dt);
-            } else {
-                t += dt;
-                dt = increase_step<Tab, double>(dt, err, a.step_pow, &a.ctl->pow_undecided);
-            }
+            t += dt;
+            dt = increase_step<Tab, double>(dt, err, a.step_pow, &a.ctl->pow_undecided);
             accept_state<M, Tab, double>(y, y, k0, ynew, ynew, knew, p, t);
             at_top = true;
             done++;
@@ -863,8 +854,6 @@ __global__ void __launch_bounds__(256) backward_team_kernel_2level(AdjParams a)
             R = (T + SK - 1) / SK + 1;
             last = a.inst_last[b];
             t1 = a.inst_t1[b];
-            if constexpr (Tab::FIXED)
-                t_start = a.inst_t0[b];
             q = 0;
             start_seed();
             return true;
