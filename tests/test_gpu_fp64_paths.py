@@ -179,7 +179,7 @@ def test_lotka_volterra_warps(oracle, cuda, N, tab, B):
 
 @pytest.mark.parametrize("model", sorted(NP))
 @pytest.mark.parametrize("tab", ["dopri5", "ck54"])
-@pytest.mark.parametrize("B,nout", [(1, 2), (33, 3), (700, 2), (2500, 5)])
+@pytest.mark.parametrize("B,nout", [(1, 2), (33, 3), (700, 2), (2500, 5), (6000, 2)])
 def test_two_seeds_at_once(cuda, model, tab, B, nout):
     """Seed rows two at a time against one call per seed row: gradients, status and lambda history, an odd last seed, direct
     gradients, failed instances, instances without a step, a seed that is not finite."""

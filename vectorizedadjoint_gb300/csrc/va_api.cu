@@ -227,8 +227,8 @@ void fp64_path(va_handle *h)
             for (const va::TeamKernel &c : k->team[t][w])
                 if (c.fn)
                     h->teams[w].push_back(c);
-    if (!h->teams[va::FP64_BACKWARD].empty() && k->pair[t].fn && h->prob.nout > 1)
-        h->teams[va::FP64_BACKWARD].front() = k->pair[t];
+    if (!h->teams[va::FP64_BACKWARD].empty() && h->prob.nout > 1 && k->seeds_per_quad[t] > 0.0f)
+        h->teams[va::FP64_BACKWARD].front().per_quad = k->seeds_per_quad[t];
     if (!k->int_fwd[t])
         return;
     if (h->prob.batch >= k->int_fwd_min)
@@ -643,7 +643,7 @@ va_status launch_teams(va_handle *h, int sweep, Params &a, cudaStream_t s, bool 
         float to = t.per_quad * quads;
         if (two_level && h->stride > 16)
             to *= 256.0f / ((float)h->stride * (float)h->stride);
-        if (!decide && 0.55f * (float)B > to)
+        if (to <= from || (!decide && 0.55f * (float)B > to))
             continue;
         const int block = two_level ? kTwoLevelBlock : h->opt.block_size > 0 ? h->opt.block_size : 128;
         int bps = two_level ? kTwoLevelBlocksPerSm : t.bps;

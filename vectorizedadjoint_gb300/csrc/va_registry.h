@@ -108,14 +108,14 @@ inline int team_segments(int g, int stride)
     return n < 1 ? 1 : n < g ? n : g;
 }
 enum { FP64_FORWARD = 0, FP64_BACKWARD = 1, FP64_TWO_LEVEL = 2, kFp64Sweeps = 3 };
-constexpr int kTeams = 3;
+constexpr int kTeams = 4;
 struct Fp64Kernels {
     const void *int_fwd[kTableaux], *int_bwd[kTableaux];
     int int_fwd_min, int_bwd_min; // smallest batches they take
     TeamKernel team[kTableaux][kFp64Sweeps][kTeams]; // widest first
-    // two seed rows at once: takes the place of the widest backward team when
-    // there are two or more
-    TeamKernel pair[kTableaux];
+    // limit of the widest backward team when there are two seed rows or more
+    // (0: the listed one)
+    float seeds_per_quad[kTableaux];
 };
 // the team sweeps (va_inst_team_fp64.cu, va_inst_team_rkf78_fp64.cu)
 void fill_team_vdp(Fp64Kernels &k);
