@@ -96,61 +96,125 @@ __global__ void order_hist(OrderArgs a)
             atomicAdd(&a.work[i], h[i]);
 }
 
-// Exclusive scan from the top bucket down: offset of bucket k = number of
-// instances in buckets > k.  One block of 1024 threads, 4 buckets each.
-__global__ void order_scan(OrderArgs a)
+// Over one block of 1024 threads, thread t holding the counts v[j] of buckets
+// kBuckets - 1 - (4 t + j): the number of instances in the buckets above its
+// first (the exclusive scan from the top bucket down); and what the sort
+// leaves for the sweeps, the load and where a forward order came from.
+// Shuffles within the warps and two barriers; with a barrier for each of the
+// ten scan steps and the load summed by one thread the scan took ~2 us more.
+__device__ __forceinline__ int scan_from_top(const OrderArgs &a, const int (&v)[4])
+{
+    __shared__ int part[32];
+    __shared__ float sum[32], top[32];
+    const int t = threadIdx.x, lane = t & 31, warp = t >> 5;
+    const bool prev = a.prev_work && a.prev_valid && *a.prev_valid;
+    const bool counted = a.steps || prev;
+    const int s = v[0] + v[1] + v[2] + v[3];
+    int run = s;
+    float s1 = 0.0f, m1 = 0.0f;
+    if (s) {
+#pragma unroll
+        for (int j = 0; j < 4; j++) {
+            const float l = v[j] ? bucket_length(counted, kBuckets - 1 - (t * 4 + j)) : 0.0f;
+            s1 += l * (float)v[j];
+            m1 = fmaxf(m1, l);
+        }
+    }
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+        const int x = __shfl_up_sync(0xffffffffu, run, o);
+        run += lane >= o ? x : 0;
+        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+        m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+    }
+    if (lane == 31) {
+        part[warp] = run;
+        sum[warp] = s1;
+        top[warp] = m1;
+    }
+    __syncthreads();
+    if (warp == 0) {
+        const int own = part[lane];
+        int x = own;
+        s1 = sum[lane];
+        m1 = top[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int y = __shfl_up_sync(0xffffffffu, x, o);
+            x += lane >= o ? y : 0;
+            s1 += __shfl_xor_sync(0xffffffffu, s1, o);
+            m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
+        }
+        part[lane] = x - own;
+        if (t == 0) {
+            // at most one per instance, at least one instance's (a batch of length 0 too)
+            const float load = m1 > 0.0f ? s1 / m1 : 1.0f;
+            a.work[kLoadSlot] = __float_as_int(fminf(fmaxf(load, 1.0f), (float)a.B));
+            if (!a.steps) // a forward order: say whether it came from counts
+                a.work[kCountedFlag] = prev ? 1 : 0;
+        }
+    }
+    __syncthreads();
+    return part[warp] + run - s;
+}
+
+__global__ void __launch_bounds__(1024) order_scan(OrderArgs a)
 {
     if (reusing(a))
         return;
-    __shared__ int part[1024];
     const int t = threadIdx.x;
-    int v[4], s = 0;
-    for (int j = 0; j < 4; j++) {
+    int v[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++)
         v[j] = a.work[kBuckets - 1 - (t * 4 + j)];
-        s += v[j];
-    }
-    part[t] = s;
-    __syncthreads();
-    for (int o = 1; o < 1024; o <<= 1) {
-        const int x = t >= o ? part[t - o] : 0;
-        __syncthreads();
-        part[t] += x;
-        __syncthreads();
-    }
-    int run = t ? part[t - 1] : 0;
+    int run = scan_from_top(a, v);
+#pragma unroll
     for (int j = 0; j < 4; j++) {
         a.work[kBuckets + (kBuckets - 1 - (t * 4 + j))] = run;
         run += v[j];
     }
-    const bool prev = a.prev_work && a.prev_valid && *a.prev_valid;
-    if (t == 0 && !a.steps) // a forward order: say whether it came from counts
-        a.work[kCountedFlag] = prev ? 1 : 0;
-    __shared__ float sum[32], top[32];
-    const bool counted = a.steps || prev;
-    float s1 = 0.0f, m1 = 0.0f;
-    for (int j = 0; j < 4; j++) {
-        const float l = v[j] ? bucket_length(counted, kBuckets - 1 - (t * 4 + j)) : 0.0f;
-        s1 += l * (float)v[j];
-        m1 = fmaxf(m1, l);
+}
+
+// The whole sort of a small batch in one block, the buckets in shared memory
+// and four keys a thread in registers: one launch where the large batch's
+// memset and three kernels are four, ~2 us each.
+constexpr int kSmallBatch = 4 * 1024;
+__global__ void __launch_bounds__(1024) order_small(OrderArgs a)
+{
+    __shared__ int cnt[kBuckets];
+    const int t = threadIdx.x;
+    if (reusing(a)) {
+        for (int b = t; b < a.B; b += 1024)
+            a.order[b] = a.reuse[b];
+        return;
     }
-    for (int o = 16; o; o >>= 1) {
-        s1 += __shfl_xor_sync(0xffffffffu, s1, o);
-        m1 = fmaxf(m1, __shfl_xor_sync(0xffffffffu, m1, o));
-    }
-    if ((t & 31) == 0) {
-        sum[t >> 5] = s1;
-        top[t >> 5] = m1;
+    int key[4];
+#pragma unroll
+    for (int i = 0; i < 4; i++) {
+        cnt[t + 1024 * i] = 0;
+        key[i] = t + 1024 * i < a.B ? key_of(a, t + 1024 * i) : -1;
     }
     __syncthreads();
-    if (t == 0) {
-        for (int w = 1; w < 32; w++) {
-            s1 += sum[w];
-            m1 = fmaxf(m1, top[w]);
-        }
-        // at most one per instance, at least one instance's (a batch of length 0 too)
-        const float load = m1 > 0.0f ? s1 / m1 : 1.0f;
-        a.work[kLoadSlot] = __float_as_int(fminf(fmaxf(load, 1.0f), (float)a.B));
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        if (key[i] >= 0)
+            atomicAdd(&cnt[key[i]], 1);
+    __syncthreads();
+    int v[4];
+#pragma unroll
+    for (int j = 0; j < 4; j++)
+        v[j] = cnt[kBuckets - 1 - (t * 4 + j)];
+    int run = scan_from_top(a, v);
+#pragma unroll
+    for (int j = 0; j < 4; j++) {
+        cnt[kBuckets - 1 - (t * 4 + j)] = run;
+        run += v[j];
     }
+    __syncthreads();
+#pragma unroll
+    for (int i = 0; i < 4; i++)
+        if (key[i] >= 0)
+            a.order[atomicAdd(&cnt[key[i]], 1)] = t + 1024 * i;
 }
 
 // Each block takes a contiguous range of instances: it counts its range per
@@ -190,6 +254,10 @@ const float *order_load(const int *work) { return reinterpret_cast<const float *
 
 cudaError_t enqueue_order(const OrderArgs &a, cudaStream_t s)
 {
+    if (a.B <= kSmallBatch) {
+        order_small<<<1, 1024, 0, s>>>(a);
+        return cudaGetLastError();
+    }
     cudaError_t e = cudaMemsetAsync(a.work, 0, sizeof(int) * kBuckets, s);
     if (e != cudaSuccess)
         return e;
