@@ -206,3 +206,47 @@ def test_two_seeds_at_once(cuda, model, tab, B, nout):
         for both, one in zip(got[0][3], got[1 + k][3]):
             np.testing.assert_array_equal(both[k], one[0])
     np.testing.assert_array_equal(got[0][2], got[nout][2])  # the last seed row's status
+
+
+@pytest.mark.parametrize("B,nout", [(4097, 1), (12000, 1), (12000, 2), (40000, 1)])
+@pytest.mark.parametrize("tab", ["dopri5", "ck54"])
+def test_longest_instances_apart(cuda, tab, B, nout):
+    """Uneven batches, whose longest instances run in teams beside the rest, against the same call in an explicit launch
+    shape (one sweep for all): every instance's outputs, failed instances, short chunks, the lambda history, a stream of
+    its own with graph replays."""
+    rng = np.random.default_rng(B)
+    y0, p, _ = draw("dho", B, B)
+    t1 = np.exp(rng.uniform(np.log(0.2), np.log(30.0), B))
+    p[3, 0], t1[4], y0[5, 0] = np.nan, 0.0, np.inf
+    t1[6], p[6] = 80.0, (5.0, 0.0)  # out of steps
+    lam, mud = rng.standard_normal((B, nout, 2)), rng.standard_normal((B, nout, 2))
+    got, keys = [], ("yT", "n_acc", "n_rej", "status")
+    for kw in (dict(block_size=64), dict(), dict(chunk_len=3)):
+        s = Solver("dho", 2, 2, B, nout=nout, tableau=tab, precision="fp64", atol=1e-7, rtol=1e-7, max_steps=900, **kw)
+        s.set_adjoint_history(3)
+        for _ in range(2):  # ordered by horizon, then by counts
+            f = s.forward(dev(y0), dev(p), dev(np.zeros(B)), dev(t1))
+            g = s.backward(dev(p), dev(lam), dev(mud))
+            got.append([f[k].cpu().numpy() for k in keys] + [g[k].cpu().numpy() for k in ("status", "dy0", "dp")] +
+                       [s.adjoint_history(b)[1] for b in (0, int(np.argmax(t1 * (np.arange(B) != 6))))])
+        s.close()
+    assert got[0][3][6] != 0 and (got[0][3] == 0).sum() >= B - 4
+    for r in got[1:]:
+        for a, b in zip(r, got[0]):
+            np.testing.assert_array_equal(a, b)
+    if nout > 1:
+        return
+    s = Solver("dho", 2, 2, B, tableau=tab, precision="fp64", atol=1e-7, rtol=1e-7, max_steps=900)
+    ins = [dev(v) for v in (y0, p, np.zeros(B), t1)]
+    side = torch.cuda.Stream()
+    side.wait_stream(torch.cuda.current_stream())
+    with torch.cuda.stream(side):
+        for _ in range(3):
+            r = s.gradient("sumsq", *ins)
+    side.synchronize()
+    np.testing.assert_array_equal(r["yT"].cpu().numpy(), got[0][0])
+    np.testing.assert_array_equal(r["n_acc"].cpu().numpy(), got[0][1])
+    ref = Solver("dho", 2, 2, B, tableau=tab, precision="fp64", atol=1e-7, rtol=1e-7, max_steps=900, block_size=64)
+    want = ref.gradient("sumsq", *ins)
+    for k in ("dy0", "dp", "status"):
+        np.testing.assert_array_equal(r[k].cpu().numpy(), want[k].cpu().numpy())

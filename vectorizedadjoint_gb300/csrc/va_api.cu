@@ -60,6 +60,10 @@ struct va_handle {
     // and teams of lanes for smaller loads, widest first
     const void *sw_fwd = nullptr, *sw_bwd = nullptr;
     std::vector<va::TeamKernel> teams[va::kFp64Sweeps];
+    // the longest instances of an uneven batch in a sweep of their own (split_path)
+    va::TeamKernel long_fwd{}, long_bwd{};
+    cudaStream_t side = nullptr;
+    cudaEvent_t fork = nullptr, join = nullptr;
     int bps = 0; // resident blocks per SM of the default launch shape (0: the occupancy limit)
     bool default_shape = true; // neither given by the caller nor tuned
     int N = 0, P = 0;
@@ -239,6 +243,28 @@ void fp64_path(va_handle *h)
         h->fwd_block = h->bwd_block = h->prob.batch > 256 * h->sm_count ? 256 : 128;
         h->bps = 1;
     }
+}
+
+// A side stream for the longest instances of an uneven batch (split_rule):
+// one-thread models, 5(4) pairs, the default launch shape.  The longest
+// instance of a batch that is otherwise best left to one lane each would keep
+// its one lane busy long after the others are done; teams of 16 take the long
+// ones beside it.
+va_status split_path(va_handle *h)
+{
+    const va::Fp64Kernels *k = h->user || !h->ks ? nullptr : va::fp64_kernels(h->prob.model, h->N);
+    const int t = h->opt.tableau;
+    if (!k || h->opt.precision != VA_PREC_FP64 || h->ks->tpi != 1 || !k->int_fwd[t] || h->opt.block_size > 0 ||
+        h->opt.blocks_per_sm > 0 || h->prob.batch <= va::kSmallBatch)
+        return VA_OK;
+    h->long_fwd = k->team[t][va::FP64_FORWARD][0];
+    h->long_bwd = k->team[t][va::FP64_BACKWARD][h->prob.nout > 1 ? 0 : 1];
+    int low = 0, high = 0;
+    VA_CUDA(h, cudaDeviceGetStreamPriorityRange(&low, &high));
+    VA_CUDA(h, cudaEventCreateWithFlags(&h->fork, cudaEventDisableTiming));
+    VA_CUDA(h, cudaEventCreateWithFlags(&h->join, cudaEventDisableTiming));
+    VA_CUDA(h, cudaStreamCreateWithPriority(&h->side, cudaStreamNonBlocking, high));
+    return VA_OK;
 }
 
 int grid_for(va_handle *h, const void *fn, int block, int instances)
@@ -653,9 +679,10 @@ va_status launch_teams(va_handle *h, int sweep, Params &a, cudaStream_t s, bool 
                 bps = std::min(bps, h->opt.blocks_per_sm);
         }
         const int grid = team_grid(h, t, block, bps);
-        const bool last = !decide || (float)B <= to;
+        const bool last = !decide || ((float)B <= to && !a.split); // what is left of a split batch takes one lane each
         a.load_from = from;
         a.load_to = decide && !(last && from == 0.0f) ? (last ? 3.0e38f : to) : 0.0f;
+        a.part = a.split ? va::SPLIT_NEVER : va::SPLIT_NONE;
         VA_CUDA(h, launch(h, t.fn, grid, block, &a, s));
         if (!two_level && (last || !decide)) { // what va_get_launch reports
             (sweep == va::FP64_FORWARD ? h->fwd_team_block : h->bwd_team_block) = block;
@@ -670,6 +697,45 @@ va_status launch_teams(va_handle *h, int sweep, Params &a, cudaStream_t s, bool 
     a.load_from = from;
     a.load_to = decide ? 3.0e38f : 0.0f;
     a.rest_sms = rest;
+    a.part = a.split ? va::SPLIT_REST : va::SPLIT_NONE;
+    return VA_OK;
+}
+
+// When the batch is split: its load is above 1.5 warps' worth per quadrant
+// (below, teams of 16 take all of it as fast) and a quarter more than one lane
+// each (above, its throughput sets the pace), and no more than 2 of it are long.
+// Damped oscillators (lengths to 1,877 attempts, mean 210), forward + backward,
+// ms, unsplit and split: 10,000 instances (load per quadrant 1.8) 11.9, 10.7;
+// 20,000 (3.8) 13.2, 11.0; 65,536 (12) 22.5, 15.0 (with at most 0.5 long 18.5, 1
+// 16.2, 3 14.9; two blocks of teams per SM 17.0).  Van der Pol, where half of
+// the load is long, is not split or gains little: 20,000 instances 4.97, 4.75.
+void split_rule(const va_handle *h, va::OrderArgs &o)
+{
+    if (!h->side)
+        return;
+    const float quads = 4.0f * (float)h->sm_count;
+    o.split_from = 1.5f * quads;
+    o.split_to = 40.0f * quads;
+    o.split_load = 2.0f * quads;
+}
+
+// The sweep of the longest instances on the handle's side stream, beside the
+// launches that follow on s; join_long waits for it.  Without a split it
+// returns at once.
+template <class Params>
+va_status fork_long(va_handle *h, const va::TeamKernel &t, Params &a, cudaStream_t s)
+{
+    a.split = va::order_split(h->order_work);
+    a.part = va::SPLIT_LONG;
+    VA_CUDA(h, cudaEventRecord(h->fork, s));
+    VA_CUDA(h, cudaStreamWaitEvent(h->side, h->fork, 0));
+    VA_CUDA(h, launch(h, t.fn, h->sm_count, 128, &a, h->side));
+    VA_CUDA(h, cudaEventRecord(h->join, h->side));
+    return VA_OK;
+}
+va_status join_long(va_handle *h, cudaStream_t s)
+{
+    VA_CUDA(h, cudaStreamWaitEvent(s, h->join, 0));
     return VA_OK;
 }
 
@@ -734,6 +800,7 @@ va_status enqueue_forward(va_handle *h, const double *y0, const double *params, 
     if (h->order_fwd) {
         const int *valid = h->inst_work + a.B;
         va::OrderArgs o{a.B, nullptr, t0, t1, h->inst_work, valid, h->order_work, h->order_fwd, nullptr};
+        split_rule(h, o);
         VA_CUDA(h, va::enqueue_order(o, s));
         a.order = h->order_fwd;
         a.load = va::order_load(h->order_work);
@@ -742,12 +809,17 @@ va_status enqueue_forward(va_handle *h, const double *y0, const double *params, 
         a.work_valid = h->inst_work + a.B;
     }
     VA_CUDA(h, cudaMemsetAsync(h->ctl, 0, sizeof(va::Control), s));
+    if (h->side && a.load) {
+        const va_status st = fork_long(h, h->long_fwd, a, s);
+        if (st != VA_OK)
+            return st;
+    }
     bool one_lane;
     const va_status st = launch_teams(h, va::FP64_FORWARD, a, s, one_lane);
-    if (st != VA_OK || !one_lane)
-        return st;
-    VA_CUDA(h, launch(h, fn, h->fwd_grid, h->fwd_block, &a, s));
-    return VA_OK;
+    const cudaError_t e = st == VA_OK && one_lane ? launch(h, fn, h->fwd_grid, h->fwd_block, &a, s) : cudaSuccess;
+    const va_status joined = a.split ? join_long(h, s) : VA_OK;
+    VA_CUDA(h, e);
+    return st != VA_OK ? st : joined;
 }
 
 va_status enqueue_backward(va_handle *h, const double *params, const double *lambdaT,
@@ -776,6 +848,7 @@ va_status enqueue_backward(va_handle *h, const double *params, const double *lam
         // reused order made the backward 11% slower)
         const int *reuse = h->ks->tpi == 1 ? h->order_fwd : nullptr;
         va::OrderArgs o{a.B, h->inst_T, nullptr, nullptr, nullptr, nullptr, h->order_work, h->order_bwd, reuse};
+        split_rule(h, o);
         VA_CUDA(h, va::enqueue_order(o, s));
         a.order = h->order_bwd;
         a.load = va::order_load(h->order_work);
@@ -889,12 +962,18 @@ va_status enqueue_backward(va_handle *h, const double *params, const double *lam
     if (h->bwd_grid <= 0)
         h->bwd_grid = grid_for(h, fn, h->bwd_block, a.B);
     VA_CUDA(h, cudaMemsetAsync(&h->ctl->adj_next, 0, sizeof(unsigned int), s));
+    if (h->side && a.load) {
+        VA_CUDA(h, cudaMemsetAsync(&h->ctl->adj_long, 0, sizeof(unsigned int), s));
+        const va_status st = fork_long(h, h->long_bwd, a, s);
+        if (st != VA_OK)
+            return st;
+    }
     bool one_lane;
     const va_status st = launch_teams(h, va::FP64_BACKWARD, a, s, one_lane);
-    if (st != VA_OK || !one_lane)
-        return st;
-    VA_CUDA(h, launch(h, fn, h->bwd_grid, h->bwd_block, &a, s));
-    return VA_OK;
+    const cudaError_t e = st == VA_OK && one_lane ? launch(h, fn, h->bwd_grid, h->bwd_block, &a, s) : cudaSuccess;
+    const va_status joined = a.split ? join_long(h, s) : VA_OK;
+    VA_CUDA(h, e);
+    return st != VA_OK ? st : joined;
 }
 
 // CUDA events of one autotune sweep, destroyed on every return path
@@ -1261,6 +1340,10 @@ va_status create_handle(const va_problem *prob, const va_options *opt, const va:
         return VA_CUDA_ERROR;
     }
     fp64_path(h);
+    if (split_path(h) != VA_OK) {
+        va_destroy(h);
+        return VA_CUDA_ERROR;
+    }
     *out = h;
     return VA_OK;
 }
@@ -1331,6 +1414,11 @@ va_status va_destroy(va_handle *h)
     if (!h)
         return VA_BAD_ARGS;
     drop_graph(h);
+    if (h->side)
+        cudaStreamDestroy(h->side);
+    for (cudaEvent_t e : {h->fork, h->join})
+        if (e)
+            cudaEventDestroy(e);
     void *ptrs[] = {h->pool_rec, h->chunk_prev, h->inst_T,  h->inst_last, h->inst_status,
                     h->ctl,      h->s_y0,       h->s_par,   h->s_t0,      h->s_t1,
                     h->s_yT,     h->s_dy0,      h->s_dpar,  h->s_nacc,    h->s_status,

@@ -50,6 +50,7 @@ struct Control {
     unsigned int pool_next; // next free checkpoint chunk
     unsigned int pool_fail; // set when the pool ran out
     unsigned int pow_undecided; // step factors whose rounding test failed (cr_step_pow)
+    unsigned int fwd_long, adj_long; // next of the longest instances (SPLIT_LONG)
 };
 
 // Checkpoint pool: chunks of `chunk_len` records of `rs` doubles.
@@ -91,12 +92,27 @@ struct FwdParams {
     const float *load;   // the batch's load (va_order.cu; device float, may be null: no decisions)
     float load_from, load_to; // run only for load_from < load <= load_to (load_to 0: any)
     int rest_sms;        // SMs (blocks b, b + rest_sms, ... share one) for resting, 0: no rest
+    const int *split;    // device: how many of the longest instances a sweep of their own takes (0: none)
+    int part;            // this sweep's part of a split batch
 };
 
+// Parts of a split batch: no split for this sweep, the longest instances alone,
+// none of a split batch, the others (all of a batch that is not split).
+enum : int { SPLIT_NONE = 0, SPLIT_LONG = 1, SPLIT_NEVER = 2, SPLIT_REST = 3 };
+template <class Params>
+__device__ __forceinline__ int split_of(const Params &a)
+{
+    return a.part != SPLIT_NONE ? *a.split : 0;
+}
 // Whether another sweep of the same launch takes this batch.
 template <class Params>
 __device__ __forceinline__ bool gated_off(const Params &a)
 {
+    const int n = split_of(a);
+    if (a.part == SPLIT_LONG)
+        return n == 0;
+    if (n > 0)
+        return a.part == SPLIT_NEVER;
     return a.load && a.load_to > 0.0f && !(*a.load > a.load_from && *a.load <= a.load_to);
 }
 // Whether this warp stays idle: beyond the warps per quadrant that are useful
@@ -151,6 +167,8 @@ struct AdjParams {
     const float *load; // as FwdParams
     float load_from, load_to;
     int rest_sms;
+    const int *split; // as FwdParams
+    int part;
 };
 
 __host__ __device__ constexpr int record_doubles(int n) { return (2 + n + 1) & ~1; }
@@ -680,9 +698,10 @@ __global__ void __launch_bounds__(256) forward_kernel(FwdParams a)
     int count = 0, rej = 0, fails = 0, status = ST_OK, chunk = -1, slot = 0;
     bool at_top = true;
 
+    const int skip = split_of(a);
     // Take the next instance; false when the batch is exhausted.
     auto fetch = [&]() -> bool {
-        b = (int)atomicAdd(&a.ctl->fwd_next, 1u);
+        b = (int)atomicAdd(&a.ctl->fwd_next, 1u) + skip;
         if (b >= a.B)
             return false;
         if (a.order)
@@ -1046,9 +1065,10 @@ __global__ void __launch_bounds__(256) backward_kernel(AdjParams a)
         j = T - 1;
     };
 
+    const unsigned skip = (unsigned)split_of(a);
     auto fetch = [&]() -> bool {
         for (;;) {
-            unsigned w = atomicAdd(&a.ctl->adj_next, 1u);
+            unsigned w = atomicAdd(&a.ctl->adj_next, 1u) + skip;
             if ((int)w >= a.B)
                 return false;
             b = a.order ? a.order[w] : (int)w;

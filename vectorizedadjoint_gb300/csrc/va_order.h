@@ -7,6 +7,9 @@
 
 namespace va {
 
+// Batches up to this size are sorted in one block, without a split.
+constexpr int kSmallBatch = 4096;
+
 struct OrderArgs {
     int B;
     const int *steps;  // backward: accepted steps per instance (or null)
@@ -18,12 +21,17 @@ struct OrderArgs {
     int *order;        // [B] output permutation, longest first
     const int *reuse;  // backward: the forward's order, copied instead of sorting when
                        //   that order came from counts (flag in work); may be null
+    // When the batch may be split (order_split): above this load and up to
+    // that one (0: never), and the most load that goes into the longest part
+    float split_from, split_to, split_load;
 };
 
 size_t order_work_ints();
 // In `work`, on the device: the batch's load, the sum of its instances'
 // lengths in units of the longest, set with the order (see va_order.cu).
 const float *order_load(const int *work);
+// The number of longest instances that a sweep of their own should take.
+const int *order_split(const int *work);
 cudaError_t enqueue_order(const OrderArgs &a, cudaStream_t s);
 
 } // namespace va

@@ -398,9 +398,10 @@ __global__ void __launch_bounds__(256) forward_team_kernel(FwdParams a)
         return shfl(v, tf.team.base, tf.team.mask);
     };
 
+    const int limit = a.part == SPLIT_LONG ? split_of(a) : a.B;
     auto fetch = [&]() -> bool {
-        b = take(&a.ctl->fwd_next);
-        if (b >= a.B)
+        b = take(a.part == SPLIT_LONG ? &a.ctl->fwd_long : &a.ctl->fwd_next);
+        if (b >= limit)
             return false;
         if (a.order)
             b = a.order[b];
@@ -645,13 +646,14 @@ __global__ void __launch_bounds__(256) backward_team_kernel(AdjParams a)
         j = T - 1;
         ready = pos = 0;
     };
+    const int limit = a.part == SPLIT_LONG ? split_of(a) : a.B;
     auto fetch = [&]() -> bool {
         for (;;) {
             int w = 0;
             if (first)
-                w = (int)atomicAdd(&a.ctl->adj_next, 1u);
+                w = (int)atomicAdd(a.part == SPLIT_LONG ? &a.ctl->adj_long : &a.ctl->adj_next, 1u);
             w = shfl(w, tb.team.base, tb.team.mask);
-            if (w >= a.B)
+            if (w >= limit)
                 return false;
             b = a.order ? a.order[w] : w;
             const int st = a.inst_status[b];
