@@ -153,7 +153,7 @@ typedef struct {
                             correctly rounded, i.e. what odeint's std::pow gives
                             wherever the host libm rounds correctly, so the sweep
                             takes the reference's accepted steps; 0 -- Newton's
-                            inverse root (a few ulps off, ~25% cheaper per attempt).
+                            inverse root (a few ulps off; not cheaper).
                             The reduced precisions keep their own controllers     */
     int32_t tensor_products; /* shared-matrix GLV, N = 256, mixed_dw, every step
                             checkpointed with stage records: 0 (default) -- the
