@@ -648,7 +648,9 @@ int rest_sms(const va_handle *h)
 // every team whose turn can come (the load is at most the batch size) is
 // launched, and all but one return at once (~2 us each); one_lane tells
 // whether the one-lane sweep can take the batch too, and `a` is then set up
-// for it.  With a launch shape from the caller, or without an order: the one
+// for it.  A split batch (split_rule) takes none of these: its longest
+// instances are on the side stream, the others take one lane each.  With a
+// launch shape from the caller, or without an order: the one
 // that suits a load of 0.55 B, in that shape.
 template <class Params>
 va_status launch_teams(va_handle *h, int sweep, Params &a, cudaStream_t s, bool &one_lane)
