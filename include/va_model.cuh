@@ -56,6 +56,7 @@
 #include "va.h"
 #include "../vectorizedadjoint_gb300/csrc/va_kernels.cuh"
 #include "../vectorizedadjoint_gb300/csrc/va_kernels_dw.cuh"
+#include "../vectorizedadjoint_gb300/csrc/va_model_abi.h"
 #include "../vectorizedadjoint_gb300/csrc/va_registry.h"
 #include "../vectorizedadjoint_gb300/csrc/va_replay.cuh"
 

@@ -3,6 +3,7 @@ entry point include/va.h declares (no compute calls without a GPU)."""
 import ctypes
 import os
 import re
+import struct
 
 ROOT = os.path.dirname(os.path.dirname(os.path.abspath(__file__)))
 
@@ -60,3 +61,20 @@ def test_create_rejects_bad_problems(valib):
     o.tableau = 7
     p = _lib.VaProblem(0, 2, 1, 4, 1)
     assert L.va_create(ctypes.byref(p), ctypes.byref(o), ctypes.byref(h)) == 5
+
+
+def test_model_table_of_another_version_is_refused(valib):
+    """A caller's kernel table from headers with other parameter blocks (its version word differs) is refused before any
+    device call: its kernels would read past the end of the block the library passes."""
+    L = valib.load()
+    from vectorizedadjoint_gb300 import _lib
+    o = _lib.VaOptions()
+    L.va_default_options(ctypes.byref(o))
+    for abi in (0, 1, 2, 3):  # 1: the table before the blocks carried the batch's load
+        table = bytearray(b"\x01" * 4096)  # every kernel and launcher present
+        table[:20] = struct.pack("<IIiii", 0x4B4D4156, abi, 2, 1, 1)
+        buf = (ctypes.c_char * len(table)).from_buffer(table)
+        h = ctypes.c_void_p()
+        p = _lib.VaProblem(6, 2, 1, 4, 1)
+        assert L.va_create_model(ctypes.byref(p), ctypes.byref(o), ctypes.addressof(buf), ctypes.byref(h)) == 5, abi
+        assert not h.value

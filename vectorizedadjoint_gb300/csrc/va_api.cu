@@ -22,6 +22,7 @@
 #include "va_bundle_tc.cuh"
 #include "va_group_2level.cuh"
 #include "va_kernels.cuh"
+#include "va_model_abi.h"
 #include "va_order.h"
 #include "va_registry.h"
 #include "va_replay.cuh"

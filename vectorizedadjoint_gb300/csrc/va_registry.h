@@ -49,9 +49,9 @@ inline int record_doubles_for(const KernelSet *ks, int tableau, int precision, i
 // compiled in the same translation unit, so its kernels are launched through
 // the CUDA runtime they were registered with (the model's shared object may
 // link its own copy of the runtime).  magic and abi guard against a table
-// built from another version of the sweep templates.
+// built from another version of the sweep templates: abi is kModelAbi of
+// va_model_abi.h, which follows the layout of what the kernels are passed.
 constexpr uint32_t kModelMagic = 0x4B4D4156u; // "VAMK"
-constexpr uint32_t kModelAbi = 1;
 struct ModelKernels {
     uint32_t magic, abi;
     KernelSet set;
