@@ -106,6 +106,15 @@ def test_oracle_user_model_matches_reference(oracle, host_models, c):
         assert rel(g, np.array(fd)) < 1e-7
 
 
+def test_model_with_a_rate_of_its_own(tmp_path):
+    """A member that shares its name with one of the library's model hooks does not change what the sweeps call."""
+    from vectorizedadjoint_gb300 import build as vbuild
+    exe = str(tmp_path / "rate_model_check")
+    subprocess.run([vbuild.NVCC, "-gencode=arch=compute_103a,code=sm_103a", "-std=c++17", "-O1",
+                    "--expt-relaxed-constexpr", os.path.join(CPP, "rate_model_check.cu"), "-o", exe], check=True)
+    assert subprocess.run([exe], check=True, capture_output=True, text=True).stdout.strip() == "same"
+
+
 # ------------------------------------------------------------------- GPU
 
 

@@ -90,6 +90,7 @@ struct ModelGLVLane {
         }
     }
 
+    static constexpr bool kSharesRate = true;
     // r_i + sum_j A_ij x_j
     template <class S>
     __device__ __forceinline__ static S rate(const S *x, const S *p)

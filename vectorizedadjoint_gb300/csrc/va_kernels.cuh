@@ -861,12 +861,13 @@ __global__ void __launch_bounds__(256) forward_kernel(FwdParams a)
 // ----------------------------------------------------------- backward sweep
 
 // Models that share a part of f between the right-hand side and the VJP at the
-// same point (rate, vjp_rate: the lane-group Lotka-Volterra model).
-template <class M, class S, class = void>
-struct HasRate : std::false_type {
+// same point (rate, vjp_rate: the lane-group Lotka-Volterra model).  They say so
+// with kSharesRate: a caller's model may have a function `rate` of its own.
+template <class M, class = void>
+struct SharesRate : std::false_type {
 };
-template <class M, class S>
-struct HasRate<M, S, std::void_t<decltype(M::template rate<S>(nullptr, nullptr))>> : std::true_type {
+template <class M>
+struct SharesRate<M, std::void_t<decltype(M::kSharesRate)>> : std::bool_constant<M::kSharesRate> {
 };
 
 // One back_prop_step (backpropagation.hpp:160-229) for step n with state y_n,
@@ -884,7 +885,7 @@ __host__ __device__ __forceinline__ void back_step_general(const double (&y)[M::
     for (int i = 0; i < N; i++)
         ys[i] = from_d<S>(y[i]);
     const S shh = from_d<S>(h);
-    constexpr bool RATE = HasRate<M, S>::value;
+    constexpr bool RATE = SharesRate<M>::value;
     S rate[NS];
     // recompute the stages from y_n (compute_intermediate_states, :24-64)
 #pragma unroll
