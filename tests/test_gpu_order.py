@@ -33,3 +33,86 @@ def test_every_instance_once(cuda, precision, B):
     for g in got[1:]:
         for k in ("yT", "dy0", "dp", "n_acc", "status"):
             np.testing.assert_array_equal(g[k], got[0][k], err_msg=k)
+
+
+def inputs(model, B, seed, T):
+    rng = np.random.default_rng(seed)
+    if model == "vdp":
+        return rng.uniform(-2, 2, (B, 2)), 10 ** rng.uniform(-1, 1, (B, 1)), np.full(B, T)
+    if model == "dho":
+        return (rng.uniform(-1, 1, (B, 2)), np.stack([rng.uniform(0.5, 5.0, B), rng.uniform(0.0, 0.5, B)], 1),
+                rng.uniform(0.1 * T, T, B))
+    A = rng.normal(0, 0.1, (B, 5, 5))
+    A[:, np.arange(5), np.arange(5)] = -1.0
+    return rng.uniform(0.1, 1.0, (B, 5)), np.concatenate([rng.uniform(0.5, 1.5, (B, 5)), A.reshape(B, 25)], 1), np.full(B, T)
+
+
+def one_long(model, ins, T):
+    """The same batch with horizons of next to nothing but for one instance: a load of a few hundred at most."""
+    y0, p, t1 = ins
+    t1 = np.full_like(t1, 1e-3 * T)
+    t1[len(t1) // 2] = 4 * T
+    if model == "dho":
+        p = p.copy()
+        p[len(t1) // 2] = (5.0, 0.0)
+    return y0, p, t1
+
+
+@pytest.mark.parametrize("model,tab,precision,B,stride", [
+    ("vdp", "dopri5", "fp64", 9000, 0), ("vdp", "ck54", "fp64", 20000, 0), ("vdp", "rkf78", "fp64", 9000, 0),
+    ("dho", "ck54", "fp64", 20000, 0), ("vdp", "dopri5", "fp64", 9000, 4), ("vdp", "dopri5", "mixed", 40000, 0),
+    ("vdp", "dopri5", "mixed_dw", 70000, 0), ("dho", "ck54", "mixed_dw", 70000, 0), ("glv", "dopri5", "fp64", 3000, 0)])
+def test_other_inputs_than_the_call_before(cuda, model, tab, precision, B, stride):
+    """A batch after one whose lengths were quite others, in both directions: every output of a handle that has seen
+    nothing else (the sweeps that the wrong lengths chose hand their queue over; the backward sorts anew)."""
+    T = 5.0
+    a = inputs(model, B, 1, T)
+    b = one_long(model, a, T)
+    shape = a[0].shape[1], a[1].shape[1]
+
+    def run(*batches):
+        s, out = Solver(model, *shape, B, tableau=tab, precision=precision, ckpt_stride=stride), []
+        for y0, p, t1 in batches:
+            r = s.gradient("sumsq", dev(y0), dev(p), dev(np.zeros(B)), dev(t1))
+            out.append({k: v.cpu().numpy() for k, v in r.items()})
+            for v in r.values():
+                v.zero_()
+        s.close()
+        return out
+
+    wa, wb = run(a)[0], run(b)[0]
+    assert (wa["status"] == 0).all() and (wb["status"] == 0).all()
+    for want, got in zip((wa, wb, wb, wa, wa), run(a, b, b, a, a)):
+        for k in want:
+            np.testing.assert_array_equal(got[k], want[k], err_msg=k)
+
+
+@pytest.mark.parametrize("precision,B,limit", [("fp64", 65536, 3.0), ("mixed_dw", 262144, 1.9)])
+def test_time_after_other_inputs(cuda, precision, B, limit):
+    """The lengths of the call before choose the sweeps; when they are wrong a call must not take as long as the sweep they
+    chose would.  Times of a call against the same call repeated: chosen for one long instance and kept, FP64 teams of 16
+    take ~5 times as long on an even batch, one double-word warp per quadrant 2.2 times (all of them from the start, in an
+    order that says nothing: 1.5)."""
+    a = inputs("vdp", B, 1, 20.0)
+    b = one_long("vdp", a, 5.0)
+    s = Solver("vdp", 2, 1, B, precision=precision)
+    ins = [[dev(v) for v in (y0, p, np.zeros(B), t1)] for y0, p, t1 in (a, b)]
+
+    def timed(x):
+        e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+        torch.cuda.synchronize()
+        e[0].record()
+        s.gradient("sumsq", *x)
+        e[1].record()
+        torch.cuda.synchronize()
+        return e[0].elapsed_time(e[1])
+
+    timed(ins[0])
+    repeated = min(timed(ins[0]) for _ in range(3))
+    after = []
+    for _ in range(3):
+        timed(ins[1])
+        timed(ins[1])
+        after.append(timed(ins[0]))
+    s.close()
+    assert min(after) <= limit * repeated, (after, repeated)

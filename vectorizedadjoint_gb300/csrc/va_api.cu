@@ -423,11 +423,11 @@ va_status alloc_buffers(va_handle *h)
     if (!h->bks && h->opt.schedule == 0) {
         VA_CUDA(h, cudaMalloc(&h->order_fwd, (size_t)B * sizeof(int)));
         VA_CUDA(h, cudaMalloc(&h->order_bwd, (size_t)B * sizeof(int)));
-        VA_CUDA(h, cudaMalloc(&h->order_work, va::order_work_ints() * sizeof(int)));
-        VA_CUDA(h, cudaMemset(h->order_work, 0, va::order_work_ints() * sizeof(int)));
+        VA_CUDA(h, cudaMalloc(&h->order_work, va::order_work_ints(B) * sizeof(int)));
+        VA_CUDA(h, cudaMemset(h->order_work, 0, va::order_work_ints(B) * sizeof(int)));
         // attempts per instance of the last forward sweep, then its valid flag
         VA_CUDA(h, cudaMalloc(&h->inst_work, ((size_t)B + 1) * sizeof(int)));
-        VA_CUDA(h, cudaMemset(h->inst_work + B, 0, sizeof(int)));
+        VA_CUDA(h, cudaMemset(h->inst_work, 0, ((size_t)B + 1) * sizeof(int)));
     }
     if (h->bks) {
         const size_t NN = (size_t)h->N * h->N;
@@ -684,7 +684,7 @@ va_status launch_teams(va_handle *h, int sweep, Params &a, cudaStream_t s, bool 
         const int grid = team_grid(h, t, block, bps);
         const bool last = !decide || ((float)B <= to && !a.split); // what is left of a split batch takes one lane each
         a.load_from = from;
-        a.load_to = decide && !(last && from == 0.0f) ? (last ? 3.0e38f : to) : 0.0f;
+        a.load_to = decide && !(last && from == 0.0f) ? (last ? va::kNoLimit : to) : 0.0f;
         a.part = a.split ? va::SPLIT_NEVER : va::SPLIT_NONE;
         VA_CUDA(h, launch(h, t.fn, grid, block, &a, s));
         if (!two_level && (last || !decide)) { // what va_get_launch reports
@@ -698,7 +698,7 @@ va_status launch_teams(va_handle *h, int sweep, Params &a, cudaStream_t s, bool 
         from = to;
     }
     a.load_from = from;
-    a.load_to = decide ? 3.0e38f : 0.0f;
+    a.load_to = decide ? va::kNoLimit : 0.0f;
     a.rest_sms = rest;
     a.part = a.split ? va::SPLIT_REST : va::SPLIT_NONE;
     return VA_OK;
@@ -802,7 +802,7 @@ va_status enqueue_forward(va_handle *h, const double *y0, const double *params, 
         h->fwd_grid = grid_for(h, fn, h->fwd_block, a.B);
     if (h->order_fwd) {
         const int *valid = h->inst_work + a.B;
-        va::OrderArgs o{a.B, nullptr, t0, t1, h->inst_work, valid, h->order_work, h->order_fwd, nullptr};
+        va::OrderArgs o{a.B, nullptr, t0, t1, h->inst_work, valid, h->order_work, h->order_fwd};
         split_rule(h, o);
         VA_CUDA(h, va::enqueue_order(o, s));
         a.order = h->order_fwd;
@@ -850,7 +850,8 @@ va_status enqueue_backward(va_handle *h, const double *params, const double *lam
         // +3%); the lane groups sort by their own step counts (GLV-10: the
         // reused order made the backward 11% slower)
         const int *reuse = h->ks->tpi == 1 ? h->order_fwd : nullptr;
-        va::OrderArgs o{a.B, h->inst_T, nullptr, nullptr, nullptr, nullptr, h->order_work, h->order_bwd, reuse};
+        va::OrderArgs o{a.B, h->inst_T, nullptr, nullptr, nullptr, nullptr, h->order_work, h->order_bwd, reuse,
+                        h->inst_work, 4.0f * 128.0f * (float)h->sm_count};
         split_rule(h, o);
         VA_CUDA(h, va::enqueue_order(o, s));
         a.order = h->order_bwd;

@@ -24,6 +24,7 @@
 #include <type_traits>
 
 #include "va_dword.cuh"
+#include "va_order.h"
 #include "va_step64.cuh"
 #include "va_stepfactor.cuh"
 #include "va_tableau.cuh"
@@ -51,6 +52,11 @@ struct Control {
     unsigned int pool_fail; // set when the pool ran out
     unsigned int pow_undecided; // step factors whose rounding test failed (cr_step_pow)
     unsigned int fwd_long, adj_long; // next of the longest instances (SPLIT_LONG)
+    // a forward team sweep's finished instances (note_finished; a sample of them):
+    // the attempts of the longest and of all
+    unsigned int longest;
+    unsigned int handed; // it left the rest of the queue to the last sweep
+    unsigned long long attempts;
 };
 
 // Checkpoint pool: chunks of `chunk_len` records of `rs` doubles.
@@ -84,8 +90,8 @@ struct FwdParams {
                      // two-level backward re-forms t_0 + n dt from them; may be null)
     int stride;      // store every stride-th accepted step (and the last); 1 = all
     const int *order;// [B] work order (may be null = index order)
-    int *inst_work;  // [B] attempts (accepted + rejected) of this sweep, the next
-                     // sweep's length estimate (may be null)
+    int *inst_work;  // [B] attempts (accepted + rejected) of this sweep (0 before an
+                     // instance is finished), the next sweep's length estimate (may be null)
     int *work_valid; // set to 1 once inst_work holds a sweep's counts (may be null)
     Pool pool;
     Control *ctl;
@@ -99,11 +105,37 @@ struct FwdParams {
 // Parts of a split batch: no split for this sweep, the longest instances alone,
 // none of a split batch, the others (all of a batch that is not split).
 enum : int { SPLIT_NONE = 0, SPLIT_LONG = 1, SPLIT_NEVER = 2, SPLIT_REST = 3 };
+constexpr float kNoLimit = 3.0e38f; // load_to of the last sweep of a launch
+constexpr int kLooks = 2000;        // of a resting warp (resting), ~0.1 s
 template <class Params>
 __device__ __forceinline__ int split_of(const Params &a)
 {
     return a.part != SPLIT_NONE ? *a.split : 0;
 }
+// Which instances a team sweep counts: all of a small batch, one in 16 of a large
+// one.
+__device__ __forceinline__ int sampled(int B) { return B >= 32768 ? 16 : 1; }
+__device__ __forceinline__ void note_finished(const FwdParams &a, int b, int attempts)
+{
+    if (a.load && b % sampled(a.B) == 0) {
+        atomicMax(&a.ctl->longest, (unsigned int)attempts);
+        atomicAdd(&a.ctl->attempts, (unsigned long long)attempts);
+    }
+}
+// The load of the instances that a team sweep has finished: the batch's is no
+// less, however wrong the lengths were that the order went by.
+__device__ __forceinline__ float load_seen(const FwdParams &a)
+{
+    const volatile Control *c = a.ctl;
+    const unsigned int m = c->longest;
+    return m ? (float)c->attempts * (float)sampled(a.B) / (float)m : 0.0f;
+}
+// Whether a team sweep gave up on the batch (gives_up; forward sweeps alone:
+// the backward knows the lengths).
+__device__ __forceinline__ bool handed_over(const FwdParams &a) { return *(volatile unsigned int *)&a.ctl->handed != 0; }
+struct AdjParams;
+__device__ __forceinline__ bool handed_over(const AdjParams &) { return false; }
+
 // Whether another sweep of the same launch takes this batch.
 template <class Params>
 __device__ __forceinline__ bool gated_off(const Params &a)
@@ -113,17 +145,74 @@ __device__ __forceinline__ bool gated_off(const Params &a)
         return n == 0;
     if (n > 0)
         return a.part == SPLIT_NEVER;
-    return a.load && a.load_to > 0.0f && !(*a.load > a.load_from && *a.load <= a.load_to);
+    if (!(a.load && a.load_to > 0.0f) || (*a.load > a.load_from && *a.load <= a.load_to))
+        return false;
+    return !(a.load_to >= kNoLimit && handed_over(a));
+}
+// Whether a forward team sweep takes no more instances and leaves the queue to
+// the last sweep of the launch.  It was chosen by the load that the lengths of the
+// call before (or the horizons) gave; on other inputs the load may be many times
+// that, and wide teams then take several times as long as one lane each
+// (20,000 Van der Pol instances after a batch with one long one: 15.2 ms, 5.0 with
+// the right choice, 9.8 so).  What is finished shows it: a quarter more than the
+// load this sweep is for.
+__device__ __forceinline__ bool gives_up(const FwdParams &a)
+{
+    if (!a.load || !(a.load_to > 0.0f) || a.load_to >= kNoLimit || a.part == SPLIT_LONG)
+        return false;
+    if (handed_over(a))
+        return true;
+    if (!(load_seen(a) > 1.25f * a.load_to))
+        return false;
+    *(volatile unsigned int *)&a.ctl->handed = 1;
+    return true;
 }
 // Whether this warp stays idle: beyond the warps per quadrant that are useful
 // beside the longest instance.
-template <class Params>
-__device__ __forceinline__ bool resting(const Params &a)
+__device__ __forceinline__ bool beyond_useful(int sms, float load)
 {
-    if (!a.load || !a.rest_sms)
+    const float warps = fmaxf(1.0f, ceilf(load / (1.25f * 128.0f * (float)sms)));
+    return (float)(blockIdx.x / (unsigned)sms * (blockDim.x / 32) + threadIdx.x / 32) >= 4.0f * warps;
+}
+__device__ __forceinline__ bool resting(const AdjParams &a);
+// A forward sweep's load is that of other inputs, perhaps: a warp that would be
+// useful if all instances were as long as the longest looks again every 50 us
+// until the queue is empty, and comes in when a sample of the batch shows the load
+// for it (inst_work is 0 until an instance is finished).  Double-word Van der Pol
+// after a batch with one long instance, 262,144: forward 7.0 ms with the idle
+// warps gone for good, 4.0 with all of them at work from the start, 5.0 so.  A
+// function of its own, and no counting by the warps at work: an atomic or a flag
+// in the loop that takes the next instance cost the one-lane sweeps 3 to 8%.
+static __device__ __noinline__ bool never_useful(const volatile unsigned int *next, const volatile int *work, int B,
+                                                 int skip, int sms)
+{
+    constexpr int kSample = 512;
+    const int every = B / kSample;
+#pragma unroll 1
+    for (int look = 0; look < kLooks; look++) {
+        __nanosleep(50000);
+        if (*next + (unsigned int)skip >= (unsigned int)B)
+            return true;
+        int sum = 0, top = 0;
+#pragma unroll 1
+        for (int k = threadIdx.x & 31; k < kSample; k += 32) {
+            const int n = work[k * every];
+            sum += n;
+            top = n > top ? n : top;
+        }
+        sum = __reduce_add_sync(0xffffffffu, sum);
+        top = __reduce_max_sync(0xffffffffu, top);
+        if (top > 0 && !beyond_useful(sms, (float)sum * (float)every / (float)top))
+            return false;
+    }
+    return true;
+}
+__device__ __forceinline__ bool resting(const FwdParams &a)
+{
+    if (!a.load || !a.rest_sms || !beyond_useful(a.rest_sms, *a.load))
         return false;
-    const float warps = fmaxf(1.0f, ceilf(*a.load / (1.25f * 128.0f * (float)a.rest_sms)));
-    return (float)(blockIdx.x / (unsigned)a.rest_sms * (blockDim.x / 32) + threadIdx.x / 32) >= 4.0f * warps;
+    return beyond_useful(a.rest_sms, (float)a.B) ||
+           never_useful(&a.ctl->fwd_next, a.inst_work, a.B, split_of(a), a.rest_sms);
 }
 
 // Record an instance's attempt count for the next forward sweep's order.
@@ -170,6 +259,10 @@ struct AdjParams {
     const int *split; // as FwdParams
     int part;
 };
+__device__ __forceinline__ bool resting(const AdjParams &a)
+{
+    return a.load && a.rest_sms && beyond_useful(a.rest_sms, *a.load);
+}
 
 __host__ __device__ constexpr int record_doubles(int n) { return (2 + n + 1) & ~1; }
 

@@ -104,6 +104,7 @@ extern "C" va_status va_gradient_noalloc(int32_t model, int32_t tableau, int32_t
     // chunk_prev | checkpoint chunks.  Every instance needs at least one
     // chunk; a batch whose metadata and first chunks do not fit is rejected.
     const size_t B = (size_t)batch;
+    static_assert(sizeof(va::Control) <= 256, "the control block's place in the array");
     const size_t off_T = 256, off_last = off_T + align256(B * 4), off_st = off_last + align256(B * 4);
     const size_t off_prev = off_st + align256(B * 4);
     if (off_prev >= kScratchBytes)

@@ -17,6 +17,13 @@
 // attempts, nearly the same ranking as this sweep's accepted steps): no
 // second sort, and the backward then visits the checkpoint chunks in the
 // order the forward allocated them (the caller decides; one-thread models).
+// Not when the inputs are others than the call's before: when the lengths of
+// more than 1 in 32 instances moved by more than an eighth, or the longest did,
+// the backward sorts by its own step counts, and its load and its longest part
+// are this batch's too.  Where the load fills four warps per quadrant a lane
+// carries several instances, the order matters less than the chunks' locality, and
+// the forward's order stays (262,144 double-word Van der Pol instances on new
+// inputs: backward 3.52 ms with it, 3.64 sorted; 65,536: 1.12 with it, 0.72 sorted).
 //
 // The sort also leaves the batch's load, sum(length) / max(length), by which
 // the one-thread sweeps choose on the device how many warps they keep busy
@@ -56,17 +63,45 @@ __device__ __forceinline__ int horizon_bucket(double h)
 
 __device__ __forceinline__ int count_bucket(int n) { return n < kBuckets ? (n < 0 ? 0 : n) : kBuckets - 1; }
 
-// work[2 kBuckets]: 1 when the last forward order came from step counts
-constexpr int kCountedFlag = 2 * kBuckets;
+// work[0 ..): the buckets' counts, then, zeroed with them, how many instances
+// moved and the longest of now (order_moved)
+constexpr int kMovedSlot = kBuckets, kLongestSlot = kBuckets + 1, kZeroed = kBuckets + 2;
+// work[kOffsets ..): the buckets' offsets
+constexpr int kOffsets = kZeroed;
 
-// work[2 kBuckets + 1]: the load (a float)
+// 1 when the last forward order came from step counts
+constexpr int kCountedFlag = kOffsets + kBuckets;
+
+// the load (a float)
 constexpr int kLoadSlot = kCountedFlag + 1;
 
-// work[2 kBuckets + 2]: the size of the longest part
+// the size of the longest part
 constexpr int kSplitSlot = kLoadSlot + 1;
 
-// the backward reuses the forward's order when that one was count-based
-__device__ __forceinline__ bool reusing(const OrderArgs &a) { return a.reuse && a.work[kCountedFlag] == 1; }
+// the longest length by which the last forward order went, and all of them
+// (B ints), when it came from step counts
+constexpr int kTopSlot = kSplitSlot + 1, kTaken = kTopSlot + 1;
+
+// the backward reuses the forward's order when that one was count-based and the
+// counts were this batch's, all but a few
+__device__ __forceinline__ bool reusing(const OrderArgs &a, int moved, int longest)
+{
+    return a.reuse && a.work[kCountedFlag] == 1 && moved <= a.B / 32 &&
+           !length_moved(a.work[kTopSlot], count_bucket(longest));
+}
+__device__ __forceinline__ bool reusing(const OrderArgs &a)
+{
+    return reusing(a, a.work[kMovedSlot], a.work[kLongestSlot]);
+}
+// For the order of a forward sweep: what it takes instance b's length to be, out
+// of the place where the sweep puts it when it is known.  After the last key_of.
+__device__ __forceinline__ void keep_length(const OrderArgs &a, int b)
+{
+    if (!a.steps && a.prev_work) {
+        a.work[kTaken + b] = a.prev_work[b];
+        a.prev_work[b] = 0;
+    }
+}
 
 __device__ __forceinline__ int key_of(const OrderArgs &a, int b)
 {
@@ -81,6 +116,36 @@ __device__ __forceinline__ int key_of(const OrderArgs &a, int b)
 __device__ __forceinline__ float bucket_length(bool counted, int k)
 {
     return counted ? (float)k : exp2f((float)k * (1.0f / 64.0f) - 32.0f);
+}
+
+// How many instances moved and the longest of now, before the order of a
+// backward sweep: two loads an instance, and a launch of ~2 us.  One atomic a
+// block: one a warp (262,144 instances: 8,192 on one address) took 20 us.
+__global__ void __launch_bounds__(1024) order_moved(OrderArgs a)
+{
+    __shared__ int block_moved, block_top;
+    if (a.work[kCountedFlag] != 1)
+        return;
+    if (threadIdx.x == 0)
+        block_moved = block_top = 0;
+    __syncthreads();
+    int moved = 0, top = 0;
+    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < a.B; b += gridDim.x * blockDim.x) {
+        const int n = a.now[b];
+        moved += length_moved(a.work[kTaken + b], n) ? 1 : 0;
+        top = n > top ? n : top;
+    }
+    moved = __reduce_add_sync(0xffffffffu, moved);
+    top = __reduce_max_sync(0xffffffffu, top);
+    if ((threadIdx.x & 31) == 0) {
+        atomicAdd(&block_moved, moved);
+        atomicMax(&block_top, top);
+    }
+    __syncthreads();
+    if (threadIdx.x == 0) {
+        atomicAdd(&a.work[kMovedSlot], block_moved);
+        atomicMax(&a.work[kLongestSlot], block_top);
+    }
 }
 
 __global__ void order_hist(OrderArgs a)
@@ -153,8 +218,10 @@ __device__ __forceinline__ int scan_from_top(const OrderArgs &a, const int (&v)[
             // at most one per instance, at least one instance's (a batch of length 0 too)
             const float load = m1 > 0.0f ? s1 / m1 : 1.0f;
             a.work[kLoadSlot] = __float_as_int(fminf(fmaxf(load, 1.0f), (float)a.B));
-            if (!a.steps) // a forward order: say whether it came from counts
+            if (!a.steps) { // a forward order: say whether it came from counts
                 a.work[kCountedFlag] = prev ? 1 : 0;
+                a.work[kTopSlot] = prev ? (int)m1 : 0;
+            }
         }
     }
     __syncthreads();
@@ -224,7 +291,7 @@ __global__ void __launch_bounds__(1024) order_scan(OrderArgs a)
     int run = above;
 #pragma unroll
     for (int j = 0; j < 4; j++) {
-        a.work[kBuckets + (kBuckets - 1 - (t * 4 + j))] = run;
+        a.work[kOffsets + (kBuckets - 1 - (t * 4 + j))] = run;
         run += v[j];
     }
     find_split(a, v, above);
@@ -236,18 +303,32 @@ __global__ void __launch_bounds__(1024) order_scan(OrderArgs a)
 static_assert(kSmallBatch == 4 * 1024, "four keys a thread");
 __global__ void __launch_bounds__(1024) order_small(OrderArgs a)
 {
-    __shared__ int cnt[kBuckets];
+    __shared__ int cnt[kBuckets], top;
     const int t = threadIdx.x;
-    if (reusing(a)) {
-        for (int b = t; b < a.B; b += 1024)
-            a.order[b] = a.reuse[b];
-        return;
+    if (a.reuse && a.work[kCountedFlag] == 1) { // the same for every thread
+        if (t == 0)
+            top = 0;
+        __syncthreads();
+        int moved = 0;
+        for (int i = 0; i < 4; i++) {
+            const int b = t + 1024 * i, n = b < a.B ? a.now[b] : 0;
+            moved += __syncthreads_count(b < a.B && length_moved(a.work[kTaken + b], n));
+            atomicMax(&top, n);
+        }
+        __syncthreads();
+        if (reusing(a, moved, top)) {
+            for (int b = t; b < a.B; b += 1024)
+                a.order[b] = a.reuse[b];
+            return;
+        }
     }
     int key[4];
 #pragma unroll
     for (int i = 0; i < 4; i++) {
         cnt[t + 1024 * i] = 0;
         key[i] = t + 1024 * i < a.B ? key_of(a, t + 1024 * i) : -1;
+        if (key[i] >= 0)
+            keep_length(a, t + 1024 * i);
     }
     __syncthreads();
 #pragma unroll
@@ -283,7 +364,8 @@ __global__ void __launch_bounds__(1024) order_scatter(OrderArgs a)
     __shared__ int cnt[kBuckets];
     const int per = (a.B + gridDim.x - 1) / gridDim.x;
     const int lo = blockIdx.x * per, hi = min(a.B, lo + per);
-    if (reusing(a)) {
+    if (reusing(a) ||
+        (a.reuse && a.work[kCountedFlag] == 1 && __int_as_float(a.work[kLoadSlot]) > a.keep_from)) {
         for (int b = lo + threadIdx.x; b < hi; b += blockDim.x)
             a.order[b] = a.reuse[b];
         return;
@@ -296,15 +378,17 @@ __global__ void __launch_bounds__(1024) order_scatter(OrderArgs a)
     __syncthreads();
     for (int i = threadIdx.x; i < kBuckets; i += blockDim.x)
         if (cnt[i])
-            cnt[i] = atomicAdd(&a.work[kBuckets + i], cnt[i]); // this block's slice of bucket i
+            cnt[i] = atomicAdd(&a.work[kOffsets + i], cnt[i]); // this block's slice of bucket i
     __syncthreads();
-    for (int b = lo + threadIdx.x; b < hi; b += blockDim.x)
+    for (int b = lo + threadIdx.x; b < hi; b += blockDim.x) {
         a.order[atomicAdd(&cnt[key_of(a, b)], 1)] = b;
+        keep_length(a, b);
+    }
 }
 
 } // namespace
 
-size_t order_work_ints() { return 2 * kBuckets + 3; }
+size_t order_work_ints(int B) { return kTaken + (size_t)B; }
 const float *order_load(const int *work) { return reinterpret_cast<const float *>(work + kLoadSlot); }
 
 const int *order_split(const int *work) { return work + kSplitSlot; }
@@ -315,13 +399,15 @@ cudaError_t enqueue_order(const OrderArgs &a, cudaStream_t s)
         order_small<<<1, 1024, 0, s>>>(a);
         return cudaGetLastError();
     }
-    cudaError_t e = cudaMemsetAsync(a.work, 0, sizeof(int) * kBuckets, s);
+    cudaError_t e = cudaMemsetAsync(a.work, 0, sizeof(int) * kZeroed, s);
     if (e != cudaSuccess)
         return e;
     const int grid = (a.B + 255) / 256 < 1024 ? (a.B + 255) / 256 : 1024;
+    const int sgrid = (a.B + 1023) / 1024 < 256 ? (a.B + 1023) / 1024 : 256;
+    if (a.reuse)
+        order_moved<<<sgrid, 1024, 0, s>>>(a);
     order_hist<<<grid, 256, 0, s>>>(a);
     order_scan<<<1, 1024, 0, s>>>(a);
-    const int sgrid = (a.B + 1023) / 1024 < 256 ? (a.B + 1023) / 1024 : 256;
     order_scatter<<<sgrid, 1024, 0, s>>>(a);
     return cudaGetLastError();
 }

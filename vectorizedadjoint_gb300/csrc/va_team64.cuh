@@ -400,6 +400,8 @@ __global__ void __launch_bounds__(256) forward_team_kernel(FwdParams a)
 
     const int limit = a.part == SPLIT_LONG ? split_of(a) : a.B;
     auto fetch = [&]() -> bool {
+        if (__shfl_sync(tf.team.mask, first && gives_up(a) ? 1 : 0, tf.team.base))
+            return false;
         b = take(a.part == SPLIT_LONG ? &a.ctl->fwd_long : &a.ctl->fwd_next);
         if (b >= limit)
             return false;
@@ -477,6 +479,7 @@ __global__ void __launch_bounds__(256) forward_team_kernel(FwdParams a)
         a.inst_last[b] = chunk;
         a.inst_status[b] = status;
         note_work(a, b, count + rej);
+        note_finished(a, b, count + rej);
         if (a.inst_t1)
             a.inst_t1[b] = t1;
         if (a.n_acc_out)

@@ -160,6 +160,8 @@ __global__ void __launch_bounds__(256) forward_glv_warp_kernel(FwdParams a)
         return y * (p[0] + s);
     };
     auto fetch = [&]() -> bool {
+        if (__shfl_sync(mask, first && gives_up(a) ? 1 : 0, 0))
+            return false;
         b = wp.take(&a.ctl->fwd_next);
         if (b >= a.B)
             return false;
@@ -233,6 +235,7 @@ __global__ void __launch_bounds__(256) forward_glv_warp_kernel(FwdParams a)
             if (a.inst_t1)
                 a.inst_t1[b] = t1;
             note_work(a, b, count + rej);
+            note_finished(a, b, count + rej);
             if (a.n_acc_out)
                 a.n_acc_out[b] = count;
             if (a.n_rej_out)
