@@ -400,7 +400,7 @@ __global__ void __launch_bounds__(256) forward_team_kernel(FwdParams a)
 
     const int limit = a.part == SPLIT_LONG ? split_of(a) : a.B;
     auto fetch = [&]() -> bool {
-        if (__shfl_sync(tf.team.mask, first && gives_up(a) ? 1 : 0, tf.team.base))
+        if (__shfl_sync(tf.team.mask, first && gives_up(a, G) ? 1 : 0, tf.team.base))
             return false;
         b = take(a.part == SPLIT_LONG ? &a.ctl->fwd_long : &a.ctl->fwd_next);
         if (b >= limit)

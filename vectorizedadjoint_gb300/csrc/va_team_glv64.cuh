@@ -160,7 +160,7 @@ __global__ void __launch_bounds__(256) forward_glv_warp_kernel(FwdParams a)
         return y * (p[0] + s);
     };
     auto fetch = [&]() -> bool {
-        if (__shfl_sync(mask, first && gives_up(a) ? 1 : 0, 0))
+        if (__shfl_sync(mask, first && gives_up(a, 32) ? 1 : 0, 0))
             return false;
         b = wp.take(&a.ctl->fwd_next);
         if (b >= a.B)
