@@ -101,3 +101,26 @@ def test_bundle_width_axis(cuda, cache_file, precision):
             g, g0 = np.concatenate([o["dy0"], o["dp"]], 1), np.concatenate([base["dy0"], base["dp"]], 1)
             assert np.abs(g - g0).max() <= 1e-9 * np.abs(g0).max()
         assert np.abs(o["dA"] - base["dA"]).max() <= 1e-8 * np.abs(base["dA"]).max()
+
+
+def test_shapes_of_other_kernels_are_not_taken(cuda, cache_file):
+    """A stored line without the kernels' revision, as files of before have, is passed over: the handle tunes anew."""
+    B = 4500
+    w = W.make("vdpb", batch=B)
+    c = w["cfg"]
+    args = (dev(w["y0"]), dev(w["params"]), dev(w["t0"]), dev(w["t1"]))
+
+    def tune():
+        s = Solver(c["model"], c["n"], c["npar"], B, tableau=c["tableau"], precision="mixed_dw", atol=c["tol"],
+                   rtol=c["tol"])
+        launch = s.autotune(c["cost"], *args)
+        s.close()
+        return launch
+
+    tune()
+    key = cache_file.read_text().splitlines()[-1].split("\t")[0]
+    old = "|".join(key.split("|")[:12])  # GPU .. batch size, as written before
+    cache_file.write_text(f"{old}\t32 1 32 1 0\n")
+    launch = tune()
+    assert launch["fwd_block"] != 32 and launch["bwd_block"] != 32
+    assert len(cache_file.read_text().splitlines()) == 2

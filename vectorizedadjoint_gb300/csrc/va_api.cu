@@ -1112,7 +1112,9 @@ va_status autotune_sweep(va_handle *h, int32_t cost, const double *y0, const dou
 // $HOME/.cache/vectorizedadjoint_gb300/autotune.tsv.  The key: GPU name and
 // SM count, model (and a model compiled outside the library's name), n,
 // npar, nout, tableau, precision, stage records, checkpoint stride, step
-// factor and the batch size's power of two.  The last matching line wins.
+// factor and the batch size's power of two, then kSweepRevision and how many
+// blocks of 128 threads of each sweep an SM holds: a shape measured for other
+// kernels is not taken.  The last matching line wins.
 
 std::string cache_path()
 {
@@ -1132,11 +1134,13 @@ std::string cache_key(const va_handle *h)
     int lb = 0;
     while ((1L << (lb + 1)) <= (long)h->prob.batch)
         lb++;
+    const int occ_f = h->bks ? 0 : occupancy_of(h, fwd_kernel(h), 128);
+    const int occ_b = h->bks ? 0 : occupancy_of(h, bwd_kernel(h), 128);
     char buf[512];
-    std::snprintf(buf, sizeof(buf), "%s|%d|%d%s%s|%d|%d|%d|%d|%d|%d|%d|%d|%d", prop.name, h->sm_count,
+    std::snprintf(buf, sizeof(buf), "%s|%d|%d%s%s|%d|%d|%d|%d|%d|%d|%d|%d|%d|r%d|%d|%d", prop.name, h->sm_count,
                   h->prob.model, h->user ? ":" : "", h->user && h->user->name ? h->user->name : "", h->prob.n,
                   h->prob.npar, h->prob.nout, h->opt.tableau, h->opt.precision, (int)h->stages_on, h->stride,
-                  h->opt.step_pow, lb);
+                  h->opt.step_pow, lb, va::kSweepRevision, occ_f, occ_b);
     for (char *c = buf; *c; c++)
         if (*c == '\t' || *c == '\n')
             *c = ' ';

@@ -14,6 +14,10 @@ namespace va {
 // 3 fixed-step runge_kutta4, 4 fixed-step euler
 constexpr int kTableaux = 5;
 
+// Of the sweep kernels, for shapes tuned and kept on disk: raised when their
+// times by launch shape change.
+constexpr int kSweepRevision = 2;
+
 struct KernelSet {
     int N, P;          // state and parameter counts (0 = runtime n)
     int tpi;           // threads that carry one instance
