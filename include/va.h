@@ -284,10 +284,11 @@ VA_API va_status va_forward_frozen(va_handle *h, int32_t count, int32_t times_st
 /* Picks the launch shape by timing candidate runs of both sweeps on the given
  * inputs (device pointers) and keeps it in the handle: for the one-thread
  * and lane-group models the block size and resident blocks per SM of each
- * sweep, for the shared-matrix model the bundle width (instances per CTA:
- * 2 or 4).  Runs forward+backward several times per candidate.  The choice
+ * sweep, by the time of both together (the default shape stays unless another
+ * is 1% faster), for the shared-matrix model the bundle width (instances per
+ * CTA: 2 or 4).  Runs forward+backward several times per candidate.  The choice
  * is also kept on disk, one line per problem (GPU, model, sizes, tableau,
- * precision, record layout, batch size's power of two), in the file named
+ * precision, record layout, batch size's power of two, kernels), in the file named
  * by the environment variable VA_AUTOTUNE_CACHE ("" or "off": none), else
  * $XDG_CACHE_HOME/vectorizedadjoint_gb300/autotune.tsv or
  * $HOME/.cache/vectorizedadjoint_gb300/autotune.tsv; a later call for the

@@ -26,6 +26,7 @@
 #include "va_order.h"
 #include "va_registry.h"
 #include "va_replay.cuh"
+#include "va_tune.h"
 
 namespace {
 
@@ -66,7 +67,10 @@ struct va_handle {
     cudaStream_t side = nullptr;
     cudaEvent_t fork = nullptr, join = nullptr;
     int bps = 0; // resident blocks per SM of the default launch shape (0: the occupancy limit)
-    bool default_shape = true; // neither given by the caller nor tuned
+    // the sweep runs in the default launch shape, neither given by the caller nor
+    // tuned, and the block size of that
+    bool default_fwd = true, default_bwd = true;
+    int default_block = 128;
     int N = 0, P = 0;
     int RS = 0; // doubles per checkpoint record at the current stride (record_layout)
     bool stages_on = true; // opt.stage_records, cleared by the automatic checkpoint ladder
@@ -640,9 +644,9 @@ cudaError_t launch(const va_handle *h, const void *fn, int grid, int block, void
 // SMs for the resting rule of the sweeps of one lane per instance: their
 // default launch shape only (one that the caller gave or the autotuner
 // measured stands)
-int rest_sms(const va_handle *h)
+int rest_sms(const va_handle *h, bool default_shape)
 {
-    return h->ks && h->ks->tpi == 1 && h->default_shape ? h->sm_count : 0;
+    return h->ks && h->ks->tpi == 1 && default_shape ? h->sm_count : 0;
 }
 
 // Launches the sweep's teams.  By the batch's load, decided on the device:
@@ -807,7 +811,7 @@ va_status enqueue_forward(va_handle *h, const double *y0, const double *params, 
         VA_CUDA(h, va::enqueue_order(o, s));
         a.order = h->order_fwd;
         a.load = va::order_load(h->order_work);
-        a.rest_sms = rest_sms(h);
+        a.rest_sms = rest_sms(h, h->default_fwd);
         a.inst_work = h->inst_work;
         a.work_valid = h->inst_work + a.B;
     }
@@ -856,7 +860,7 @@ va_status enqueue_backward(va_handle *h, const double *params, const double *lam
         VA_CUDA(h, va::enqueue_order(o, s));
         a.order = h->order_bwd;
         a.load = va::order_load(h->order_work);
-        a.rest_sms = rest_sms(h);
+        a.rest_sms = rest_sms(h, h->default_bwd);
     }
     if (h->bks && h->stride > 1) {
         // two-level: segments re-run from the strided checkpoints, in bundles
@@ -992,7 +996,8 @@ struct AutotuneEvents {
 };
 
 // A tuned launch shape: block size and resident blocks per SM of each sweep
-// (one-thread and lane-group models) and the bundle width (shared matrix).
+// (one-thread and lane-group models; 0: the default) and the bundle width (shared
+// matrix).
 struct TunedShape {
     int fb = 0, fbps = 0, bb = 0, bbps = 0, alt = 0;
 };
@@ -1014,11 +1019,13 @@ void apply_shape(va_handle *h, const TunedShape &t)
     }
     const void *ffn = fwd_kernel(h);
     const void *bfn = bwd_kernel(h);
-    h->default_shape = false;
-    h->fwd_block = t.fb;
-    h->fwd_grid = grid_of(h, ffn, t.fb, t.fbps);
-    h->bwd_block = t.bb;
-    h->bwd_grid = grid_of(h, bfn, t.bb, t.bbps);
+    const bool given = h->opt.block_size > 0 || h->opt.blocks_per_sm > 0;
+    h->default_fwd = !given && t.fb == 0;
+    h->fwd_block = t.fb > 0 ? t.fb : h->default_block;
+    h->fwd_grid = t.fb > 0 ? grid_of(h, ffn, t.fb, t.fbps) : grid_for(h, ffn, h->fwd_block, h->prob.batch);
+    h->default_bwd = !given && t.bb == 0;
+    h->bwd_block = t.bb > 0 ? t.bb : h->default_block;
+    h->bwd_grid = t.bb > 0 ? grid_of(h, bfn, t.bb, t.bbps) : grid_for(h, bfn, h->bwd_block, h->prob.batch);
 }
 
 // Forward and backward once untimed, then the best of two timed runs.
@@ -1050,8 +1057,8 @@ va_status time_sweeps(va_handle *h, int32_t cost, const double *y0, const double
 }
 
 // Times the candidates and leaves the best shape in `best`.  One-thread and
-// lane-group models: every (block size, resident blocks per SM) of each
-// sweep; shared-matrix bundles: both compiled bundle widths.
+// lane-group models: the default shape and every (block size, resident blocks per
+// SM); shared-matrix bundles: both compiled bundle widths.
 va_status autotune_sweep(va_handle *h, int32_t cost, const double *y0, const double *params,
                          const double *t0, const double *t1, cudaStream_t s, AutotuneEvents &ev, TunedShape &best)
 {
@@ -1074,34 +1081,27 @@ va_status autotune_sweep(va_handle *h, int32_t cost, const double *y0, const dou
     }
     const void *ffn = fwd_kernel(h);
     const void *bfn = bwd_kernel(h);
-    float best_f = 1e30f, best_b = 1e30f;
-    const int blocks[] = {64, 128, 256};
-    for (int blk : blocks) {
-        const int occf = occupancy_of(h, ffn, blk), occb = occupancy_of(h, bfn, blk);
+    std::vector<va::Shape> shapes;
+    for (int blk : {64, 128, 256}) {
         // every resident-block count: the best differs between the sweeps and
         // between workloads (stage-record traffic favours fewer warps in the
         // backward, issue rate more in the forward)
-        const int maxocc = std::max(1, std::max(occf, occb));
-        for (int bps = 1; bps <= maxocc; bps++) {
-            TunedShape cand{blk, bps, blk, bps, 0};
-            apply_shape(h, cand);
-            float tf, tb;
-            const va_status st = time_sweeps(h, cost, y0, params, t0, t1, s, ev, tf, tb);
-            if (st != VA_OK)
-                return st;
-            if (tf < best_f) {
-                best_f = tf;
-                best.fb = blk;
-                best.fbps = bps;
-            }
-            if (tb < best_b) {
-                best_b = tb;
-                best.bb = blk;
-                best.bbps = bps;
-            }
-        }
+        const int occ = std::max({1, occupancy_of(h, ffn, blk), occupancy_of(h, bfn, blk)});
+        for (int bps = 1; bps <= occ; bps++)
+            shapes.push_back({blk, bps});
     }
-    return VA_OK;
+    va_status st = VA_OK;
+    va::ShapePair pair;
+    va::tune_pair(
+        shapes,
+        [&](va::Shape f, va::Shape b, float &tf, float &tb) {
+            apply_shape(h, TunedShape{f.block, f.bps, b.block, b.bps, 0});
+            st = time_sweeps(h, cost, y0, params, t0, t1, s, ev, tf, tb);
+            return st == VA_OK;
+        },
+        pair);
+    best = TunedShape{pair.fwd.block, pair.fwd.bps, pair.bwd.block, pair.bwd.bps, 0};
+    return st;
 }
 
 // ------------------------------------------------------ autotune cache
@@ -1336,7 +1336,7 @@ va_status create_handle(const va_problem *prob, const va_options *opt, const va:
     h->P = P;
     h->chunk_len = o.chunk_len > 0 ? o.chunk_len : 64;
     record_layout(h);
-    h->default_shape = o.block_size <= 0 && o.blocks_per_sm <= 0;
+    h->default_fwd = h->default_bwd = o.block_size <= 0 && o.blocks_per_sm <= 0;
     if (o.block_size > 0) {
         h->fwd_block = h->bwd_block = o.block_size;
     }
@@ -1348,6 +1348,7 @@ va_status create_handle(const va_problem *prob, const va_options *opt, const va:
         return VA_CUDA_ERROR;
     }
     fp64_path(h);
+    h->default_block = h->fwd_block;
     if (split_path(h) != VA_OK) {
         va_destroy(h);
         return VA_CUDA_ERROR;
@@ -1861,7 +1862,8 @@ va_status va_autotune(va_handle *h, int32_t cost, const double *y0, const double
         return st;
     const std::string key = cache_key(h);
     TunedShape t;
-    if (cache_lookup(key, t) && (h->bks || (t.fb > 0 && t.bb > 0 && t.fbps > 0 && t.bbps > 0))) {
+    auto shape = [](int block, int bps) { return block == 0 ? bps == 0 : block > 0 && bps > 0; };
+    if (cache_lookup(key, t) && (h->bks || (shape(t.fb, t.fbps) && shape(t.bb, t.bbps)))) {
         apply_shape(h, t);
         drop_graph(h);
         return VA_OK;
@@ -1869,7 +1871,7 @@ va_status va_autotune(va_handle *h, int32_t cost, const double *y0, const double
     cudaStream_t s = (cudaStream_t)stream;
     // the launch shape before tuning, restored if a candidate run fails
     const int prev[4] = {h->fwd_block, h->fwd_grid, h->bwd_block, h->bwd_grid};
-    const bool prev_alt = h->bundle_alt, prev_default = h->default_shape;
+    const bool prev_alt = h->bundle_alt, prev_default[2] = {h->default_fwd, h->default_bwd};
     AutotuneEvents ev;
     st = autotune_sweep(h, cost, y0, params, t0, t1, s, ev, t);
     if (st != VA_OK) {
@@ -1877,7 +1879,8 @@ va_status va_autotune(va_handle *h, int32_t cost, const double *y0, const double
         h->fwd_grid = prev[1];
         h->bwd_block = prev[2];
         h->bwd_grid = prev[3];
-        h->default_shape = prev_default;
+        h->default_fwd = prev_default[0];
+        h->default_bwd = prev_default[1];
         h->bundle_alt = prev_alt;
         drop_graph(h);
         return st;
