@@ -124,3 +124,57 @@ def test_shapes_of_other_kernels_are_not_taken(cuda, cache_file):
     launch = tune()
     assert launch["fwd_block"] != 32 and launch["bwd_block"] != 32
     assert len(cache_file.read_text().splitlines()) == 2
+
+
+def vdp(B, seed, uneven=False):
+    rng = np.random.default_rng(seed)
+    t1 = np.full(B, 20.0)
+    if uneven:
+        t1[:] = 0.02
+        t1[B // 2] = 40.0
+    return [dev(v) for v in (rng.uniform(-2, 2, (B, 2)), 10 ** rng.uniform(-1, 1, (B, 1)), np.zeros(B), t1)]
+
+
+def test_fp64_batch_that_teams_take(cuda, cache_file):
+    """Teams take an FP64 batch of this size whatever its lengths: there is no shape to tune, and none is stored for the
+    larger batches of the same power of two."""
+    B = 1000
+    ins, got = vdp(B, 1), []
+    for tune in (False, True):
+        s = Solver("vdp", 2, 1, B, tableau="dopri5", precision="fp64")
+        if tune:
+            assert all(v > 0 for v in s.autotune("sumsq", *ins).values())
+        got.append({k: v.cpu().numpy() for k, v in s.gradient("sumsq", *ins).items()})
+        s.close()
+    assert not cache_file.exists()
+    for k in got[0]:
+        np.testing.assert_array_equal(got[1][k], got[0][k])
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed_dw"])
+def test_tuned_on_another_batch(cuda, cache_file, precision):
+    """A handle tuned on a batch with one long instance, which teams take in FP64, and then given an even one: the bits of
+    an untuned handle, in no more than 1.25 times its time (every candidate timed the same team; the arbitrary winner
+    may take twice as long)."""
+    B = 65536
+    even, uneven, got, ms = vdp(B, 1), vdp(B, 1, uneven=True), [], []
+    for tune in (False, True):
+        s = Solver("vdp", 2, 1, B, tableau="dopri5", precision=precision)
+        if tune:
+            s.autotune("sumsq", *uneven)
+        for _ in range(2):
+            out = s.gradient("sumsq", *even)
+        got.append({k: v.cpu().numpy() for k, v in out.items()})
+        best = []
+        for _ in range(4):
+            e = [torch.cuda.Event(enable_timing=True) for _ in range(2)]
+            e[0].record()
+            s.gradient("sumsq", *even)
+            e[1].record()
+            torch.cuda.synchronize()
+            best.append(e[0].elapsed_time(e[1]))
+        ms.append(min(best))
+        s.close()
+    for k in got[0]:
+        np.testing.assert_array_equal(got[1][k], got[0][k])
+    assert ms[1] <= 1.25 * ms[0], ms

@@ -71,6 +71,7 @@ struct va_handle {
     // tuned, and the block size of that
     bool default_fwd = true, default_bwd = true;
     int default_block = 128;
+    bool tuning = false; // va_autotune is timing shapes: one lane each, no teams, no split
     int N = 0, P = 0;
     int RS = 0; // doubles per checkpoint record at the current stride (record_layout)
     bool stages_on = true; // opt.stage_records, cleared by the automatic checkpoint ladder
@@ -662,7 +663,7 @@ va_status launch_teams(va_handle *h, int sweep, Params &a, cudaStream_t s, bool 
 {
     const std::vector<va::TeamKernel> &teams = h->teams[sweep];
     one_lane = true;
-    if (teams.empty())
+    if (teams.empty() || (h->tuning && sweep != va::FP64_TWO_LEVEL))
         return VA_OK;
     const int64_t B = h->prob.batch;
     const float quads = 4.0f * (float)h->sm_count;
@@ -816,7 +817,7 @@ va_status enqueue_forward(va_handle *h, const double *y0, const double *params, 
         a.work_valid = h->inst_work + a.B;
     }
     VA_CUDA(h, cudaMemsetAsync(h->ctl, 0, sizeof(va::Control), s));
-    if (h->side && a.load) {
+    if (h->side && a.load && !h->tuning) {
         const va_status st = fork_long(h, h->long_fwd, a, s);
         if (st != VA_OK)
             return st;
@@ -970,7 +971,7 @@ va_status enqueue_backward(va_handle *h, const double *params, const double *lam
     if (h->bwd_grid <= 0)
         h->bwd_grid = grid_for(h, fn, h->bwd_block, a.B);
     VA_CUDA(h, cudaMemsetAsync(&h->ctl->adj_next, 0, sizeof(unsigned int), s));
-    if (h->side && a.load) {
+    if (h->side && a.load && !h->tuning) {
         VA_CUDA(h, cudaMemsetAsync(&h->ctl->adj_long, 0, sizeof(unsigned int), s));
         const va_status st = fork_long(h, h->long_bwd, a, s);
         if (st != VA_OK)
@@ -1026,6 +1027,18 @@ void apply_shape(va_handle *h, const TunedShape &t)
     h->default_bwd = !given && t.bb == 0;
     h->bwd_block = t.bb > 0 ? t.bb : h->default_block;
     h->bwd_grid = t.bb > 0 ? grid_of(h, bfn, t.bb, t.bbps) : grid_for(h, bfn, h->bwd_block, h->prob.batch);
+}
+
+// Whether teams take every batch of the handle's size whatever its load, in both
+// sweeps: no launch shape to tune.
+bool teams_always(const va_handle *h)
+{
+    auto all = [&](int sweep) {
+        const std::vector<va::TeamKernel> &t = h->teams[sweep];
+        return !t.empty() && (float)h->prob.batch <= t.back().per_quad * 4.0f * (float)h->sm_count;
+    };
+    return !h->bks && h->prob.batch <= va::kSmallBatch && all(va::FP64_FORWARD) &&
+           (h->stride > 1 || all(va::FP64_BACKWARD));
 }
 
 // Forward and backward once untimed, then the best of two timed runs.
@@ -1092,6 +1105,7 @@ va_status autotune_sweep(va_handle *h, int32_t cost, const double *y0, const dou
     }
     va_status st = VA_OK;
     va::ShapePair pair;
+    h->tuning = true;
     va::tune_pair(
         shapes,
         [&](va::Shape f, va::Shape b, float &tf, float &tb) {
@@ -1100,6 +1114,7 @@ va_status autotune_sweep(va_handle *h, int32_t cost, const double *y0, const dou
             return st == VA_OK;
         },
         pair);
+    h->tuning = false;
     best = TunedShape{pair.fwd.block, pair.fwd.bps, pair.bwd.block, pair.bwd.bps, 0};
     return st;
 }
@@ -1860,6 +1875,10 @@ va_status va_autotune(va_handle *h, int32_t cost, const double *y0, const double
         st = ensure_scratch(h);
     if (st != VA_OK)
         return st;
+    if (teams_always(h)) {
+        apply_shape(h, TunedShape{});
+        return VA_OK;
+    }
     const std::string key = cache_key(h);
     TunedShape t;
     auto shape = [](int block, int bps) { return block == 0 ? bps == 0 : block > 0 && bps > 0; };
