@@ -241,9 +241,10 @@ void fp64_path(va_handle *h)
         h->teams[va::FP64_BACKWARD].front().per_quad = k->seeds_per_quad[t];
     if (!k->int_fwd[t])
         return;
-    if (h->prob.batch >= k->int_fwd_min)
+    const float per_quad = (float)h->prob.batch / (4.0f * (float)h->sm_count);
+    if (per_quad >= k->int_fwd_min)
         h->sw_fwd = k->int_fwd[t];
-    if (h->prob.batch >= k->int_bwd_min)
+    if (per_quad >= k->int_bwd_min)
         h->sw_bwd = k->int_bwd[t];
     if (h->ks->tpi == 1 && h->opt.block_size <= 0 && h->opt.blocks_per_sm <= 0) {
         h->fwd_block = h->bwd_block = h->prob.batch > 256 * h->sm_count ? 256 : 128;

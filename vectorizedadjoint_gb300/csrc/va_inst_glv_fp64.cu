@@ -22,7 +22,7 @@ static void fill(KernelSet &k)
 // N = 10 needs more registers than there are (9.1 -> 9.3), and with few warps
 // the longer code loses for both (777 instances, N = 5: 1.04 -> 1.41).
 // (one instance, N = 10: 0.48 -> 0.51 forward.)
-constexpr int kTwoWarps5 = 2 * 608 * 6; // groups of 5 that fill two warps per quadrant of 152 SMs
+constexpr float kTwoWarps5 = 2 * 6; // groups of 5 that fill two warps
 template <int NN>
 static Fp64Kernels make_int()
 {
@@ -34,7 +34,7 @@ static Fp64Kernels make_int()
         k.int_bwd[0] = (const void *)backward_group_kernel<M, TabDopri5, double, true>;
         k.int_bwd[1] = (const void *)backward_group_kernel<M, TabCK54, double, true>;
     }
-    k.int_fwd_min = NN == 5 ? kTwoWarps5 : 32;
+    k.int_fwd_min = NN == 5 ? kTwoWarps5 : 0.05f;
     k.int_bwd_min = kTwoWarps5;
     // A warp per instance (va_team_glv64.cuh); limits where the lane groups are
     // faster, ms (load ~0.8 B):

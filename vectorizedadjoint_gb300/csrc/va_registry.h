@@ -115,7 +115,7 @@ enum { FP64_FORWARD = 0, FP64_BACKWARD = 1, FP64_TWO_LEVEL = 2, kFp64Sweeps = 3 
 constexpr int kTeams = 4;
 struct Fp64Kernels {
     const void *int_fwd[kTableaux], *int_bwd[kTableaux];
-    int int_fwd_min, int_bwd_min; // smallest batches they take
+    float int_fwd_min, int_bwd_min; // smallest batches they take, per SM quadrant
     TeamKernel team[kTableaux][kFp64Sweeps][kTeams]; // widest first
     // limit of the widest backward team when there are two seed rows or more
     // (0: the listed one)
