@@ -138,7 +138,7 @@ struct ModelGLVLane {
 
     // the same with the products on the integer pipe (va_step64.cuh): the
     // factors that cross lanes are exchanged unpacked
-    static constexpr bool kProducts64 = true, kForwardRhsFp64 = false;
+    static constexpr bool kForwardRhsFp64 = false;
     __device__ __forceinline__ static MulR from_lane(const MulR &v, int src, unsigned mask)
     {
         return {__shfl_sync(mask, v.h, src), __shfl_sync(mask, v.l, src), __shfl_sync(mask, v.e, src)};

@@ -45,8 +45,8 @@ static void fill(TeamKernel (&t)[kFp64Sweeps][kTeams], float &seeds_per_quad)
     t[FP64_BACKWARD][2] = {(const void *)backward_team_kernel<M, Tab, 4>, 4, 1, 6.6f};
     t[FP64_BACKWARD][3] = {(const void *)backward_team_kernel<M, Tab, 2>, 2, 1, 13.0f};
     seeds_per_quad = 13.0f;
-    t[FP64_TWO_LEVEL][0] = {(const void *)backward_team_kernel_2level<M, Tab, 32>, 32, 2, 0.75f};
-    t[FP64_TWO_LEVEL][1] = {(const void *)backward_team_kernel_2level<M, Tab, 16>, 16, 2, 50.0f};
+    t[FP64_TWO_LEVEL][0] = {(const void *)backward_team_kernel_2level<M, Tab, 32>, 32, 0, 0.75f};
+    t[FP64_TWO_LEVEL][1] = {(const void *)backward_team_kernel_2level<M, Tab, 16>, 16, 0, 50.0f};
 }
 template <class M>
 static void fill_model(Fp64Kernels &k)

@@ -25,8 +25,8 @@ static void fill(Fp64Kernels &k)
     t[FP64_BACKWARD][0] = {(const void *)backward_team_kernel<M, TabRKF78, 32>, 32, 2, 1.2f};
     t[FP64_BACKWARD][1] = {(const void *)backward_team_kernel<M, TabRKF78, 16>, 16, 2, 7.0f};
     t[FP64_BACKWARD][2] = {(const void *)backward_team_kernel<M, TabRKF78, 8>, 8, 2, 18.0f};
-    t[FP64_TWO_LEVEL][0] = {(const void *)backward_team_kernel_2level<M, TabRKF78, 32>, 32, 2, 0.5f};
-    t[FP64_TWO_LEVEL][1] = {(const void *)backward_team_kernel_2level<M, TabRKF78, 16>, 16, 2, 35.0f};
+    t[FP64_TWO_LEVEL][0] = {(const void *)backward_team_kernel_2level<M, TabRKF78, 32>, 32, 0, 0.5f};
+    t[FP64_TWO_LEVEL][1] = {(const void *)backward_team_kernel_2level<M, TabRKF78, 16>, 16, 0, 35.0f};
 }
 
 void fill_team_rkf78_vdp(Fp64Kernels &k) { fill<ModelVdP>(k); }

@@ -628,12 +628,7 @@ VA_HD_NOINLINE Attempt64<M::N> attempt_general64(State64<M::N, M::P> s, double a
 {
     Attempt64<M::N> o;
     double same[M::N];
-    if constexpr (Tab::FIXED) {
-        step_fixed<M, Tab, double>(s.y, s.y, s.k0, s.p, s.t, s.dt, o.ynew, same);
-        o.err = 0.0;
-    } else {
-        o.err = attempt_pair<M, Tab, double>(s.y, s.y, s.k0, s.p, s.t, s.dt, atol, rtol, o.ynew, same, o.knew);
-    }
+    o.err = attempt_pair<M, Tab, double>(s.y, s.y, s.k0, s.p, s.t, s.dt, atol, rtol, o.ynew, same, o.knew);
     return o;
 }
 
@@ -1090,7 +1085,7 @@ __host__ __device__ __forceinline__ void back_step(const double (&y)[M::N], doub
 {
     if constexpr (INT64) {
         double l[M::N], m[M::PG];
-        if (uniform64<M>(back_step64<M, Tab>(y, tn, h, p, lam, mu, l, m))) {
+        if (uniform64<M>(back_step64<M, Tab>(y, h, p, lam, mu, l, m))) {
 #pragma unroll
             for (int i = 0; i < M::N; i++)
                 lam[i] = l[i];
@@ -1253,7 +1248,7 @@ __global__ void __launch_bounds__(256) backward_kernel(AdjParams a)
 // back_step through the segment in reverse.  Memory: one record per stride
 // steps plus (stride + 1) scratch records per thread, for one extra forward
 // evaluation of every step.
-template <class M, class Tab, class S, bool INT64 = false>
+template <class M, class Tab, class S>
 __global__ void __launch_bounds__(256) backward_kernel_2level(AdjParams a)
 {
     constexpr int N = M::N, P = M::P;
@@ -1405,7 +1400,7 @@ __global__ void __launch_bounds__(256) backward_kernel_2level(AdjParams a)
             }
             double ynew[N];
             S ynew_s[N], knew[N];
-            const double err = attempt<M, Tab, S, INT64>(y, ys, k0, p, t, dt, a.atol, a.rtol, ynew, ynew_s, knew);
+            const double err = attempt<M, Tab, S>(y, ys, k0, p, t, dt, a.atol, a.rtol, ynew, ynew_s, knew);
             if (is_nan64(err) || fails >= a.max_fail) {
                 fail_instance(ST_RECOMPUTE_MISMATCH);
                 alive = fetch();
@@ -1455,7 +1450,7 @@ __global__ void __launch_bounds__(256) backward_kernel_2level(AdjParams a)
                 yj[i] = r[2 + i];
             const double tn = r[0];
             const double h = scr[(size_t)(jb + 1) * RS] - tn;
-            back_step<M, Tab, S, INT64>(yj, tn, h, p, lam, mu);
+            back_step<M, Tab, S>(yj, tn, h, p, lam, mu);
             note_lambda<N>(a, b, q, first + jb, lam);
             jb--;
             if (jb < 0) {

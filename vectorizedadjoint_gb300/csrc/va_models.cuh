@@ -76,7 +76,7 @@ struct ModelVdP {
             gp[0] = w[1] * ((S(1) - x[0] * x[0]) * x[1]);
         }
     }
-    static constexpr bool kProducts64 = true, kForwardRhsFp64 = true;
+    static constexpr bool kForwardRhsFp64 = true;
     __host__ __device__ __forceinline__ static void rhs64(const double *x, const double *p, double *f, MulRange &r)
     {
         const double a = 1.0 - mul_rn(mul_left(x[0], r), mul_right_in(x[0]));
@@ -136,7 +136,7 @@ struct ModelVdPPetsc {
             gp[0] = w[1] * ((S(1) - x[0] * x[0]) * x[1] - x[0]);
         }
     }
-    static constexpr bool kProducts64 = true, kForwardRhsFp64 = true;
+    static constexpr bool kForwardRhsFp64 = true;
     __host__ __device__ __forceinline__ static void rhs64(const double *x, const double *p, double *f, MulRange &r)
     {
         const double a = 1.0 - mul_rn(mul_left(x[0], r), mul_right_in(x[0]));
@@ -204,7 +204,7 @@ struct ModelDHO {
             gp[1] = w[1] * (S(-2) * om * x[1]);
         }
     }
-    static constexpr bool kProducts64 = true, kForwardRhsFp64 = true;
+    static constexpr bool kForwardRhsFp64 = true;
     __host__ __device__ __forceinline__ static void rhs64(const double *x, const double *p, double *f, MulRange &r)
     {
         const MulL om = mul_left_in(p[0]), ze = mul_left_in(p[1]);
@@ -251,7 +251,7 @@ struct ModelDecay {
         gx[0] = -p[0] * w[0];
         gp[0] = -x[0] * w[0];
     }
-    static constexpr bool kProducts64 = true, kForwardRhsFp64 = true;
+    static constexpr bool kForwardRhsFp64 = true;
     __host__ __device__ __forceinline__ static void rhs64(const double *x, const double *p, double *f, MulRange &r)
     {
         f[0] = mul_rn(mul_neg(mul_left_in(p[0])), mul_right(x[0], r));

@@ -98,7 +98,7 @@ void fill_fixed_glv10(KernelSet &k);
 struct TeamKernel {
     const void *fn;
     int lanes;       // per instance
-    int bps;         // resident blocks of 128 threads per SM
+    int bps;         // resident blocks of 128 threads per SM (two-level: 0, kTwoLevelBlocksPerSm)
     float per_quad;  // highest load, per SM quadrant, that the team takes
 };
 // Segments that a team of g lanes re-integrates at once in the two-level

@@ -15,8 +15,7 @@
 // right-hand sides as well 4.99, the coefficients c h as well 5.1; the error's
 // terms of one component 4.17 forward).
 //
-// The operations and their order are those of attempt_pair, step_fixed and
-// back_step; every sum is the FP64 instruction and every product the
+// The operations and their order are those of attempt_pair and back_step; every sum is the FP64 instruction and every product the
 // correctly rounded one, so the results have the same bits.  For the 5(4)
 // pairs: no a_mj is zero, and a zero b_m or e_m is left out of the sums as it
 // is in attempt_pair.
@@ -40,50 +39,24 @@ namespace va {
 
 constexpr int kChainRange = 240;
 
-// Models that write their right-hand side and VJP with integer products
-// (rhs64, vjp64); for the others (a model compiled by the caller) the model
-// functions run as they are.
-template <class M, class = void>
-struct HasProducts64 : std::false_type {
-};
-template <class M>
-struct HasProducts64<M, std::void_t<decltype(M::kProducts64)>> : std::bool_constant<M::kProducts64> {
-};
-
-// the model's parameters into the range, once per step (rhs64 and vjp64 take
-// them as noted)
+// the model's parameters into the range, once per step (rhs64 and vjp64, the
+// model's functions with integer products, take them as noted)
 template <class M>
 __host__ __device__ __forceinline__ void note_params64(const double (&p)[M::P], MulRange &r)
 {
-    if constexpr (HasProducts64<M>::value) {
 #pragma unroll
-        for (int k = 0; k < M::P; k++)
-            r.note(f64_hi(p[k]), f64_lo(p[k]));
-    }
+    for (int k = 0; k < M::P; k++)
+        r.note(f64_hi(p[k]), f64_lo(p[k]));
 }
-template <class M, bool FORWARD = false>
-__host__ __device__ __forceinline__ void model_rhs64(const double *x, const double *p, double t, double *f,
-                                                     MulRange &r)
-{
-    if constexpr (HasProducts64<M>::value && !(FORWARD && M::kForwardRhsFp64)) {
-        (void)t;
-        M::rhs64(x, p, f, r);
-    } else {
-        (void)r;
-        M::template rhs<double>(x, p, t, f);
-    }
-}
+// the right-hand side of a forward stage
 template <class M>
-__host__ __device__ __forceinline__ void model_vjp64(const double *w, const double *x, const double *p, double t,
-                                                     double *gx, double *gp, MulRange &r)
+__host__ __device__ __forceinline__ void forward_rhs64(const double *x, const double *p, double t, double *f,
+                                                       MulRange &r)
 {
-    if constexpr (HasProducts64<M>::value) {
-        (void)t;
-        M::vjp64(w, x, p, gx, gp, r);
-    } else {
-        (void)r;
-        M::template vjp<double>(w, x, p, t, gx, gp);
-    }
+    if constexpr (M::kForwardRhsFp64)
+        M::template rhs<double>(x, p, t, f);
+    else
+        M::rhs64(x, p, f, r);
 }
 
 // Whether every lane that carries the instance stayed in range (a lane-group
@@ -146,7 +119,7 @@ __host__ __device__ __forceinline__ bool attempt64(const double (&y)[M::N], cons
     for (int m = 1; m < NS; m++) {
         double X[N], f[N];
         form_stage64<Tab, N>(m, y, K, h, X);
-        model_rhs64<M, true>(X, p, t + Tab::c(m) * dt, f, r);
+        forward_rhs64<M>(X, p, t + Tab::c(m) * dt, f, r);
 #pragma unroll
         for (int i = 0; i < N; i++)
             K[m][i] = mul_left(f[i], r);
@@ -176,7 +149,7 @@ __host__ __device__ __forceinline__ bool attempt64(const double (&y)[M::N], cons
             first = false;
         }
     if constexpr (Tab::FSAL) {
-        model_rhs64<M, true>(ynew, p, t + dt, knew, r);
+        forward_rhs64<M>(ynew, p, t + dt, knew, r);
         const MulR c = coef_right(Tab::E_NEW, h);
 #pragma unroll
         for (int i = 0; i < N; i++)
@@ -198,7 +171,7 @@ __host__ __device__ __forceinline__ bool attempt64(const double (&y)[M::N], cons
 // back_step for double stages: lambda_n in ybar, mu's new sums in ms.  False:
 // out of range.
 template <class M, class Tab>
-__host__ __device__ __forceinline__ bool back_step64(const double (&y)[M::N], double tn, double hh,
+__host__ __device__ __forceinline__ bool back_step64(const double (&y)[M::N], double hh,
                                                      const double (&p)[M::P], const double (&lam)[M::N],
                                                      const double (&mu)[M::PG], double (&ybar)[M::N],
                                                      double (&ms)[M::PG])
@@ -215,7 +188,7 @@ __host__ __device__ __forceinline__ bool back_step64(const double (&y)[M::N], do
             form_stage64<Tab, N>(m, y, K, h, X[m]);
             if (m < NS - 1) {
                 double f[N];
-                model_rhs64<M>(X[m], p, tn + Tab::c(m) * hh, f, r);
+                M::rhs64(X[m], p, f, r);
 #pragma unroll
                 for (int i = 0; i < N; i++)
                     K[m][i] = mul_left(f[i], r);
@@ -243,7 +216,7 @@ __host__ __device__ __forceinline__ bool back_step64(const double (&y)[M::N], do
 #pragma unroll
     for (int m = NS - 1; m >= 0; m--) {
         double gx[N], gp[P];
-        model_vjp64<M>(Kbar[m], X[m], p, tn + Tab::c(m) * hh, gx, gp, r);
+        M::vjp64(Kbar[m], X[m], p, gx, gp, r);
 #pragma unroll
         for (int i = 0; i < N; i++) {
             ybar[i] += gx[i];
