@@ -100,3 +100,17 @@ def test_similar_magnitudes_reach_the_double_word_level():
         folded, _, exact, _ = scheme(a, v)
         total = sum(abs(x) * abs(y) for x, y in zip(a, v))
         assert float(abs(folded - exact)) <= 2e-15 * total
+
+
+def test_digits_in_place_are_the_digits(tmp_path):
+    """The contraction's digits with their weights (split_digits_in_place) against split_digits, on the host: columns of
+    every size, values far below the column's maximum, ties and their neighbours, zeros of both signs."""
+    import os
+    import subprocess
+    from vectorizedadjoint_gb300 import build as vbuild
+    src = os.path.join(os.path.dirname(os.path.abspath(__file__)), "cpp", "digits_check.cu")
+    exe = str(tmp_path / "digits_check")
+    subprocess.run([vbuild.NVCC, "-gencode=arch=compute_103a,code=sm_103a", "-std=c++17", "-O2",
+                    "--expt-relaxed-constexpr", "-Xcompiler", "-ffp-contract=off", src, "-o", exe], check=True)
+    differ, tried = map(int, subprocess.run([exe], check=True, capture_output=True, text=True).stdout.split())
+    assert tried > 3_000_000 and differ == 0

@@ -250,3 +250,94 @@ def test_longest_instances_apart(cuda, tab, B, nout):
     want = ref.gradient("sumsq", *ins)
     for k in ("dy0", "dp", "status"):
         np.testing.assert_array_equal(r[k].cpu().numpy(), want[k].cpu().numpy())
+
+
+@pytest.mark.parametrize("model", ["vdp", "vdp_petsc", "dho"])
+@pytest.mark.parametrize("tab", ["dopri5", "ck54"])
+@pytest.mark.parametrize("B", [1, 45, 700])
+def test_special_values_one_lane(oracle, cuda, model, tab, B):
+    """One lane per instance with integer products, forward and backward, at any batch size (a block size that teams do not
+    take): zeros of both signs, states and parameters across and beyond the products' range, infinities and NaN, where
+    attempt64 and back_step64 refuse and the general step takes over, beside ordinary lanes of the same warp."""
+    y0, p, t1 = draw(model, B, 11)
+    t1 = np.minimum(t1, 1.0)
+    special = [(0.0, 1.0), (-0.0, 1.0), (1.0, -0.0), (0.0, 0.0), (1e-70, 1e-75), (1e-90, 1.0), (1e-310, 1e-300),
+               (0.5, 4e-320), (np.inf, 1.0), (1.0, -np.inf), (np.nan, 0.0)]
+    if model == "dho":  # (a nonlinear model would be stiff there)
+        special += [(1e-30, -1e74), (1e74, -1e70), (3e150, 1.0)]
+    for k, v in enumerate(special):
+        y0[k % B] = v
+        if B == 1:
+            break
+    if B > 40:
+        for k, v in enumerate([0.0, -0.0, 1e-80, 1e-310, 2.0 ** -241, 2.0 ** -239]):
+            p[20 + k, 0] = v
+            p[30 + k, -1] = v
+        p[26], t1[26] = 1e3, 1e-3
+        t1[27], t1[28] = 0.0, 1e-12
+    n = y0.shape[1]
+    s = Solver(model, n, NP[model], B, tableau=tab, precision="fp64", atol=1e-6, rtol=1e-6, block_size=48)
+    out = s.gradient("sumsq", dev(y0), dev(p), dev(np.zeros(B)), dev(t1))
+    torch.cuda.synchronize()
+    r = {k: v.cpu().numpy() for k, v in out.items()}
+    s.close()
+    pb = oracle.problem(model, tab, n, NP[model], 1e-6, 1e-6)
+    ran = 0
+    for b in range(min(B, 45)):
+        g = oracle.gradient(pb, "sumsq", y0[b], p[b], 0.0, t1[b])
+        assert int(r["status"][b]) == g["status"], b
+        if g["status"] != 0:
+            continue
+        ran += 1
+        assert int(r["n_acc"][b]) == g["n_acc"], b
+        for k in ("yT", "dy0", "dp"):
+            np.testing.assert_array_equal(r[k][b], g[k], err_msg=f"{k} {b}")
+    assert ran >= min(B, 30)
+
+
+def parts(lengths, quads):
+    """What the longest-first sort makes of a batch: its load and the size of the longest part (0: not split)."""
+    top = lengths.max()
+    load = lengths.sum() / top
+    if not 1.5 * quads < load <= 40 * quads:
+        return load, 0
+    for share in (0.4, 0.5, 0.6, 0.75):
+        part = lengths[lengths > share * top]
+        if part.sum() / top <= 2 * quads:
+            return load, len(part)
+    return load, 0
+
+
+@pytest.mark.parametrize("nout,stride", [(1, 0), (2, 0), (3, 0), (1, 5)])
+@pytest.mark.parametrize("tab", ["dopri5", "ck54"])
+def test_split_batch(cuda, tab, nout, stride):
+    """Batches well inside the range in which the longest instances run apart, by horizons (first call) and by step counts
+    (second), several hundred of them and all successful: forward, backward with one and several seed rows, and the
+    forward's split with the two-level backward, against one sweep for all in an explicit launch shape."""
+    B = 40000
+    quads = 4.0 * torch.cuda.get_device_properties(0).multi_processor_count
+    rng = np.random.default_rng(3)
+    y0, p, _ = draw("dho", B, 4)
+    t1 = rng.uniform(0.2, 5.0, B)
+    long = rng.choice(B, 1200, replace=False)
+    t1[long] = rng.uniform(15.0, 30.0, len(long))
+    lam, mud = rng.standard_normal((B, nout, 2)), rng.standard_normal((B, nout, 2))
+    got = []
+    for kw in (dict(block_size=64), dict()):
+        s = Solver("dho", 2, 2, B, nout=nout, tableau=tab, precision="fp64", atol=1e-7, rtol=1e-7, ckpt_stride=stride, **kw)
+        if not stride:
+            s.set_adjoint_history(3)
+        for _ in range(2):
+            f = s.forward(dev(y0), dev(p), dev(np.zeros(B)), dev(t1))
+            g = s.backward(dev(p), dev(lam), dev(mud))
+            got.append([f[k].cpu().numpy() for k in ("yT", "n_acc", "n_rej", "status")] +
+                       [g[k].cpu().numpy() for k in ("status", "dy0", "dp")] +
+                       ([s.adjoint_history(int(b))[1] for b in (long[0], 0)] if not stride else []))
+        s.close()
+    assert (got[0][3] == 0).all() and (got[0][4] == 0).all()
+    for lengths in (t1, (got[0][1] + got[0][2]).astype(float), got[0][1].astype(float)):
+        load, part = parts(lengths, quads)
+        assert 1.6 * quads < load < 30 * quads and 200 <= part <= 2000, (load, part)  # else this tests nothing
+    for r in got[1:]:
+        for a, b in zip(r, got[0]):
+            np.testing.assert_array_equal(a, b)
