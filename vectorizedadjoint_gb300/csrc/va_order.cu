@@ -64,7 +64,7 @@ __device__ __forceinline__ int horizon_bucket(double h)
 __device__ __forceinline__ int count_bucket(int n) { return n < kBuckets ? (n < 0 ? 0 : n) : kBuckets - 1; }
 
 // work[0 ..): the buckets' counts, then, zeroed with them, how many instances
-// moved and the longest of now (order_moved)
+// moved and the longest of now (order_hist)
 constexpr int kMovedSlot = kBuckets, kLongestSlot = kBuckets + 1, kZeroed = kBuckets + 2;
 // work[kOffsets ..): the buckets' offsets
 constexpr int kOffsets = kZeroed;
@@ -118,22 +118,27 @@ __device__ __forceinline__ float bucket_length(bool counted, int k)
     return counted ? (float)k : exp2f((float)k * (1.0f / 64.0f) - 32.0f);
 }
 
-// How many instances moved and the longest of now, before the order of a
-// backward sweep: two loads an instance, and a launch of ~2 us.  One atomic a
-// block: one a warp (262,144 instances: 8,192 on one address) took 20 us.
-__global__ void __launch_bounds__(1024) order_moved(OrderArgs a)
+// The buckets' counts and, where the forward's order may be reused, how many
+// instances moved and the longest of now: two loads an instance more, and one
+// atomic a block (one a warp, 8,192 on one address for 262,144 instances, took
+// 20 us; a launch of its own 4 us).
+__global__ void __launch_bounds__(1024) order_hist(OrderArgs a)
 {
-    __shared__ int block_moved, block_top;
-    if (a.work[kCountedFlag] != 1)
-        return;
+    __shared__ int h[kBuckets], block_moved, block_top;
+    const bool compare = a.reuse && a.work[kCountedFlag] == 1;
+    for (int i = threadIdx.x; i < kBuckets; i += blockDim.x)
+        h[i] = 0;
     if (threadIdx.x == 0)
         block_moved = block_top = 0;
     __syncthreads();
     int moved = 0, top = 0;
     for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < a.B; b += gridDim.x * blockDim.x) {
-        const int n = a.now[b];
-        moved += length_moved(a.work[kTaken + b], n) ? 1 : 0;
-        top = n > top ? n : top;
+        atomicAdd(&h[key_of(a, b)], 1);
+        if (compare) {
+            const int n = a.now[b];
+            moved += length_moved(a.work[kTaken + b], n) ? 1 : 0;
+            top = n > top ? n : top;
+        }
     }
     moved = __reduce_add_sync(0xffffffffu, moved);
     top = __reduce_max_sync(0xffffffffu, top);
@@ -142,23 +147,10 @@ __global__ void __launch_bounds__(1024) order_moved(OrderArgs a)
         atomicMax(&block_top, top);
     }
     __syncthreads();
-    if (threadIdx.x == 0) {
+    if (compare && threadIdx.x == 0) {
         atomicAdd(&a.work[kMovedSlot], block_moved);
         atomicMax(&a.work[kLongestSlot], block_top);
     }
-}
-
-__global__ void order_hist(OrderArgs a)
-{
-    if (reusing(a))
-        return;
-    __shared__ int h[kBuckets];
-    for (int i = threadIdx.x; i < kBuckets; i += blockDim.x)
-        h[i] = 0;
-    __syncthreads();
-    for (int b = blockIdx.x * blockDim.x + threadIdx.x; b < a.B; b += gridDim.x * blockDim.x)
-        atomicAdd(&h[key_of(a, b)], 1);
-    __syncthreads();
     for (int i = threadIdx.x; i < kBuckets; i += blockDim.x)
         if (h[i])
             atomicAdd(&a.work[i], h[i]);
@@ -402,13 +394,10 @@ cudaError_t enqueue_order(const OrderArgs &a, cudaStream_t s)
     cudaError_t e = cudaMemsetAsync(a.work, 0, sizeof(int) * kZeroed, s);
     if (e != cudaSuccess)
         return e;
-    const int grid = (a.B + 255) / 256 < 1024 ? (a.B + 255) / 256 : 1024;
-    const int sgrid = (a.B + 1023) / 1024 < 256 ? (a.B + 1023) / 1024 : 256;
-    if (a.reuse)
-        order_moved<<<sgrid, 1024, 0, s>>>(a);
-    order_hist<<<grid, 256, 0, s>>>(a);
+    const int grid = (a.B + 1023) / 1024 < 256 ? (a.B + 1023) / 1024 : 256;
+    order_hist<<<grid, 1024, 0, s>>>(a);
     order_scan<<<1, 1024, 0, s>>>(a);
-    order_scatter<<<sgrid, 1024, 0, s>>>(a);
+    order_scatter<<<grid, 1024, 0, s>>>(a);
     return cudaGetLastError();
 }
 
