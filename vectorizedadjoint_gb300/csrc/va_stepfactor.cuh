@@ -234,13 +234,14 @@ VA_HD inline void step_pow_dd(double x, double &ph, double &pl)
 //  2. rho = 1 - x r0^K from the exact integers X and M: M^K to >= 112 bits,
 //     times X, of which 2^p - Q is kept at 2^-80 (|rho| < 2^-18).
 //  3. w = rho/K + c2 rho^2 (64-bit products) + c3 rho^3 + u (1 + rho/K)
-//     (FP32), u = -(e/K) ln x as above; terms dropped < 2^-78.
+//     (FP32), u = -(e/K) ln x as above; dropped: c4 rho^4 < 2^-74.8 (K = 3 at
+//     the largest |rho| let through, 2^-18; the float root's are below 2^-21).
 //  4. r0 (1 + w) at 2^-64 of r0's last place.
 //  5. The rounding test: decided unless the value lies within 2^-70 of a
-//     rounding boundary (one call in ~2^16).  The error is below 2^-71.5:
+//     rounding boundary (one call in ~2^16).  The error is below 2^-71.2:
 //     ln x from a float logarithm (device __log2f: 2 ulp, < 2^-16 absolute,
-//     moves u by < 2^-72), the FP32 sum rounded at 2^31 2^-24 2^-80, and
-//     the terms of 2-4 below 2^-77 each.
+//     moves u by < 2^-72), the FP32 sum rounded at 2^31 2^-24 2^-80, the
+//     dropped term, and what 2-4 round, below 2^-77 each.
 //
 // false: not decided (or |rho| out of range); the caller then takes the
 // double-double pass.  0 < x < 1e30, x normal in FP32.
